@@ -1,7 +1,7 @@
 // The learned preconditioner's network: a 3-level 3-D convolutional U-Net
 // (channels c1/c2/c3, 3x3x3 kernels, BF16 weights and activations, FP32
 // accumulation), trained and run by the project's own kernels
-// (pps_unet_kernels.cu).  No reference counterpart.
+// (pps_unet_conv.cu).  No reference counterpart.
 //
 //   x0 --conv0,relu--> e1a --conv1,relu--> e1 ----------------------------(skip)--+
 //                                           |pool                                 |
@@ -56,14 +56,14 @@ int pad16(int c) { return (c + 15) / 16 * 16; }
 
 struct Acts {
     Dims s1{0, 0, 0}, s2{0, 0, 0}, s3{0, 0, 0};   // grid of each level
-    bf16 *x0 = nullptr, *e1a = nullptr, *cat1 = nullptr, *d1a = nullptr, *d1 = nullptr;
-    bf16 *p1 = nullptr, *e2a = nullptr, *cat2 = nullptr, *d2a = nullptr, *d2 = nullptr;
-    bf16 *p2 = nullptr, *e3a = nullptr, *e3 = nullptr;
-    float* out = nullptr;
-    // gradients
-    bf16 *g_out = nullptr, *g_d1 = nullptr, *g_d1a = nullptr, *g_cat1 = nullptr, *g_d2 = nullptr, *g_d2a = nullptr,
-         *g_cat2 = nullptr, *g_e3 = nullptr, *g_e3a = nullptr, *g_p2 = nullptr, *g_e2a = nullptr, *g_p1 = nullptr,
-         *g_e1a = nullptr;
+    bf16 *e1a = nullptr, *e1 = nullptr, *d1a = nullptr, *d1 = nullptr;
+    bf16 *e2a = nullptr, *e2 = nullptr, *d2a = nullptr, *d2 = nullptr;
+    bf16 *e3a = nullptr, *e3 = nullptr;
+    // gradients: of the outputs of layers 9, 8, 6, 4, 2, 0 (masked where stored), of the
+    // two concatenations and the two pooled tensors, and of the dense output
+    bf16 *g_d1 = nullptr, *g_d1a = nullptr, *g_cat1 = nullptr, *g_d2a = nullptr, *g_cat2 = nullptr, *g_e3a = nullptr,
+         *g_p2 = nullptr, *g_e2a = nullptr, *g_p1 = nullptr, *g_e1a = nullptr;
+    float* g_out = nullptr;
     bool grads = false;
 };
 
@@ -77,10 +77,11 @@ struct pps_unet {
     std::vector<Layer> L;
     size_t npad = 0, nreal = 0;
     float *P = nullptr, *G = nullptr, *M = nullptr, *V = nullptr;   // FP32 master, grads, Adam moments
-    bf16* PB = nullptr;    // BF16 copy of the padded parameters
-    bf16* WF = nullptr;    // flipped weights of one layer (backward data)
-    float* dtmp = nullptr; // device scalar: rms of the input
-    double* dloss = nullptr;
+    bf16 *WP = nullptr, *WB = nullptr;   // BF16 weights in fragment order: forward, data gradient
+    PackTable pt{};
+    float* dtmp = nullptr; // device scalars: rms of the input, rms of the gradient
+    double* dloss = nullptr;   // behind the gradients in one allocation: one fill zeroes both
+    RmsScratch* drms = nullptr;
     int step = 0;
     Acts A;
 };
@@ -89,22 +90,18 @@ namespace {
 
 void free_acts(Acts& A)
 {
-    bf16* b[] = {A.x0, A.e1a, A.cat1, A.d1a, A.d1, A.p1, A.e2a, A.cat2, A.d2a, A.d2, A.p2, A.e3a, A.e3,
-                 A.g_out, A.g_d1, A.g_d1a, A.g_cat1, A.g_d2, A.g_d2a, A.g_cat2, A.g_e3, A.g_e3a, A.g_p2,
-                 A.g_e2a, A.g_p1, A.g_e1a};
+    bf16* b[] = {A.e1a, A.e1, A.d1a, A.d1, A.e2a, A.e2, A.d2a, A.d2, A.e3a, A.e3, A.g_d1, A.g_d1a, A.g_cat1, A.g_d2a,
+                 A.g_cat2, A.g_e3a, A.g_p2, A.g_e2a, A.g_p1, A.g_e1a};
     for (bf16* q : b)
         if (q) cudaFree(q);
-    if (A.out) cudaFree(A.out);
+    if (A.g_out) cudaFree(A.g_out);
     A = Acts();
 }
 
-// Zeroed on `s`, the stream whose kernels use the buffer next (the legacy stream's
-// fills are not ordered with the library's non-blocking streams).
-bf16* balloc(long long n, cudaStream_t s)
+bf16* balloc(long long n)
 {
     bf16* p = nullptr;
     UK(cudaMalloc((void**)&p, sizeof(bf16) * (size_t)n));
-    UK(cudaMemsetAsync(p, 0, sizeof(bf16) * (size_t)n, s));
     return p;
 }
 
@@ -113,144 +110,188 @@ void ensure_acts(pps_unet* u, int nx, int ny, int nz, bool grads)
     Acts& A = u->A;
     if (A.s1.W == nx && A.s1.H == ny && A.s1.D == nz && (A.grads || !grads)) return;
     free_acts(A);
+    const long long v1 = (long long)nx * ny * nz, v2 = v1 / 8, v3 = v2 / 8;
+    const int c1 = u->c1, c2 = u->c2, c3 = u->c3;
+    A.e1a = balloc(v1 * c1);
+    A.e1 = balloc(v1 * c1);
+    A.d1a = balloc(v1 * c1);
+    A.d1 = balloc(v1 * c1);
+    A.e2a = balloc(v2 * c2);
+    A.e2 = balloc(v2 * c2);
+    A.d2a = balloc(v2 * c2);
+    A.d2 = balloc(v2 * c2);
+    A.e3a = balloc(v3 * c3);
+    A.e3 = balloc(v3 * c3);
+    if (grads) {
+        UK(cudaMalloc((void**)&A.g_out, sizeof(float) * (size_t)v1));
+        A.g_d1 = balloc(v1 * c1);
+        A.g_d1a = balloc(v1 * c1);
+        A.g_cat1 = balloc(v1 * (c2 + c1));
+        A.g_d2a = balloc(v2 * c2);
+        A.g_cat2 = balloc(v2 * (c3 + c2));
+        A.g_e3a = balloc(v3 * c3);
+        A.g_p2 = balloc(v3 * c2);
+        A.g_e2a = balloc(v2 * c2);
+        A.g_p1 = balloc(v2 * c1);
+        A.g_e1a = balloc(v1 * c1);
+        A.grads = true;
+    }
+    // the extents last: an allocation that failed half way leaves none
     A.s1 = Dims{nz, ny, nx};
     A.s2 = Dims{nz / 2, ny / 2, nx / 2};
     A.s3 = Dims{nz / 4, ny / 4, nx / 4};
-    const long long v1 = (long long)nx * ny * nz, v2 = v1 / 8, v3 = v2 / 8;
-    const int c1 = u->c1, c2 = u->c2, c3 = u->c3;
-    A.x0 = balloc(v1 * 16, u->stream);
-    A.e1a = balloc(v1 * c1, u->stream);
-    A.cat1 = balloc(v1 * (c2 + c1), u->stream);
-    A.d1a = balloc(v1 * c1, u->stream);
-    A.d1 = balloc(v1 * c1, u->stream);
-    A.p1 = balloc(v2 * c1, u->stream);
-    A.e2a = balloc(v2 * c2, u->stream);
-    A.cat2 = balloc(v2 * (c3 + c2), u->stream);
-    A.d2a = balloc(v2 * c2, u->stream);
-    A.d2 = balloc(v2 * c2, u->stream);
-    A.p2 = balloc(v3 * c2, u->stream);
-    A.e3a = balloc(v3 * c3, u->stream);
-    A.e3 = balloc(v3 * c3, u->stream);
-    UK(cudaMalloc((void**)&A.out, sizeof(float) * (size_t)v1 * 16));
-    if (grads) {
-        A.g_out = balloc(v1 * 16, u->stream);
-        A.g_d1 = balloc(v1 * c1, u->stream);
-        A.g_d1a = balloc(v1 * c1, u->stream);
-        A.g_cat1 = balloc(v1 * (c2 + c1), u->stream);
-        A.g_d2 = balloc(v2 * c2, u->stream);
-        A.g_d2a = balloc(v2 * c2, u->stream);
-        A.g_cat2 = balloc(v2 * (c3 + c2), u->stream);
-        A.g_e3 = balloc(v3 * c3, u->stream);
-        A.g_e3a = balloc(v3 * c3, u->stream);
-        A.g_p2 = balloc(v3 * c2, u->stream);
-        A.g_e2a = balloc(v2 * c2, u->stream);
-        A.g_p1 = balloc(v2 * c1, u->stream);
-        A.g_e1a = balloc(v1 * c1, u->stream);
-        A.grads = true;
-    }
 }
 
-const bf16* Wb(const pps_unet* u, int l) { return u->PB + u->L[(size_t)l].w; }
 const float* Bf(const pps_unet* u, int l) { return u->P + u->L[(size_t)l].b; }
 
-// The forward pass.  With `dense_out` (inference) the glue kernels fold into the
-// convolutions next to them: the first reads the dense input scaled by 1/(*rms_dev),
-// the two after an upsampling read the coarse tensor for the upsampled channels, and
-// the last writes channel 0 times (*rms_dev) * gain into dense_out (the same values;
-// A.x0, the upsampled slots of A.cat1/A.cat2 and A.out are then not written).
-// Without it (training) every activation is stored for the backward pass.
-void forward(pps_unet* u, const float* in, const float* rms_dev, float* dense_out = nullptr, float gain = 1.0f)
+Src plain(const bf16* X, int ld, int c0 = 0)
+{
+    Src s;
+    s.X = X;
+    s.ld = ld;
+    s.c0 = c0;
+    return s;
+}
+Src pooled(const bf16* fine, int ld)
+{
+    Src s = plain(fine, ld);
+    s.kind = SRC_POOL;
+    return s;
+}
+// the concatenation [upsampled coarse tensor | skip tensor]
+Src concat(const bf16* up, int c_up, const bf16* skip, int c_skip)
+{
+    Src s = plain(skip, c_skip, -c_up);
+    s.kind = SRC_UP;
+    s.up = up;
+    s.ld_up = c_up;
+    s.c_up = c_up;
+    return s;
+}
+Src dense(const float* in, const float* rms_dev)
+{
+    Src s;
+    s.kind = SRC_DENSE;
+    s.dense = in;
+    s.rms = rms_dev;
+    return s;
+}
+// the gradient of a tensor that was upsampled: its channels lie first in the
+// concatenation's gradient
+Src children(const bf16* gcat, int ld, const bf16* mask, int ldm)
+{
+    Src s = plain(gcat, ld);
+    s.kind = SRC_CHILDREN;
+    s.mask = mask;
+    s.ldm = ldm;
+    return s;
+}
+// the gradient of a skip tensor: its slot of the concatenation's gradient plus the pooled path
+Src skip(const bf16* gcat, int ld, int c0, const bf16* gpool, int c, const bf16* mask)
+{
+    Src s = plain(gcat, ld, c0);
+    s.kind = SRC_SKIP;
+    s.up = gpool;
+    s.ld_up = c;
+    s.mask = mask;
+    s.ldm = c;
+    return s;
+}
+
+// What each layer reads; with `rms_dev` the input is scaled by 1/(*rms_dev).
+Src layer_input(const pps_unet* u, int l, const float* in, const float* rms_dev)
+{
+    const Acts& A = u->A;
+    const int c1 = u->c1, c2 = u->c2, c3 = u->c3;
+    switch (l) {
+    case 0: return dense(in, rms_dev);
+    case 1: return plain(A.e1a, c1);
+    case 2: return pooled(A.e1, c1);
+    case 3: return plain(A.e2a, c2);
+    case 4: return pooled(A.e2, c2);
+    case 5: return plain(A.e3a, c3);
+    case 6: return concat(A.e3, c3, A.e2, c2);
+    case 7: return plain(A.d2a, c2);
+    case 8: return concat(A.d2, c2, A.e1, c1);
+    case 9: return plain(A.d1a, c1);
+    default: return plain(A.d1, c1);
+    }
+}
+
+const Dims& layer_dims(const pps_unet* u, int l)
+{
+    return l == 4 || l == 5 ? u->A.s3 : (l == 2 || l == 3 || l == 6 || l == 7) ? u->A.s2 : u->A.s1;
+}
+
+// The forward pass: every layer one convolution, the pooling, upsampling and
+// concatenations folded into its loads.  `last` is what the last layer does with its
+// sums: the dense output, or the loss and its gradient.
+void forward(pps_unet* u, const float* in, const float* rms_dev, Epi last)
 {
     Acts& A = u->A;
-    cudaStream_t s = u->stream;
+    bf16* out[10] = {A.e1a, A.e1, A.e2a, A.e2, A.e3a, A.e3, A.d2a, A.d2, A.d1a, A.d1};
+    for (int l = 0; l < UNET_LAYERS; l++) {
+        const Layer& L = u->L[(size_t)l];
+        Epi e = last;
+        if (l < 10) {
+            e = Epi();
+            e.Y = out[l];
+            e.ld = L.cout_p;
+            e.relu = u->linear ? 0 : 1;
+        }
+        e.bias = Bf(u, l);
+        conv(layer_dims(u, l), layer_input(u, l, in, rms_dev), u->WP + L.w, L.cin_p, L.cout_p, e, u->stream);
+    }
+}
+
+// Gradients of the parameters from A.g_out, the gradient of the dense output: the data
+// gradients layer by layer (each a convolution of the output gradient G_l with the
+// mirrored weights), then all weight and bias gradients in one launch.
+void backward(pps_unet* u, const float* in)
+{
+    Acts& A = u->A;
     const int c1 = u->c1, c2 = u->c2, c3 = u->c3;
-    const long long v1 = (long long)A.s1.D * A.s1.H * A.s1.W;
     const bool R = !u->linear;
-    const bool infer = dense_out != nullptr;
-    ConvIO first, up2io, up1io, last;
-    if (infer) {
-        first.dense_in = in;
-        first.rms = rms_dev;
-        up2io.up = A.e3;
-        up2io.ld_up = c3;
-        up2io.c_up = c3;
-        up1io.up = A.d2;
-        up1io.ld_up = c2;
-        up1io.c_up = c2;
-        last.dense_out = dense_out;
-        last.rms = rms_dev;
-        last.gain = gain;
-    } else {
-        dense_to_act(v1, in, rms_dev, A.x0, 16, s);
+    const Src G[UNET_LAYERS] = {
+        plain(A.g_e1a, c1),
+        skip(A.g_cat1, c2 + c1, c2, A.g_p1, c1, R ? A.e1 : nullptr),
+        plain(A.g_e2a, c2),
+        skip(A.g_cat2, c3 + c2, c3, A.g_p2, c2, R ? A.e2 : nullptr),
+        plain(A.g_e3a, c3),
+        children(A.g_cat2, c3 + c2, R ? A.e3 : nullptr, c3),
+        plain(A.g_d2a, c2),
+        children(A.g_cat1, c2 + c1, R ? A.d2 : nullptr, c2),
+        plain(A.g_d1a, c1),
+        plain(A.g_d1, c1),
+        dense(A.g_out, nullptr),
+    };
+    // gradient of layer l's input, and the activation whose ReLU it passes (where that
+    // input is one layer's stored output)
+    bf16* gin[UNET_LAYERS] = {nullptr, A.g_e1a, A.g_p1, A.g_e2a, A.g_p2, A.g_e3a, A.g_cat2, A.g_d2a, A.g_cat1, A.g_d1a, A.g_d1};
+    const bf16* act[UNET_LAYERS] = {nullptr, A.e1a, nullptr, A.e2a, nullptr, A.e3a, nullptr, A.d2a, nullptr, A.d1a, A.d1};
+    for (int l = 10; l >= 1; l--) {
+        const Layer& L = u->L[(size_t)l];
+        Epi e;
+        e.Y = gin[l];
+        e.ld = L.cin_p;
+        e.mask = R ? act[l] : nullptr;
+        e.ldm = L.cin_p;
+        conv(layer_dims(u, l), G[l], u->WB + L.w, L.cout_p, L.cin_p, e, u->stream);
     }
-    conv(A.s1, A.x0, 16, 0, 16, Wb(u, 0), Bf(u, 0), A.e1a, c1, 0, c1, R, false, s, first);
-    conv(A.s1, A.e1a, c1, 0, c1, Wb(u, 1), Bf(u, 1), A.cat1, c2 + c1, c2, c1, R, false, s);
-    pool2(A.s2, A.cat1, c2 + c1, c2, A.p1, c1, s);
-    conv(A.s2, A.p1, c1, 0, c1, Wb(u, 2), Bf(u, 2), A.e2a, c2, 0, c2, R, false, s);
-    conv(A.s2, A.e2a, c2, 0, c2, Wb(u, 3), Bf(u, 3), A.cat2, c3 + c2, c3, c2, R, false, s);
-    pool2(A.s3, A.cat2, c3 + c2, c3, A.p2, c2, s);
-    conv(A.s3, A.p2, c2, 0, c2, Wb(u, 4), Bf(u, 4), A.e3a, c3, 0, c3, R, false, s);
-    conv(A.s3, A.e3a, c3, 0, c3, Wb(u, 5), Bf(u, 5), A.e3, c3, 0, c3, R, false, s);
-    if (!infer) up2(A.s2, A.e3, c3, A.cat2, c3 + c2, 0, s);
-    conv(A.s2, A.cat2, c3 + c2, 0, c3 + c2, Wb(u, 6), Bf(u, 6), A.d2a, c2, 0, c2, R, false, s, up2io);
-    conv(A.s2, A.d2a, c2, 0, c2, Wb(u, 7), Bf(u, 7), A.d2, c2, 0, c2, R, false, s);
-    if (!infer) up2(A.s1, A.d2, c2, A.cat1, c2 + c1, 0, s);
-    conv(A.s1, A.cat1, c2 + c1, 0, c2 + c1, Wb(u, 8), Bf(u, 8), A.d1a, c1, 0, c1, R, false, s, up1io);
-    conv(A.s1, A.d1a, c1, 0, c1, Wb(u, 9), Bf(u, 9), A.d1, c1, 0, c1, R, false, s);
-    conv(A.s1, A.d1, c1, 0, c1, Wb(u, 10), Bf(u, 10), A.out, 16, 0, 16, false, true, s, last);
-}
-
-// gradient of layer l: weights/bias from (X, G), then the data gradient Gin = conv(G, flip(W_l))
-void layer_bwd(pps_unet* u, int l, const Dims& d, const bf16* X, int ldx, int cx0, const bf16* Gv, int ldg, int cg0,
-               bf16* Gin, int ldgi, int cgi0)
-{
-    const Layer& Ly = u->L[(size_t)l];
-    cudaStream_t s = u->stream;
-    const long long nv = (long long)d.D * d.H * d.W;
-    conv_wgrad(d, X, ldx, cx0, Ly.cin_p, Gv, ldg, cg0, Ly.cout_p, u->G + Ly.w, s);
-    bias_grad(nv, Gv, ldg, cg0, Ly.cout_p, u->G + Ly.b, s);
-    if (Gin) {
-        flip(u->PB + Ly.w, u->WF, Ly.cin_p, Ly.cout_p, s);
-        conv(d, Gv, ldg, cg0, Ly.cout_p, u->WF, nullptr, Gin, ldgi, cgi0, Ly.cin_p, false, false, s);
+    WgTable T;
+    T.n = UNET_LAYERS;
+    for (int l = 0; l < UNET_LAYERS; l++) {
+        const Layer& L = u->L[(size_t)l];
+        WgLayer& W = T.L[l];
+        W.d = layer_dims(u, l);
+        W.X = layer_input(u, l, in, nullptr);
+        W.G = G[l];
+        W.Cin = L.cin_p;
+        W.Cout = L.cout_p;
+        W.dW = u->G + L.w;
+        W.db = u->G + L.b;
     }
-}
-
-void backward(pps_unet* u)
-{
-    Acts& A = u->A;
-    cudaStream_t s = u->stream;
-    const int c1 = u->c1, c2 = u->c2, c3 = u->c3;
-    const long long v1 = (long long)A.s1.D * A.s1.H * A.s1.W, v2 = v1 / 8, v3 = v2 / 8;
-    UK(cudaMemsetAsync(u->G, 0, sizeof(float) * u->npad, s));
-    // out <- d1
-    layer_bwd(u, 10, A.s1, A.d1, c1, 0, A.g_out, 16, 0, A.g_d1, c1, 0);
-    if (!u->linear) relu_bwd(v1, A.g_d1, c1, 0, A.d1, c1, 0, c1, s);
-    layer_bwd(u, 9, A.s1, A.d1a, c1, 0, A.g_d1, c1, 0, A.g_d1a, c1, 0);
-    if (!u->linear) relu_bwd(v1, A.g_d1a, c1, 0, A.d1a, c1, 0, c1, s);
-    layer_bwd(u, 8, A.s1, A.cat1, c2 + c1, 0, A.g_d1a, c1, 0, A.g_cat1, c2 + c1, 0);
-    // up slot of cat1 -> d2
-    up2_bwd(A.s2, A.g_cat1, c2 + c1, 0, A.g_d2, c2, s);
-    if (!u->linear) relu_bwd(v2, A.g_d2, c2, 0, A.d2, c2, 0, c2, s);
-    layer_bwd(u, 7, A.s2, A.d2a, c2, 0, A.g_d2, c2, 0, A.g_d2a, c2, 0);
-    if (!u->linear) relu_bwd(v2, A.g_d2a, c2, 0, A.d2a, c2, 0, c2, s);
-    layer_bwd(u, 6, A.s2, A.cat2, c3 + c2, 0, A.g_d2a, c2, 0, A.g_cat2, c3 + c2, 0);
-    // up slot of cat2 -> e3
-    up2_bwd(A.s3, A.g_cat2, c3 + c2, 0, A.g_e3, c3, s);
-    if (!u->linear) relu_bwd(v3, A.g_e3, c3, 0, A.e3, c3, 0, c3, s);
-    layer_bwd(u, 5, A.s3, A.e3a, c3, 0, A.g_e3, c3, 0, A.g_e3a, c3, 0);
-    if (!u->linear) relu_bwd(v3, A.g_e3a, c3, 0, A.e3a, c3, 0, c3, s);
-    layer_bwd(u, 4, A.s3, A.p2, c2, 0, A.g_e3a, c3, 0, A.g_p2, c2, 0);
-    // pooling -> skip slot of cat2 (adds to the skip gradient of conv6)
-    pool2_bwd(A.s3, A.g_p2, A.g_cat2, c3 + c2, c3, c2, s);
-    if (!u->linear) relu_bwd(v2, A.g_cat2, c3 + c2, c3, A.cat2, c3 + c2, c3, c2, s);
-    layer_bwd(u, 3, A.s2, A.e2a, c2, 0, A.g_cat2, c3 + c2, c3, A.g_e2a, c2, 0);
-    if (!u->linear) relu_bwd(v2, A.g_e2a, c2, 0, A.e2a, c2, 0, c2, s);
-    layer_bwd(u, 2, A.s2, A.p1, c1, 0, A.g_e2a, c2, 0, A.g_p1, c1, 0);
-    pool2_bwd(A.s2, A.g_p1, A.g_cat1, c2 + c1, c2, c1, s);
-    if (!u->linear) relu_bwd(v1, A.g_cat1, c2 + c1, c2, A.cat1, c2 + c1, c2, c1, s);
-    layer_bwd(u, 1, A.s1, A.e1a, c1, 0, A.g_cat1, c2 + c1, c2, A.g_e1a, c1, 0);
-    if (!u->linear) relu_bwd(v1, A.g_e1a, c1, 0, A.e1a, c1, 0, c1, s);
-    layer_bwd(u, 0, A.s1, A.x0, 16, 0, A.g_e1a, c1, 0, nullptr, 0, 0);
+    wgrad(T, u->stream);
 }
 
 pps_status check_dims(int nx, int ny, int nz)
@@ -290,8 +331,12 @@ pps_status pps_internal_unet_apply(pps_unet* u, int nx, int ny, int nz, const fl
         u->stream = s;
         ensure_acts(u, nx, ny, nz, false);
         const long long nv = (long long)nx * ny * nz;
-        rms(nv, in, u->dtmp, s);
-        forward(u, in, u->dtmp, out, gain);
+        rms(nv, in, u->dtmp, u->drms, s);
+        Epi last;
+        last.dense_out = out;
+        last.rms = u->dtmp;
+        last.gain = gain;
+        forward(u, in, u->dtmp, last);
         u->stream = saved;
         return PPS_OK;
     });
@@ -337,15 +382,28 @@ pps_status pps_unet_create(int c1, int c2, int c3, unsigned long long seed, int 
         UK(cudaSetDevice(device));
         u->device = device;
         UK(cudaStreamCreateWithFlags(&u->stream, cudaStreamNonBlocking));
+        UK(conv_prepare());
+        // each layer's parameters are a multiple of 16 floats, so the loss behind the
+        // gradients is 8-byte aligned
         float** f[] = {&u->P, &u->G, &u->M, &u->V};
         for (float** q : f) {
-            UK(cudaMalloc((void**)q, sizeof(float) * u->npad));
-            UK(cudaMemsetAsync(*q, 0, sizeof(float) * u->npad, u->stream));
+            UK(cudaMalloc((void**)q, sizeof(float) * u->npad + sizeof(double)));
+            UK(cudaMemsetAsync(*q, 0, sizeof(float) * u->npad + sizeof(double), u->stream));
         }
-        UK(cudaMalloc((void**)&u->PB, sizeof(bf16) * u->npad));
-        UK(cudaMalloc((void**)&u->WF, sizeof(bf16) * 27 * 96 * 96));
+        u->dloss = reinterpret_cast<double*>(u->G + u->npad);
+        for (bf16** q : {&u->WP, &u->WB}) {
+            UK(cudaMalloc((void**)q, sizeof(bf16) * u->npad));
+            UK(cudaMemsetAsync(*q, 0, sizeof(bf16) * u->npad, u->stream));
+        }
         UK(cudaMalloc((void**)&u->dtmp, sizeof(float) * 4));
-        UK(cudaMalloc((void**)&u->dloss, sizeof(double)));
+        UK(cudaMalloc((void**)&u->drms, sizeof(RmsScratch)));
+        UK(cudaMemsetAsync(u->drms, 0, sizeof(RmsScratch), u->stream));
+        u->pt.n = UNET_LAYERS;
+        for (int l = 0; l < UNET_LAYERS; l++) {
+            u->pt.w[l] = (int)u->L[(size_t)l].w;
+            u->pt.cin[l] = u->L[(size_t)l].cin_p;
+            u->pt.cout[l] = u->L[(size_t)l].cout_p;
+        }
         // He initialisation of the real weights, zero biases
         std::vector<float> h(u->npad, 0.0f);
         std::mt19937_64 rng(seed);
@@ -357,7 +415,7 @@ pps_status pps_unet_create(int c1, int c2, int c3, unsigned long long seed, int 
                         h[l.w + ((size_t)t * l.cin_p + ci) * l.cout_p + co] = nd(rng) * (l.relu ? 1.0f : 0.1f);
         }
         UK(cudaMemcpyAsync(u->P, h.data(), sizeof(float) * u->npad, cudaMemcpyHostToDevice, u->stream));
-        f32_to_bf16((long long)u->npad, u->P, u->PB, u->stream);
+        pack(u->pt, (int)u->npad, u->P, u->WP, u->WB, u->stream);
         UK(cudaStreamSynchronize(u->stream));
         return PPS_OK;
     });
@@ -375,7 +433,7 @@ pps_status pps_unet_destroy(pps_unet* u)
     cudaSetDevice(u->device);
     if (u->stream) cudaStreamSynchronize(u->stream);
     free_acts(u->A);
-    void* p[] = {u->P, u->G, u->M, u->V, u->PB, u->WF, u->dtmp, u->dloss};
+    void* p[] = {u->P, u->G, u->M, u->V, u->WP, u->WB, u->dtmp, u->drms};
     for (void* q : p)
         if (q) cudaFree(q);
     if (u->stream) cudaStreamDestroy(u->stream);
@@ -434,7 +492,7 @@ pps_status pps_unet_set_params(pps_unet* u, const float* in)
         UK(cudaMemsetAsync(u->M, 0, sizeof(float) * u->npad, u->stream));
         UK(cudaMemsetAsync(u->V, 0, sizeof(float) * u->npad, u->stream));
         u->step = 0;
-        f32_to_bf16((long long)u->npad, u->P, u->PB, u->stream);
+        pack(u->pt, (int)u->npad, u->P, u->WP, u->WB, u->stream);
         UK(cudaStreamSynchronize(u->stream));
         return PPS_OK;
     });
@@ -450,10 +508,13 @@ pps_status pps_unet_forward(pps_unet* u, int nx, int ny, int nz, const float* in
         const long long nv = (long long)nx * ny * nz;
         const float* r = nullptr;
         if (normalize) {
-            rms(nv, in_dev, u->dtmp, u->stream);
+            rms(nv, in_dev, u->dtmp, u->drms, u->stream);
             r = u->dtmp;
         }
-        forward(u, in_dev, r, out_dev, 1.0f);
+        Epi last;
+        last.dense_out = out_dev;
+        last.rms = r;
+        forward(u, in_dev, r, last);
         UK(cudaStreamSynchronize(u->stream));
         return PPS_OK;
     });
@@ -464,10 +525,14 @@ static pps_status loss_and_grads(pps_unet* u, int nx, int ny, int nz, const floa
 {
     ensure_acts(u, nx, ny, nz, true);
     const long long nv = (long long)nx * ny * nz;
-    forward(u, in, nullptr);
-    UK(cudaMemsetAsync(u->dloss, 0, sizeof(double), u->stream));
-    mse(nv, u->A.out, 16, target, u->A.g_out, 16, u->dloss, u->stream);
-    backward(u);
+    UK(cudaMemsetAsync(u->G, 0, sizeof(float) * u->npad + sizeof(double), u->stream));   // and the loss
+    Epi last;
+    last.dense_out = u->A.g_out;
+    last.target = target;
+    last.loss = u->dloss;
+    last.inv_n = (float)(1.0 / (double)nv);
+    forward(u, in, nullptr, last);
+    backward(u, in);
     UK(cudaMemcpyAsync(loss, u->dloss, sizeof(double), cudaMemcpyDeviceToHost, u->stream));
     UK(cudaStreamSynchronize(u->stream));
     return PPS_OK;
@@ -500,9 +565,9 @@ pps_status pps_unet_train_step(pps_unet* u, int nx, int ny, int nz, const float*
         pps_status rc = loss_and_grads(u, nx, ny, nz, in_dev, target_dev, loss);
         if (rc != PPS_OK) return rc;
         u->step += 1;
-        rms((long long)u->npad, u->G, u->dtmp + 1, u->stream);   // global-norm clipping at 1
-        adam((long long)u->npad, u->P, u->G, u->M, u->V, u->PB, lr, 0.9f, 0.999f, 1e-8f, u->step, u->dtmp + 1, 1.0f,
-             u->stream);
+        rms((long long)u->npad, u->G, u->dtmp + 1, u->drms, u->stream);   // global-norm clipping at 1
+        adam(u->pt, (int)u->npad, u->P, u->G, u->M, u->V, u->WP, u->WB, lr, 0.9f, 0.999f, 1e-8f, u->step, u->dtmp + 1,
+             1.0f, u->stream);
         UK(cudaStreamSynchronize(u->stream));
         return PPS_OK;
     });

@@ -19,45 +19,87 @@ struct Dims {
 // Device stop flag that the forward and transfer kernels check on entry (a set flag
 // makes them return at once); null (the default) while training or outside a solve.
 void set_stop_flag(const int* done);
+const int* stop_flag();
 
 typedef __nv_bfloat16 bf16;
 
-// Optional sources and sink of a convolution that replace the glue kernels of the
-// inference pass (each gives the values the glue kernel would have stored):
-//   dense_in: the input is a dense FP32 field scaled by 1/(*rms) (rms null: 1) in
-//             channel 0 of 16, zeros elsewhere (dense_to_act);
-//   up:       input channels [0, c_up) are the nearest 2x upsampling of `up`
-//             (coarse grid, leading dimension ld_up; up2);
-//   dense_out: channel 0 of the FP32 output, times (*rms) (rms null: 1) * gain, into
-//             a dense field instead of Y (out_to_dense).
-struct ConvIO {
-    const float* dense_in = nullptr;
+// How a convolution reads its operand: stored as it is, or made from stored tensors
+// while it is loaded, with the values the step in between would have stored.
+enum SrcKind : int {
+    SRC_PLAIN = 0,      // X, leading dimension ld, channels from c0
+    SRC_DENSE = 1,      // channel 0 = BF16(dense / (*rms)) (rms null: dense itself), zeros elsewhere
+    SRC_UP = 2,         // channels [0, c_up): nearest 2x upsampling of `up`; the others: X at c0 + c
+    SRC_POOL = 3,       // mean of the 8 fine voxels of X
+    SRC_CHILDREN = 4,   // sum of the 8 fine voxels of X (upsampling backward), kept where mask > 0
+    SRC_SKIP = 5        // X + up/8 at the coarse voxel (pooling backward onto a skip gradient), kept where mask > 0
+};
+struct Src {
+    int kind = SRC_PLAIN;
+    const bf16* X = nullptr;
+    int ld = 0, c0 = 0;
+    const float* dense = nullptr;
+    const float* rms = nullptr;
     const bf16* up = nullptr;
     int ld_up = 0, c_up = 0;
+    const bf16* mask = nullptr;   // null: no mask (identity activations)
+    int ldm = 0, cm0 = 0;
+};
+// What a convolution does with its FP32 sums: + bias, ReLU, then one of
+//   Y (BF16, kept where mask > 0 when there is a mask);
+//   dense_out = channel 0 * (*rms) * gain;
+//   with target: the MSE of channel 0, loss += (val - target)^2 / n, and its gradient
+//   2 (val - target) inv_n into dense_out.
+struct Epi {
+    bf16* Y = nullptr;
+    int ld = 0, c0 = 0;
+    const float* bias = nullptr;
+    int relu = 0;
+    const bf16* mask = nullptr;
+    int ldm = 0, cm0 = 0;
     float* dense_out = nullptr;
     const float* rms = nullptr;
     float gain = 1.0f;
+    const float* target = nullptr;
+    double* loss = nullptr;
+    float inv_n = 0.0f;
 };
+// 3x3x3 zero-padded convolution on tensor cores (Cin, Cout multiples of 16, at most
+// 96), weights packed by pack().
+void conv(const Dims& d, const Src& in, const bf16* Wpacked, int Cin, int Cout, const Epi& e, cudaStream_t s);
 
-// 3x3x3 zero-padded convolution on tensor cores (Cin, Cout multiples of 16).
-void conv(const Dims& d, const bf16* X, int ldx, int cx0, int Cin, const bf16* W, const float* bias, void* Y, int ldy,
-          int cy0, int Cout, bool relu, bool out_f32, cudaStream_t s, const ConvIO& io = ConvIO());
-void conv_wgrad(const Dims& d, const bf16* X, int ldx, int cx0, int Cin, const bf16* G, int ldg, int cg0, int Cout,
-                float* dW, cudaStream_t s);
-void bias_grad(long long nv, const bf16* G, int ldg, int cg0, int Cout, float* db, cudaStream_t s);
-void relu_bwd(long long nv, bf16* G, int ldg, int cg0, const bf16* Y, int ldy, int cy0, int C, cudaStream_t s);
-void pool2(const Dims& dout, const bf16* in, int ldi, int ci0, bf16* out, int C, cudaStream_t s);
-void pool2_bwd(const Dims& dout, const bf16* gout, bf16* gin, int ldi, int ci0, int C, cudaStream_t s);
-void up2(const Dims& dfine, const bf16* in, int C, bf16* out, int ldo, int co0, cudaStream_t s);
-void up2_bwd(const Dims& dcoarse, const bf16* gout, int ldo, int co0, bf16* gin, int C, cudaStream_t s);
-void flip(const bf16* W, bf16* Wf, int Cin, int Cout, cudaStream_t s);
-void mse(long long nv, const float* out, int ldo, const float* t, bf16* G, int ldg, double* loss, cudaStream_t s);
-void adam(long long n, float* p, const float* g, float* m, float* v, bf16* pb, float lr, float b1, float b2, float eps,
-          int step, const float* g_rms, float max_norm, cudaStream_t s);
-void f32_to_bf16(long long n, const float* a, bf16* b, cudaStream_t s);
-void dense_to_act(long long nv, const float* in, const float* rms, bf16* act, int ld, cudaStream_t s);
-void out_to_dense(long long nv, const float* out, int ld, const float* rms, float gain, float* dense, cudaStream_t s);
-void rms(long long n, const float* a, float* out, cudaStream_t s);
+// Weight and bias gradients of up to 11 layers in one launch (dW, db are added to).
+struct WgLayer {
+    Dims d;
+    Src X, G;
+    int Cin, Cout;
+    float *dW, *db;
+    // filled by wgrad()
+    int lx, ly, ntx, nty, ntz, tiles_per_block, kblocks, first;
+};
+constexpr int UNET_LAYERS = 11;
+struct WgTable {
+    WgLayer L[UNET_LAYERS];
+    int n;
+};
+void wgrad(WgTable& T, cudaStream_t s);
+
+// Layout of the padded parameter array: W of layer l at w[l], 27 * cin * cout long,
+// followed by its bias.
+struct PackTable {
+    int n;
+    int w[UNET_LAYERS], cin[UNET_LAYERS], cout[UNET_LAYERS];
+};
+// BF16 weights in fragment order for the convolutions (fwd) and their data gradients (bwd)
+void pack(const PackTable& T, int n, const float* p, bf16* fwd, bf16* bwd, cudaStream_t s);
+void adam(const PackTable& T, int n, float* p, const float* g, float* m, float* v, bf16* fwd, bf16* bwd, float lr,
+          float b1, float b2, float eps, int step, const float* g_rms, float max_norm, cudaStream_t s);
+struct RmsScratch {
+    double part[256];
+    unsigned count;   // zero between launches
+};
+void rms(long long n, const float* a, float* out, RmsScratch* scratch, cudaStream_t s);
+// Lets the convolution kernels use the shared memory their tiles take (current device).
+cudaError_t conv_prepare();
 
 // Solver field (guard-padded, Dirichlet unknowns) <-> dense unknown arrays.
 template <typename T>

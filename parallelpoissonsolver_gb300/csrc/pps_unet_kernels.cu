@@ -1,12 +1,6 @@
-// Kernels of the learned preconditioner: a 3-D convolutional U-Net with BF16 weights
-// and activations and FP32 accumulation, plus the grid-transfer kernels that move a
-// solver field to the network's grid and back.  No reference counterpart.
-//
-// Activations are channels-last: act[((z*H + y)*W + x)*ld + c0 + c], BF16, where a
-// tensor may occupy a channel slot [c0, c0+C) of a wider buffer (the U-Net's skip
-// concatenations).  Convolutions are 3x3x3, zero-padded, stride 1, as implicit
-// GEMMs on the tensor cores: M = voxels, N = output channels, K = 27 taps x input
-// channels, 16x16x16 BF16 fragments with FP32 accumulators.
+// Kernels of the learned preconditioner around its network (pps_unet_conv.cu): the
+// grid transfers that move a solver field to the network's grid and back, and the
+// coarse levels of the multigrid cycle.  No reference counterpart.
 #include "pps_unet_internal.h"
 #include "pps_reduce.cuh"
 
@@ -14,9 +8,7 @@
 #include <cmath>
 #include <type_traits>
 
-#include <cuda_bf16.h>
 #include <cuda_runtime.h>
-#include <mma.h>
 
 namespace pps {
 namespace unet {
@@ -26,264 +18,7 @@ namespace unet {
 // replayed) after the iteration converged costs no more than its launches.
 static thread_local const int* g_stop = nullptr;
 void set_stop_flag(const int* done) { g_stop = done; }
-
-using namespace nvcuda;
-typedef __nv_bfloat16 bf16;
-
-constexpr int TILE_V = 64;   // voxels (along x) per conv block: 4 warps x 16
-
-// ---------------------------------------------------------------------------
-// Convolution, forward: Y[v][co] = act(bias[co] + sum_tap sum_ci X[v+off(tap)][ci] W[tap][ci][co])
-// Cin, Cout multiples of 16.  One block: one 16 x 16 output fragment (16 consecutive
-// voxels in (z, y, x) order, 16 output channels).  The K = 27 * Cin/16 steps of
-// 16 x 16 x 16 are dealt round-robin to the NW warps, so each warp's dependent chain
-// is 1/NW of K (the grids are small: at 16^3 and below latency, not the tensor pipe,
-// is the limit; the deep layers run 54-162 steps on 16-64 blocks).  Each warp stages
-// its A tile in its own shared slot (warp-level sync only) and prefetches the next
-// step's A tile and weight fragment into registers while the current step's
-// multiply-add runs; the NW partial fragments are summed at the end.
-// ---------------------------------------------------------------------------
-constexpr int CONV_V = 16;   // voxels per block
-
-template <bool RELU, bool OUT_F32, int NW>
-__global__ void __launch_bounds__(32 * NW) k_conv(Dims d, const bf16* __restrict__ X, int ldx, int cx0, int Cin,
-                                                  const bf16* __restrict__ Wt, const float* __restrict__ bias,
-                                                  void* __restrict__ Yv, int ldy, int cy0, int Cout,
-                                                  const int* __restrict__ stop, ConvIO io)
-{
-    pdl_enter();
-    if (stop && *(volatile const int*)stop) return;
-    __shared__ __align__(32) bf16 sA[NW][CONV_V * 16];
-    __shared__ __align__(32) float sC[NW][16 * 16];
-    const long long nvox = (long long)d.D * d.H * d.W;
-    const long long v0 = (long long)blockIdx.x * CONV_V;
-    const int co0 = blockIdx.y * 16;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // this lane's voxel row of the A tile and its 8-channel half
-    const int va = lane >> 1, ha = lane & 1;
-    const long long lva = v0 + va;
-    const bool va_in = lva < nvox;
-    const int xa = (int)(lva % d.W), ya = (int)((lva / d.W) % d.H), za = (int)(lva / ((long long)d.W * d.H));
-    const int csteps = Cin / 16, ksteps = 27 * csteps;
-    const float in_sc = io.dense_in && io.rms ? (*io.rms > 0.0f ? 1.0f / *io.rms : 0.0f) : 1.0f;
-    const int Hc = d.H / 2, Wc = d.W / 2;
-    auto load_a = [&](int t) -> uint4 {
-        const int tap = t / csteps, c0 = (t - tap * csteps) * 16;
-        const int zz = za + tap / 9 - 1, yy = ya + (tap / 3) % 3 - 1, xx = xa + tap % 3 - 1;
-        uint4 val = make_uint4(0, 0, 0, 0);
-        if (va_in && zz >= 0 && zz < d.D && yy >= 0 && yy < d.H && xx >= 0 && xx < d.W) {
-            const long long vox = ((long long)zz * d.H + yy) * d.W + xx;
-            if (io.dense_in) {   // channel 0 of the first 16 (Cin = 16): the scaled dense input
-                if (ha == 0) val.x = (unsigned)__bfloat16_as_ushort(__float2bfloat16(io.dense_in[vox] * in_sc));
-            } else if (c0 < io.c_up) {   // the upsampled channels, read at the coarse voxel
-                const long long cv = ((long long)(zz >> 1) * Hc + (yy >> 1)) * Wc + (xx >> 1);
-                val = *reinterpret_cast<const uint4*>(io.up + cv * io.ld_up + c0 + 8 * ha);
-            } else {
-                val = *reinterpret_cast<const uint4*>(X + vox * ldx + cx0 + c0 + 8 * ha);
-            }
-        }
-        return val;
-    };
-    auto w_at = [&](int t) {
-        const int tap = t / csteps, c0 = (t - tap * csteps) * 16;
-        return Wt + ((long long)tap * Cin + c0) * Cout + co0;
-    };
-    wmma::fragment<wmma::accumulator, 16, 16, 16, float> acc;
-    wmma::fill_fragment(acc, 0.0f);
-    wmma::fragment<wmma::matrix_b, 16, 16, 16, bf16, wmma::row_major> bcur, bnext;
-    int t = warp;
-    uint4 next = t < ksteps ? load_a(t) : make_uint4(0, 0, 0, 0);
-    if (t < ksteps) wmma::load_matrix_sync(bnext, w_at(t), Cout);
-    for (; t < ksteps; t += NW) {
-        *reinterpret_cast<uint4*>(&sA[warp][va * 16 + 8 * ha]) = next;
-        bcur = bnext;
-        __syncwarp();
-        if (t + NW < ksteps) {
-            next = load_a(t + NW);
-            wmma::load_matrix_sync(bnext, w_at(t + NW), Cout);
-        }
-        wmma::fragment<wmma::matrix_a, 16, 16, 16, bf16, wmma::row_major> a;
-        wmma::load_matrix_sync(a, sA[warp], 16);
-        wmma::mma_sync(acc, a, bcur, acc);
-        __syncwarp();
-    }
-    wmma::store_matrix_sync(sC[warp], acc, 16, wmma::mem_row_major);
-    __syncthreads();
-    for (int q = threadIdx.x; q < CONV_V * 16; q += 32 * NW) {
-        const int v = q >> 4, co = q & 15;
-        if (v0 + v >= nvox) continue;
-        float val = 0.0f;
-#pragma unroll
-        for (int w = 0; w < NW; w++) val += sC[w][q];
-        val += bias ? bias[co0 + co] : 0.0f;
-        if (RELU) val = fmaxf(val, 0.0f);
-        if (io.dense_out) {   // channel 0 only, scaled back
-            if (co0 + co == 0) io.dense_out[v0 + v] = val * ((io.rms ? *io.rms : 1.0f) * io.gain);
-            continue;
-        }
-        const long long o = (v0 + v) * ldy + cy0 + co0 + co;
-        if (OUT_F32) reinterpret_cast<float*>(Yv)[o] = val;
-        else reinterpret_cast<bf16*>(Yv)[o] = __float2bfloat16(val);
-    }
-}
-
-template <int NW>
-static void conv_nw(const dim3& grid, const Dims& d, const bf16* X, int ldx, int cx0, int Cin, const bf16* W,
-                    const float* bias, void* Y, int ldy, int cy0, int Cout, bool relu, bool out_f32, cudaStream_t s,
-                    const ConvIO& io)
-{
-    const dim3 block(32 * NW);
-    if (out_f32) {
-        if (relu) launch_pdl(k_conv<true, true, NW>, grid, block, 0, s, d, X, ldx, cx0, Cin, W, bias, Y, ldy, cy0, Cout, g_stop, io);
-        else launch_pdl(k_conv<false, true, NW>, grid, block, 0, s, d, X, ldx, cx0, Cin, W, bias, Y, ldy, cy0, Cout, g_stop, io);
-    } else {
-        if (relu) launch_pdl(k_conv<true, false, NW>, grid, block, 0, s, d, X, ldx, cx0, Cin, W, bias, Y, ldy, cy0, Cout, g_stop, io);
-        else launch_pdl(k_conv<false, false, NW>, grid, block, 0, s, d, X, ldx, cx0, Cin, W, bias, Y, ldy, cy0, Cout, g_stop, io);
-    }
-}
-
-void conv(const Dims& d, const bf16* X, int ldx, int cx0, int Cin, const bf16* W, const float* bias, void* Y, int ldy,
-          int cy0, int Cout, bool relu, bool out_f32, cudaStream_t s, const ConvIO& io)
-{
-    const dim3 grid((unsigned)(((long long)d.D * d.H * d.W + CONV_V - 1) / CONV_V), (unsigned)(Cout / 16));
-    // warps per block: enough that each warp's chain of K steps stays short
-    const int ksteps = 27 * (Cin / 16);
-    if (ksteps >= 64) conv_nw<16>(grid, d, X, ldx, cx0, Cin, W, bias, Y, ldy, cy0, Cout, relu, out_f32, s, io);
-    else conv_nw<8>(grid, d, X, ldx, cx0, Cin, W, bias, Y, ldy, cy0, Cout, relu, out_f32, s, io);
-    launches_counter_add(1);
-}
-
-// ---------------------------------------------------------------------------
-// Weight gradient: dW[tap][ci][co] += sum_v X[v+off(tap)][ci] * dY[v][co]
-// One block per (tap, z-plane): a GEMM with K = the plane's voxels, accumulated in
-// fragments and added to the FP32 gradient with atomics.
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) k_conv_wgrad(Dims d, const bf16* __restrict__ X, int ldx, int cx0, int Cin,
-                                                    const bf16* __restrict__ G, int ldg, int cg0, int Cout,
-                                                    float* __restrict__ dW)
-{
-    pdl_enter();
-    __shared__ __align__(32) bf16 sX[TILE_V * 96];    // 64 voxels x Cin   (col-major A: ci x v)
-    __shared__ __align__(32) bf16 sG[TILE_V * 96];    // 64 voxels x Cout  (row-major B: v x co)
-    __shared__ __align__(32) float sC[96 * 96 / 4];   // staging of one warp's fragments
-    const int tap = blockIdx.x % 27;
-    const int z = blockIdx.x / 27;
-    const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const int mi = Cin / 16, ni = Cout / 16, nf = mi * ni;   // fragment pairs, split over warps
-    wmma::fragment<wmma::accumulator, 16, 16, 16, float> acc[9];
-#pragma unroll
-    for (int f = 0; f < 9; f++) wmma::fill_fragment(acc[f], 0.0f);
-    const int zz = z + dz;
-    const bool plane_ok = zz >= 0 && zz < d.D;
-    if (plane_ok) {
-        const int ntx = (d.W + TILE_V - 1) / TILE_V;
-        for (int y = 0; y < d.H; y++) {
-            const int yy = y + dy;
-            const bool row_ok = yy >= 0 && yy < d.H;
-            if (!row_ok) continue;
-            for (int xt = 0; xt < ntx; xt++) {
-                const int x0 = xt * TILE_V;
-                for (int q = tid; q < TILE_V * Cin / 8; q += 128) {
-                    const int v = q / (Cin / 8), c8 = q % (Cin / 8);
-                    const int xx = x0 + v + dx;
-                    uint4 val = make_uint4(0, 0, 0, 0);
-                    if (x0 + v < d.W && xx >= 0 && xx < d.W)
-                        val = *reinterpret_cast<const uint4*>(X + ((long long)(zz * d.H + yy) * d.W + xx) * ldx + cx0 + 8 * c8);
-                    *reinterpret_cast<uint4*>(&sX[v * 96 + 8 * c8]) = val;
-                }
-                for (int q = tid; q < TILE_V * Cout / 8; q += 128) {
-                    const int v = q / (Cout / 8), c8 = q % (Cout / 8);
-                    uint4 val = make_uint4(0, 0, 0, 0);
-                    if (x0 + v < d.W)
-                        val = *reinterpret_cast<const uint4*>(G + ((long long)(z * d.H + y) * d.W + x0 + v) * ldg + cg0 + 8 * c8);
-                    *reinterpret_cast<uint4*>(&sG[v * 96 + 8 * c8]) = val;
-                }
-                __syncthreads();
-                for (int k = 0; k < TILE_V; k += 16) {
-#pragma unroll
-                    for (int f = 0; f < 9; f++) {
-                        const int pair = warp + 4 * f;
-                        if (pair < nf) {
-                            const int m = pair / ni, n = pair % ni;
-                            wmma::fragment<wmma::matrix_a, 16, 16, 16, bf16, wmma::col_major> a;
-                            wmma::fragment<wmma::matrix_b, 16, 16, 16, bf16, wmma::row_major> b;
-                            wmma::load_matrix_sync(a, sX + k * 96 + m * 16, 96);
-                            wmma::load_matrix_sync(b, sG + k * 96 + n * 16, 96);
-                            wmma::mma_sync(acc[f], a, b, acc[f]);
-                        }
-                    }
-                }
-                __syncthreads();
-            }
-        }
-    }
-    // accumulate into dW[tap][ci][co], one warp at a time through the staging tile
-    for (int w = 0; w < 4; w++) {
-        if (warp == w) {
-#pragma unroll
-            for (int f = 0; f < 9; f++) {
-                const int pair = warp + 4 * f;
-                if (pair < nf) {
-                    const int m = pair / ni, n = pair % ni;
-                    wmma::store_matrix_sync(sC, acc[f], 16, wmma::mem_row_major);
-                    __syncwarp();
-                    for (int q = tid & 31; q < 256; q += 32) {
-                        const int r = q / 16, c = q % 16;
-                        const float v = sC[q];
-                        if (v != 0.0f) atomicAdd(&dW[((long long)tap * Cin + m * 16 + r) * Cout + n * 16 + c], v);
-                    }
-                    __syncwarp();
-                }
-            }
-        }
-        __syncthreads();
-    }
-}
-
-void conv_wgrad(const Dims& d, const bf16* X, int ldx, int cx0, int Cin, const bf16* G, int ldg, int cg0, int Cout,
-                float* dW, cudaStream_t s)
-{
-    launch_pdl(k_conv_wgrad, (unsigned)(27 * d.D), 128, 0, s, d, X, ldx, cx0, Cin, G, ldg, cg0, Cout, dW);
-    launches_counter_add(1);
-}
-
-// db[co] += sum_v G[v][co]
-__global__ void k_bias_grad(long long nv, const bf16* __restrict__ G, int ldg, int cg0, int Cout, float* __restrict__ db)
-{
-    pdl_enter();
-    __shared__ float s[96];
-    for (int c = threadIdx.x; c < Cout; c += blockDim.x) s[c] = 0.0f;
-    __syncthreads();
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < nv * Cout;
-         q += (long long)gridDim.x * blockDim.x) {
-        const long long v = q / Cout;
-        const int c = (int)(q % Cout);
-        atomicAdd(&s[c], __bfloat162float(G[v * ldg + cg0 + c]));
-    }
-    __syncthreads();
-    for (int c = threadIdx.x; c < Cout; c += blockDim.x) atomicAdd(&db[c], s[c]);
-}
-
-void bias_grad(long long nv, const bf16* G, int ldg, int cg0, int Cout, float* db, cudaStream_t s)
-{
-    long long blocks = (nv * Cout + 255) / 256;
-    if (blocks > 1024) blocks = 1024;
-    launch_pdl(k_bias_grad, (unsigned)blocks, 256, 0, s, nv, G, ldg, cg0, Cout, db);
-    launches_counter_add(1);
-}
-
-// G[v][c] *= (Y[v][c] > 0): ReLU backward through the layer's own output.
-__global__ void k_relu_bwd(long long nv, bf16* __restrict__ G, int ldg, int cg0, const bf16* __restrict__ Y, int ldy,
-                           int cy0, int C)
-{
-    pdl_enter();
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < nv * C; q += (long long)gridDim.x * blockDim.x) {
-        const long long v = q / C;
-        const int c = (int)(q % C);
-        if (!(__bfloat162float(Y[v * ldy + cy0 + c]) > 0.0f)) G[v * ldg + cg0 + c] = __float2bfloat16(0.0f);
-    }
-}
+const int* stop_flag() { return g_stop; }
 
 static unsigned eblocks(long long n)
 {
@@ -291,257 +26,6 @@ static unsigned eblocks(long long n)
     if (b > sm_count() * 32LL) b = sm_count() * 32LL;
     if (b < 1) b = 1;
     return (unsigned)b;
-}
-
-void relu_bwd(long long nv, bf16* G, int ldg, int cg0, const bf16* Y, int ldy, int cy0, int C, cudaStream_t s)
-{
-    launch_pdl(k_relu_bwd, eblocks(nv * C), 256, 0, s, nv, G, ldg, cg0, Y, ldy, cy0, C);
-    launches_counter_add(1);
-}
-
-// 2x average pooling: out (D/2,H/2,W/2) dense C channels <- in slot of ldi
-__global__ void k_pool2(Dims dout, const bf16* __restrict__ in, int ldi, int ci0, bf16* __restrict__ out, int C, const int* __restrict__ stop)
-{
-    pdl_enter();
-    if (stop && *(volatile const int*)stop) return;
-    const long long n = (long long)dout.D * dout.H * dout.W * C;
-    const int Hi = dout.H * 2, Wi = dout.W * 2;
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(q % C);
-        const long long v = q / C;
-        const int x = (int)(v % dout.W), y = (int)((v / dout.W) % dout.H), z = (int)(v / ((long long)dout.W * dout.H));
-        float s = 0.0f;
-        for (int o = 0; o < 8; o++) {
-            const int zz = 2 * z + (o >> 2), yy = 2 * y + ((o >> 1) & 1), xx = 2 * x + (o & 1);
-            s += __bfloat162float(in[((long long)(zz * Hi + yy) * Wi + xx) * ldi + ci0 + c]);
-        }
-        out[q] = __float2bfloat16(0.125f * s);
-    }
-}
-
-void pool2(const Dims& dout, const bf16* in, int ldi, int ci0, bf16* out, int C, cudaStream_t s)
-{
-    launch_pdl(k_pool2, eblocks((long long)dout.D * dout.H * dout.W * C), 256, 0, s, dout, in, ldi, ci0, out, C, g_stop);
-    launches_counter_add(1);
-}
-
-// pooling backward: gin slot (fine) += g_out/8 at each of the 8 children
-__global__ void k_pool2_bwd(Dims dout, const bf16* __restrict__ gout, bf16* __restrict__ gin, int ldi, int ci0, int C)
-{
-    pdl_enter();
-    const int Hi = dout.H * 2, Wi = dout.W * 2;
-    const long long n = (long long)dout.D * 8 * dout.H * dout.W * C;
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(q % C);
-        const long long vf = q / C;
-        const int xx = (int)(vf % Wi), yy = (int)((vf / Wi) % Hi), zz = (int)(vf / ((long long)Wi * Hi));
-        const long long vc = ((long long)(zz / 2) * dout.H + yy / 2) * dout.W + xx / 2;
-        bf16* p = gin + vf * ldi + ci0 + c;
-        *p = __float2bfloat16(__bfloat162float(*p) + 0.125f * __bfloat162float(gout[vc * C + c]));
-    }
-}
-
-void pool2_bwd(const Dims& dout, const bf16* gout, bf16* gin, int ldi, int ci0, int C, cudaStream_t s)
-{
-    launch_pdl(k_pool2_bwd, eblocks((long long)dout.D * 8 * dout.H * dout.W * C), 256, 0, s, dout, gout, gin, ldi, ci0, C);
-    launches_counter_add(1);
-}
-
-// nearest 2x upsampling: out slot (fine) <- in dense (coarse)
-__global__ void k_up2(Dims dfine, const bf16* __restrict__ in, int C, bf16* __restrict__ out, int ldo, int co0, const int* __restrict__ stop)
-{
-    pdl_enter();
-    if (stop && *(volatile const int*)stop) return;
-    const long long n = (long long)dfine.D * dfine.H * dfine.W * C;
-    const int Hc = dfine.H / 2, Wc = dfine.W / 2;
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(q % C);
-        const long long v = q / C;
-        const int x = (int)(v % dfine.W), y = (int)((v / dfine.W) % dfine.H), z = (int)(v / ((long long)dfine.W * dfine.H));
-        out[v * ldo + co0 + c] = in[((long long)(z / 2) * Hc + y / 2) * Wc * C + (long long)(x / 2) * C + c];
-    }
-}
-
-void up2(const Dims& dfine, const bf16* in, int C, bf16* out, int ldo, int co0, cudaStream_t s)
-{
-    launch_pdl(k_up2, eblocks((long long)dfine.D * dfine.H * dfine.W * C), 256, 0, s, dfine, in, C, out, ldo, co0, g_stop);
-    launches_counter_add(1);
-}
-
-// upsampling backward: gin (coarse dense) = sum of the 8 children of gout's slot
-__global__ void k_up2_bwd(Dims dcoarse, const bf16* __restrict__ gout, int ldo, int co0, bf16* __restrict__ gin, int C)
-{
-    pdl_enter();
-    const long long n = (long long)dcoarse.D * dcoarse.H * dcoarse.W * C;
-    const int Hf = dcoarse.H * 2, Wf = dcoarse.W * 2;
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(q % C);
-        const long long v = q / C;
-        const int x = (int)(v % dcoarse.W), y = (int)((v / dcoarse.W) % dcoarse.H),
-                  z = (int)(v / ((long long)dcoarse.W * dcoarse.H));
-        float s = 0.0f;
-        for (int o = 0; o < 8; o++) {
-            const int zz = 2 * z + (o >> 2), yy = 2 * y + ((o >> 1) & 1), xx = 2 * x + (o & 1);
-            s += __bfloat162float(gout[((long long)(zz * Hf + yy) * Wf + xx) * ldo + co0 + c]);
-        }
-        gin[q] = __float2bfloat16(s);
-    }
-}
-
-void up2_bwd(const Dims& dcoarse, const bf16* gout, int ldo, int co0, bf16* gin, int C, cudaStream_t s)
-{
-    launch_pdl(k_up2_bwd, eblocks((long long)dcoarse.D * dcoarse.H * dcoarse.W * C), 256, 0, s, dcoarse, gout, ldo, co0, gin, C);
-    launches_counter_add(1);
-}
-
-// Wf[tap'][co][ci] = W[26-tap][ci][co]: the weights of the backward-data convolution.
-__global__ void k_flip(const bf16* __restrict__ W, bf16* __restrict__ Wf, int Cin, int Cout)
-{
-    pdl_enter();
-    const int n = 27 * Cin * Cout;
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
-        const int co = q % Cout, ci = (q / Cout) % Cin, tap = q / (Cout * Cin);
-        Wf[((long long)(26 - tap) * Cout + co) * Cin + ci] = W[q];
-    }
-}
-
-void flip(const bf16* W, bf16* Wf, int Cin, int Cout, cudaStream_t s)
-{
-    launch_pdl(k_flip, (27 * Cin * Cout + 255) / 256, 256, 0, s, W, Wf, Cin, Cout);
-    launches_counter_add(1);
-}
-
-// MSE on channel 0 of an FP32 output slab [v][ld]: loss += sum (o - t)^2 / n,
-// gradient G[v][0] = 2 (o - t) / n, other channels 0.
-__global__ void k_mse(long long nv, const float* __restrict__ out, int ldo, const float* __restrict__ t,
-                      bf16* __restrict__ G, int ldg, double* loss)
-{
-    pdl_enter();
-    double s = 0.0;
-    const float inv = (float)(1.0 / (double)nv);
-    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < nv; v += (long long)gridDim.x * blockDim.x) {
-        const float e = out[v * ldo] - t[v];
-        s += (double)e * (double)e;
-        G[v * ldg] = __float2bfloat16(2.0f * e * inv);
-        for (int c = 1; c < ldg; c++) G[v * ldg + c] = __float2bfloat16(0.0f);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, s / (double)nv);
-}
-
-void mse(long long nv, const float* out, int ldo, const float* t, bf16* G, int ldg, double* loss, cudaStream_t s)
-{
-    launch_pdl(k_mse, eblocks(nv), 256, 0, s, nv, out, ldo, t, G, ldg, loss);
-    launches_counter_add(1);
-}
-
-// Adam on FP32 master parameters; refreshes the BF16 copy of the weights.  The
-// gradient is first scaled by min(1, max_norm / ||g||) (global-norm clipping), with
-// ||g|| = (*g_rms) * sqrt(n) from k_rms.
-__global__ void k_adam(long long n, float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
-                       float* __restrict__ v, bf16* __restrict__ pb, float lr, float b1, float b2, float eps, float c1,
-                       float c2, const float* g_rms, float max_norm)
-{
-    pdl_enter();
-    float clip = 1.0f;
-    if (g_rms) {
-        const float norm = *g_rms * sqrtf((float)n);
-        if (norm > max_norm && norm > 0.0f) clip = max_norm / norm;
-    }
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
-        const float gq = g[q] * clip;
-        const float mq = b1 * m[q] + (1.0f - b1) * gq;
-        const float vq = b2 * v[q] + (1.0f - b2) * gq * gq;
-        m[q] = mq;
-        v[q] = vq;
-        const float upd = lr * (mq / c1) / (sqrtf(vq / c2) + eps);
-        const float pn = p[q] - upd;
-        p[q] = pn;
-        if (pb) pb[q] = __float2bfloat16(pn);
-    }
-}
-
-void adam(long long n, float* p, const float* g, float* m, float* v, bf16* pb, float lr, float b1, float b2, float eps,
-          int step, const float* g_rms, float max_norm, cudaStream_t s)
-{
-    const float c1 = 1.0f - powf(b1, (float)step), c2 = 1.0f - powf(b2, (float)step);
-    launch_pdl(k_adam, eblocks(n), 256, 0, s, n, p, g, m, v, pb, lr, b1, b2, eps, c1, c2, g_rms, max_norm);
-    launches_counter_add(1);
-}
-
-__global__ void k_f32_to_bf16(long long n, const float* __restrict__ a, bf16* __restrict__ b)
-{
-    pdl_enter();
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
-        b[q] = __float2bfloat16(a[q]);
-}
-
-void f32_to_bf16(long long n, const float* a, bf16* b, cudaStream_t s)
-{
-    launch_pdl(k_f32_to_bf16, eblocks(n), 256, 0, s, n, a, b);
-    launches_counter_add(1);
-}
-
-// Dense FP32 input [v] -> channel 0 of a BF16 activation [v][ld], scaled by 1/(*rms)
-// (rms == nullptr: scale 1); the other channels zero.
-__global__ void k_dense_to_act(long long nv, const float* __restrict__ in, const float* rms, bf16* __restrict__ act, int ld, const int* __restrict__ stop)
-{
-    pdl_enter();
-    if (stop && *(volatile const int*)stop) return;
-    const float sc = rms ? (*rms > 0.0f ? 1.0f / *rms : 0.0f) : 1.0f;
-    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < nv; v += (long long)gridDim.x * blockDim.x) {
-        act[v * ld] = __float2bfloat16(in[v] * sc);
-        for (int c = 1; c < ld; c++) act[v * ld + c] = __float2bfloat16(0.0f);
-    }
-}
-
-void dense_to_act(long long nv, const float* in, const float* rms, bf16* act, int ld, cudaStream_t s)
-{
-    launch_pdl(k_dense_to_act, eblocks(nv), 256, 0, s, nv, in, rms, act, ld, g_stop);
-    launches_counter_add(1);
-}
-
-// channel 0 of an FP32 output slab -> dense FP32, times (*rms) * gain
-__global__ void k_out_to_dense(long long nv, const float* __restrict__ out, int ld, const float* rms, float gain,
-                               float* __restrict__ dense, const int* __restrict__ stop)
-{
-    pdl_enter();
-    if (stop && *(volatile const int*)stop) return;
-    const float sc = (rms ? *rms : 1.0f) * gain;
-    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < nv; v += (long long)gridDim.x * blockDim.x)
-        dense[v] = out[v * ld] * sc;
-}
-
-void out_to_dense(long long nv, const float* out, int ld, const float* rms, float gain, float* dense, cudaStream_t s)
-{
-    launch_pdl(k_out_to_dense, eblocks(nv), 256, 0, s, nv, out, ld, rms, gain, dense, g_stop);
-    launches_counter_add(1);
-}
-
-// rms of a dense FP32 array into *rms (single block, deterministic)
-__global__ void k_rms(long long n, const float* __restrict__ a, float* rms, const int* __restrict__ stop)
-{
-    pdl_enter();
-    if (stop && *(volatile const int*)stop) return;
-    __shared__ double sm[32];
-    double s = 0.0;
-    for (long long q = threadIdx.x; q < n; q += blockDim.x) s += (double)a[q] * (double)a[q];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += sm[w];
-        *rms = (float)sqrt(t / (double)(n > 0 ? n : 1));
-    }
-}
-
-void rms(long long n, const float* a, float* out, cudaStream_t s)
-{
-    launch_pdl(k_rms, 1, 1024, 0, s, n, a, out, g_stop);
-    launches_counter_add(1);
 }
 
 // ---------------------------------------------------------------------------

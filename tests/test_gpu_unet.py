@@ -47,6 +47,43 @@ def test_unet_forward_and_gradients_match_cpu_autograd(gpu):
     net.close()
 
 
+@pytest.mark.parametrize("linear", [False, True])
+@pytest.mark.parametrize("shape", [(4, 4, 4),        # one voxel on the deepest level
+                                   (12, 20, 36),     # 16-voxel blocks, ragged rows on every level
+                                   (36, 44, 52),     # 256-voxel tiles, ragged along each axis
+                                   (128, 60, 8),     # 8 x 8 x 4 tiles, then 4 x 8 x 8
+                                   (124, 64, 4)])    # 4 x 8 x 8 tiles on a 4-wide grid
+def test_unet_kernels_at_tile_edges(gpu, shape, linear):
+    """Forward, loss and gradients at the sizes where the convolution kernels' blocks and
+    tiles end raggedly, with the tolerances of the test above (BF16 weights and activations)."""
+    import unet_reference as R
+    ch = (16, 32, 64)
+    net = pps.UNet(ch, seed=11, linear=linear)
+    params = net.get_params()
+    rng = np.random.default_rng(int(np.prod(shape)))
+    x = rng.standard_normal(shape).astype(np.float32)
+    t = rng.standard_normal(shape).astype(np.float32)
+    xd, td, od = dev(x), dev(t), dev(np.full(shape, np.nan))
+    net.forward(shape, xd.data_ptr(), od.data_ptr(), normalize=False)
+    layers = R.unflatten(params, ch, bf16_weights=True)
+    relu = R.F.relu
+    if linear:
+        R.F.relu = lambda y: y
+    try:
+        out = R.forward(layers, torch.tensor(x, dtype=torch.float64))
+    finally:
+        R.F.relu = relu
+    loss_ref = torch.mean((out - torch.tensor(t, dtype=torch.float64)) ** 2)
+    loss_ref.backward()
+    g_ref, out_ref, loss_ref = R.flatten_grads(layers), out.detach().numpy(), float(loss_ref.detach())
+    out = od.cpu().numpy()
+    assert np.linalg.norm(out - out_ref) <= 0.03 * np.linalg.norm(out_ref)
+    loss, g = net.gradients(shape, xd.data_ptr(), td.data_ptr())
+    assert abs(loss - loss_ref) <= 0.02 * loss_ref
+    assert np.linalg.norm(g - g_ref) <= 0.06 * np.linalg.norm(g_ref)
+    net.close()
+
+
 def test_unet_training_lowers_the_loss(gpu):
     net = pps.UNet((16, 32, 64), seed=3)
     shape = (16, 16, 16)
