@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <random>
 #include <string>
@@ -58,11 +59,11 @@ struct Acts {
     Dims s1{0, 0, 0}, s2{0, 0, 0}, s3{0, 0, 0};   // grid of each level
     bf16 *e1a = nullptr, *e1 = nullptr, *d1a = nullptr, *d1 = nullptr;
     bf16 *e2a = nullptr, *e2 = nullptr, *d2a = nullptr, *d2 = nullptr;
-    bf16 *e3a = nullptr, *e3 = nullptr;
-    // gradients: of the outputs of layers 9, 8, 6, 4, 2, 0 (masked where stored), of the
-    // two concatenations and the two pooled tensors, and of the dense output
+    bf16 *e3a = nullptr, *e3 = nullptr, *p1 = nullptr, *p2 = nullptr;   // p: pooled e1, e2
+    // gradients: of the outputs of layers 9, 8, 7, 6, 5, 4, 2, 0 (masked where stored), of
+    // the two concatenations and the two pooled tensors, and of the dense output
     bf16 *g_d1 = nullptr, *g_d1a = nullptr, *g_cat1 = nullptr, *g_d2a = nullptr, *g_cat2 = nullptr, *g_e3a = nullptr,
-         *g_p2 = nullptr, *g_e2a = nullptr, *g_p1 = nullptr, *g_e1a = nullptr;
+         *g_p2 = nullptr, *g_e2a = nullptr, *g_p1 = nullptr, *g_e1a = nullptr, *g_d2 = nullptr, *g_e3 = nullptr;
     float* g_out = nullptr;
     bool grads = false;
 };
@@ -84,14 +85,18 @@ struct pps_unet {
     RmsScratch* drms = nullptr;
     int step = 0;
     Acts A;
+    // Page-locked landing place of parameters and gradients (+ the loss behind them),
+    // allocated when first read; reads of one network from several threads take turns.
+    mutable float* stage = nullptr;
+    mutable std::mutex stage_lock;
 };
 
 namespace {
 
 void free_acts(Acts& A)
 {
-    bf16* b[] = {A.e1a, A.e1, A.d1a, A.d1, A.e2a, A.e2, A.d2a, A.d2, A.e3a, A.e3, A.g_d1, A.g_d1a, A.g_cat1, A.g_d2a,
-                 A.g_cat2, A.g_e3a, A.g_p2, A.g_e2a, A.g_p1, A.g_e1a};
+    bf16* b[] = {A.e1a, A.e1, A.d1a, A.d1, A.e2a, A.e2, A.d2a, A.d2, A.e3a, A.e3, A.p1, A.p2, A.g_d1, A.g_d1a, A.g_cat1, A.g_d2a,
+                 A.g_cat2, A.g_e3a, A.g_p2, A.g_e2a, A.g_p1, A.g_e1a, A.g_d2, A.g_e3};
     for (bf16* q : b)
         if (q) cudaFree(q);
     if (A.g_out) cudaFree(A.g_out);
@@ -122,6 +127,8 @@ void ensure_acts(pps_unet* u, int nx, int ny, int nz, bool grads)
     A.d2 = balloc(v2 * c2);
     A.e3a = balloc(v3 * c3);
     A.e3 = balloc(v3 * c3);
+    A.p1 = balloc(v2 * c1);
+    A.p2 = balloc(v3 * c2);
     if (grads) {
         UK(cudaMalloc((void**)&A.g_out, sizeof(float) * (size_t)v1));
         A.g_d1 = balloc(v1 * c1);
@@ -134,6 +141,8 @@ void ensure_acts(pps_unet* u, int nx, int ny, int nz, bool grads)
         A.g_e2a = balloc(v2 * c2);
         A.g_p1 = balloc(v2 * c1);
         A.g_e1a = balloc(v1 * c1);
+        A.g_d2 = balloc(v2 * c2);
+        A.g_e3 = balloc(v3 * c3);
         A.grads = true;
     }
     // the extents last: an allocation that failed half way leaves none
@@ -152,12 +161,6 @@ Src plain(const bf16* X, int ld, int c0 = 0)
     s.c0 = c0;
     return s;
 }
-Src pooled(const bf16* fine, int ld)
-{
-    Src s = plain(fine, ld);
-    s.kind = SRC_POOL;
-    return s;
-}
 // the concatenation [upsampled coarse tensor | skip tensor]
 Src concat(const bf16* up, int c_up, const bf16* skip, int c_skip)
 {
@@ -174,16 +177,6 @@ Src dense(const float* in, const float* rms_dev)
     s.kind = SRC_DENSE;
     s.dense = in;
     s.rms = rms_dev;
-    return s;
-}
-// the gradient of a tensor that was upsampled: its channels lie first in the
-// concatenation's gradient
-Src children(const bf16* gcat, int ld, const bf16* mask, int ldm)
-{
-    Src s = plain(gcat, ld);
-    s.kind = SRC_CHILDREN;
-    s.mask = mask;
-    s.ldm = ldm;
     return s;
 }
 // the gradient of a skip tensor: its slot of the concatenation's gradient plus the pooled path
@@ -206,9 +199,9 @@ Src layer_input(const pps_unet* u, int l, const float* in, const float* rms_dev)
     switch (l) {
     case 0: return dense(in, rms_dev);
     case 1: return plain(A.e1a, c1);
-    case 2: return pooled(A.e1, c1);
+    case 2: return plain(A.p1, c1);
     case 3: return plain(A.e2a, c2);
-    case 4: return pooled(A.e2, c2);
+    case 4: return plain(A.p2, c2);
     case 5: return plain(A.e3a, c3);
     case 6: return concat(A.e3, c3, A.e2, c2);
     case 7: return plain(A.d2a, c2);
@@ -223,8 +216,8 @@ const Dims& layer_dims(const pps_unet* u, int l)
     return l == 4 || l == 5 ? u->A.s3 : (l == 2 || l == 3 || l == 6 || l == 7) ? u->A.s2 : u->A.s1;
 }
 
-// The forward pass: every layer one convolution, the pooling, upsampling and
-// concatenations folded into its loads.  `last` is what the last layer does with its
+// The forward pass: every layer one convolution, upsampling and concatenations folded
+// into its loads, and the two poolings.  `last` is what the last layer does with its
 // sums: the dense output, or the loss and its gradient.
 void forward(pps_unet* u, const float* in, const float* rms_dev, Epi last)
 {
@@ -240,6 +233,8 @@ void forward(pps_unet* u, const float* in, const float* rms_dev, Epi last)
             e.relu = u->linear ? 0 : 1;
         }
         e.bias = Bf(u, l);
+        if (l == 2) gather8(A.s2, A.e1, u->c1, u->c1, 0.125f, nullptr, A.p1, u->stream);
+        if (l == 4) gather8(A.s3, A.e2, u->c2, u->c2, 0.125f, nullptr, A.p2, u->stream);
         conv(layer_dims(u, l), layer_input(u, l, in, rms_dev), u->WP + L.w, L.cin_p, L.cout_p, e, u->stream);
     }
 }
@@ -258,9 +253,9 @@ void backward(pps_unet* u, const float* in)
         plain(A.g_e2a, c2),
         skip(A.g_cat2, c3 + c2, c3, A.g_p2, c2, R ? A.e2 : nullptr),
         plain(A.g_e3a, c3),
-        children(A.g_cat2, c3 + c2, R ? A.e3 : nullptr, c3),
+        plain(A.g_e3, c3),
         plain(A.g_d2a, c2),
-        children(A.g_cat1, c2 + c1, R ? A.d2 : nullptr, c2),
+        plain(A.g_d2, c2),
         plain(A.g_d1a, c1),
         plain(A.g_d1, c1),
         dense(A.g_out, nullptr),
@@ -276,6 +271,9 @@ void backward(pps_unet* u, const float* in)
         e.ld = L.cin_p;
         e.mask = R ? act[l] : nullptr;
         e.ldm = L.cin_p;
+        // gradients of the upsampled tensors: their channels lie first in the concatenation's
+        if (l == 7) gather8(A.s2, A.g_cat1, c2 + c1, c2, 1.0f, R ? A.d2 : nullptr, A.g_d2, u->stream);
+        if (l == 5) gather8(A.s3, A.g_cat2, c3 + c2, c3, 1.0f, R ? A.e3 : nullptr, A.g_e3, u->stream);
         conv(layer_dims(u, l), G[l], u->WB + L.w, L.cout_p, L.cin_p, e, u->stream);
     }
     WgTable T;
@@ -436,6 +434,7 @@ pps_status pps_unet_destroy(pps_unet* u)
     void* p[] = {u->P, u->G, u->M, u->V, u->WP, u->WB, u->dtmp, u->drms};
     for (void* q : p)
         if (q) cudaFree(q);
+    if (u->stage) cudaFreeHost(u->stage);
     if (u->stream) cudaStreamDestroy(u->stream);
     delete u;
     return PPS_OK;
@@ -451,9 +450,13 @@ pps_status pps_unet_set_activation(pps_unet* u, int linear)
 }
 
 // Flat real-parameter layout: per layer W[27][cin][cout] (tap = kz*9+ky*3+kx) then b[cout].
-static void pack(const pps_unet* u, const std::vector<float>& padded, float* real)
+static void unpad(const pps_unet* u, const float* padded, float* real)
 {
     for (const Layer& l : u->L) {
+        if (l.cin == l.cin_p && l.cout == l.cout_p) {   // no padding: W and b lie as they are returned
+            memcpy(real + l.rw, padded + l.w, sizeof(float) * ((size_t)27 * l.cin * l.cout + l.cout));
+            continue;
+        }
         for (int t = 0; t < 27; t++)
             for (int ci = 0; ci < l.cin; ci++)
                 for (int co = 0; co < l.cout; co++)
@@ -462,15 +465,25 @@ static void pack(const pps_unet* u, const std::vector<float>& padded, float* rea
     }
 }
 
+// npad floats of `dev` (and the loss behind them, if asked for) read through the
+// page-locked stage after the work queued on the network's stream.
+static void read_back(const pps_unet* u, const float* dev, float* real, double* loss)
+{
+    std::lock_guard<std::mutex> hold(u->stage_lock);
+    const size_t bytes = sizeof(float) * u->npad + sizeof(double);
+    if (!u->stage) UK(cudaHostAlloc((void**)&u->stage, bytes, cudaHostAllocDefault));
+    UK(cudaMemcpyAsync(u->stage, dev, bytes, cudaMemcpyDeviceToHost, u->stream));
+    UK(cudaStreamSynchronize(u->stream));
+    unpad(u, u->stage, real);
+    if (loss) memcpy(loss, u->stage + u->npad, sizeof(double));
+}
+
 pps_status pps_unet_get_params(const pps_unet* u, float* out)
 {
     if (!u || !out) return PPS_ERR_INVALID_ARG;
     return uguard([&]() -> pps_status {
         UK(cudaSetDevice(u->device));
-        std::vector<float> h(u->npad);
-        UK(cudaMemcpyAsync(h.data(), u->P, sizeof(float) * u->npad, cudaMemcpyDeviceToHost, u->stream));
-        UK(cudaStreamSynchronize(u->stream));
-        pack(u, h, out);
+        read_back(u, u->P, out, nullptr);
         return PPS_OK;
     });
 }
@@ -520,8 +533,8 @@ pps_status pps_unet_forward(pps_unet* u, int nx, int ny, int nz, const float* in
     });
 }
 
-static pps_status loss_and_grads(pps_unet* u, int nx, int ny, int nz, const float* in, const float* target,
-                                 double* loss)
+// Queues the loss and the gradients of one sample (u->G, u->dloss behind it).
+static void loss_and_grads(pps_unet* u, int nx, int ny, int nz, const float* in, const float* target)
 {
     ensure_acts(u, nx, ny, nz, true);
     const long long nv = (long long)nx * ny * nz;
@@ -533,9 +546,6 @@ static pps_status loss_and_grads(pps_unet* u, int nx, int ny, int nz, const floa
     last.inv_n = (float)(1.0 / (double)nv);
     forward(u, in, nullptr, last);
     backward(u, in);
-    UK(cudaMemcpyAsync(loss, u->dloss, sizeof(double), cudaMemcpyDeviceToHost, u->stream));
-    UK(cudaStreamSynchronize(u->stream));
-    return PPS_OK;
 }
 
 pps_status pps_unet_gradients(pps_unet* u, int nx, int ny, int nz, const float* in_dev, const float* target_dev,
@@ -545,12 +555,8 @@ pps_status pps_unet_gradients(pps_unet* u, int nx, int ny, int nz, const float* 
     if (check_dims(nx, ny, nz) != PPS_OK) return PPS_ERR_INVALID_ARG;
     return uguard([&]() -> pps_status {
         UK(cudaSetDevice(u->device));
-        pps_status rc = loss_and_grads(u, nx, ny, nz, in_dev, target_dev, loss);
-        if (rc != PPS_OK) return rc;
-        std::vector<float> h(u->npad);
-        UK(cudaMemcpyAsync(h.data(), u->G, sizeof(float) * u->npad, cudaMemcpyDeviceToHost, u->stream));
-        UK(cudaStreamSynchronize(u->stream));
-        pack(u, h, grads);
+        loss_and_grads(u, nx, ny, nz, in_dev, target_dev);
+        read_back(u, u->G, grads, loss);
         return PPS_OK;
     });
 }
@@ -562,12 +568,12 @@ pps_status pps_unet_train_step(pps_unet* u, int nx, int ny, int nz, const float*
     if (check_dims(nx, ny, nz) != PPS_OK) return PPS_ERR_INVALID_ARG;
     return uguard([&]() -> pps_status {
         UK(cudaSetDevice(u->device));
-        pps_status rc = loss_and_grads(u, nx, ny, nz, in_dev, target_dev, loss);
-        if (rc != PPS_OK) return rc;
+        loss_and_grads(u, nx, ny, nz, in_dev, target_dev);
         u->step += 1;
         rms((long long)u->npad, u->G, u->dtmp + 1, u->drms, u->stream);   // global-norm clipping at 1
         adam(u->pt, (int)u->npad, u->P, u->G, u->M, u->V, u->WP, u->WB, lr, 0.9f, 0.999f, 1e-8f, u->step, u->dtmp + 1,
              1.0f, u->stream);
+        UK(cudaMemcpyAsync(loss, u->dloss, sizeof(double), cudaMemcpyDeviceToHost, u->stream));
         UK(cudaStreamSynchronize(u->stream));
         return PPS_OK;
     });

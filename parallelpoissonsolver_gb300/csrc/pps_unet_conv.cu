@@ -21,6 +21,7 @@
 #include "pps_unet_internal.h"
 
 #include <algorithm>
+#include <initializer_list>
 
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -84,30 +85,6 @@ __device__ __forceinline__ Words<NWORD> load_src(const Src& s, const Dims& d, in
             return ld_words<NWORD>(s.up + cv * s.ld_up + c);
         }
         break;
-    case SRC_POOL:
-    case SRC_CHILDREN: {
-        Words<NWORD> v[8];
-        const long long Hf = 2LL * d.H, Wf = 2LL * d.W;
-#pragma unroll
-        for (int o = 0; o < 8; o++)
-            v[o] = ld_words<NWORD>(s.X + (((2LL * z + (o >> 2)) * Hf + 2 * y + ((o >> 1) & 1)) * Wf + 2 * x + (o & 1)) * s.ld +
-                                   s.c0 + c);
-        Words<NWORD> r, m;
-        if (s.mask) m = ld_words<NWORD>(s.mask + vox * s.ldm + s.cm0 + c);
-        const float sc = kind == SRC_POOL ? 0.125f : 1.0f;
-#pragma unroll
-        for (int q = 0; q < NWORD; q++) {
-            float a = 0.0f, b = 0.0f;
-#pragma unroll
-            for (int o = 0; o < 8; o++) {
-                a += lo_f(v[o].w[q]);
-                b += hi_f(v[o].w[q]);
-            }
-            r.w[q] = pack_bf(sc * a, sc * b);
-            if (s.mask) r.w[q] = relu_mask(r.w[q], m.w[q]);
-        }
-        return r;
-    }
     case SRC_SKIP: {
         Words<NWORD> r = ld_words<NWORD>(s.X + vox * s.ld + s.c0 + c), m;
         const long long cv = ((long long)(z >> 1) * (d.H / 2) + (y >> 1)) * (d.W / 2) + (x >> 1);
@@ -283,111 +260,122 @@ __global__ void __launch_bounds__(32 * NW) k_conv_small(Dims d, Src in, const ui
 }
 
 // ---------------------------------------------------------------------------
-// Large grids.  One block: a tile of 256 voxels x NC output channels.  The tile's
+// Large grids.  One block: a tile of 16 NWARP MG voxels x NC output channels.  The tile's
 // input with its one-voxel halo is staged in shared memory once for all 27 taps
 // (rows padded by 16 bytes, so the 8 rows of a matrix load hit different banks); a
-// warp owns 32 voxels and runs every K step itself, chain after chain, so a chain's
-// accumulator lives in registers and the chains are added there in order.
+// warp owns MG groups of 16 voxels and runs every K step itself, chain after chain, so
+// a chain's accumulator lives in registers and the chains are added there in order.
+// CS = Cin/16 and N16 = Cout/16 where they are known when compiled: the K loop then
+// unrolls to matrix loads at fixed offsets (a table of steps in shared memory cost
+// 18 instructions per product).  CS = 0: any channel counts, by the table.
 // ---------------------------------------------------------------------------
-template <int LX, int LY, int NC>
-__global__ void __launch_bounds__(256) k_conv_tile(Dims d, Src in, const uint4* __restrict__ Wp, int Cin, int Cout,
-                                                   Epi e, int chains, int ntx, int nty, const int* __restrict__ stop)
+template <int LX, int LY, int NWARP, int MG, int NC, int CS, int N16>
+__global__ void __launch_bounds__(32 * NWARP, NWARP > 8 || NC == 48 ? 1 : 2) k_conv_tile(Dims d, Src in, const uint4* __restrict__ Wp, int Cin_,
+                                                                     int Cout, Epi e, int chains_, int ntx, int nty,
+                                                                     const int* __restrict__ stop)
 {
     pdl_enter();
     if (stop && *(volatile const int*)stop) return;
-    constexpr int TX = 1 << LX, TY = 1 << LY, TZ = 256 >> (LX + LY);
+    constexpr int TX = 1 << LX, TY = 1 << LY, TZ = (16 * NWARP * MG) >> (LX + LY);
     constexpr int HX = TX + 2, HY = TY + 2, HZ = TZ + 2, NB = NC / 16;
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ double sl[8];
+    __shared__ double sl[NWARP];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int Cin = CS > 0 ? CS * 16 : Cin_;
     const int stride = Cin * 2 + 16, nch = Cin / 8;
-    const int csteps = Cin / 16, ksteps = 27 * csteps, n16 = Cout / 16;
-    int2* tab = reinterpret_cast<int2*>(smem + HX * HY * HZ * stride);   // K steps in chain order
+    const int csteps = Cin / 16, ksteps = 27 * csteps, n16 = N16 > 0 ? N16 : Cout / 16;
+    int2* tab = reinterpret_cast<int2*>(smem + HX * HY * HZ * stride);   // K steps in chain order (CS = 0)
     const int bx = blockIdx.x % ntx, by = (blockIdx.x / ntx) % nty, bz = blockIdx.x / (ntx * nty);
     const int x0 = bx * TX, y0 = by * TY, z0 = bz * TZ;
     const unsigned sbase = smem_u32(smem);
     const float in_sc = src_scale(in);
-    for (int q = tid; q < HX * HY * HZ * nch; q += 256) {
+    for (int q = tid; q < HX * HY * HZ * nch; q += 32 * NWARP) {
         const int v = q / nch, c = (q - v * nch) * 8;
         const int x = x0 - 1 + v % HX, y = y0 - 1 + (v / HX) % HY, z = z0 - 1 + v / (HX * HY);
         const bool ok = x >= 0 && x < d.W && y >= 0 && y < d.H && z >= 0 && z < d.D;
         const int o = v * stride + c * 2;
         src_to_smem(in, d, z, y, x, c, in_sc, sbase + o, smem + o, ok);
     }
-    if (tid < chains) {
+    if (CS == 0 && tid < chains_) {
         // chain w holds steps w, w + chains, ...; the chains before it hold w whole rounds
         // of them, plus one more each for the first ksteps % chains
-        const int w = tid, full = ksteps / chains, rem = ksteps - full * chains;
+        const int w = tid, full = ksteps / chains_, rem = ksteps - full * chains_;
         int s = w * full + min(w, rem);
-        for (int t = w; t < ksteps; t += chains, s++) {
+        for (int t = w; t < ksteps; t += chains_, s++) {
             const int tap = t / csteps, c0 = (t - tap * csteps) * 16;
             const int a = ((tap / 9) * HY + (tap / 3) % 3) * HX + tap % 3;
-            tab[s] = make_int2((a * stride + c0 * 2) | (t + chains >= ksteps ? 1 : 0), t * n16 * 32);
+            tab[s] = make_int2((a * stride + c0 * 2) | (t + chains_ >= ksteps ? 1 : 0), t * n16 * 32);
         }
     }
     cp_wait_all();
     __syncthreads();
 
-    // this lane's row of the two 16-voxel groups of the warp
-    unsigned abase[2];
+    // this lane's row of the warp's 16-voxel groups
+    unsigned abase[MG];
 #pragma unroll
-    for (int m = 0; m < 2; m++) {
-        const int r = warp * 32 + m * 16 + (lane & 15);
+    for (int m = 0; m < MG; m++) {
+        const int r = (warp * MG + m) * 16 + (lane & 15);
         const int rx = r & (TX - 1), ry = (r >> LX) & (TY - 1), rz = r >> (LX + LY);
         abase[m] = sbase + ((rz * HY + ry) * HX + rx) * stride + (lane >> 4) * 16;
     }
     const uint4* wl = Wp + (long long)blockIdx.y * NB * 32 + lane;
-    float tot[2][2 * NB][4] = {}, acc[2][2 * NB][4] = {};
-    uint4 bn[NB];
-    unsigned an[2][4];
-    int2 en = tab[0];
-#pragma unroll
-    for (int n = 0; n < NB; n++) bn[n] = wl[en.y + n * 32];
-#pragma unroll
-    for (int m = 0; m < 2; m++) ldsm4(an[m], abase[m] + (en.x & ~1));
-    for (int s = 0; s < ksteps; s++) {
-        const int last = en.x & 1;
+    float tot[MG][2 * NB][4] = {}, acc[MG][2 * NB][4] = {};
+    auto step = [&](int aoff, int boff) {
         uint4 b[NB];
-        unsigned a[2][4];
 #pragma unroll
-        for (int n = 0; n < NB; n++) b[n] = bn[n];
+        for (int n = 0; n < NB; n++) b[n] = wl[boff + n * 32];
 #pragma unroll
-        for (int m = 0; m < 2; m++)
-#pragma unroll
-            for (int q = 0; q < 4; q++) a[m][q] = an[m][q];
-        if (s + 1 < ksteps) {
-            en = tab[s + 1];
-#pragma unroll
-            for (int n = 0; n < NB; n++) bn[n] = wl[en.y + n * 32];
-#pragma unroll
-            for (int m = 0; m < 2; m++) ldsm4(an[m], abase[m] + (en.x & ~1));
-        }
-#pragma unroll
-        for (int m = 0; m < 2; m++)
+        for (int m = 0; m < MG; m++) {
+            unsigned a[4];
+            ldsm4(a, abase[m] + aoff);
 #pragma unroll
             for (int n = 0; n < NB; n++) {
-                mma16816(acc[m][2 * n], a[m], b[n].x, b[n].y);
-                mma16816(acc[m][2 * n + 1], a[m], b[n].z, b[n].w);
+                mma16816(acc[m][2 * n], a, b[n].x, b[n].y);
+                mma16816(acc[m][2 * n + 1], a, b[n].z, b[n].w);
             }
-        if (last) {
+        }
+    };
+    auto end_chain = [&]() {
 #pragma unroll
-            for (int m = 0; m < 2; m++)
+        for (int m = 0; m < MG; m++)
 #pragma unroll
-                for (int n = 0; n < 2 * NB; n++)
+            for (int n = 0; n < 2 * NB; n++)
 #pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        tot[m][n][q] += acc[m][n][q];
-                        acc[m][n][q] = 0.0f;
-                    }
+                for (int q = 0; q < 4; q++) {
+                    tot[m][n][q] += acc[m][n][q];
+                    acc[m][n][q] = 0.0f;
+                }
+    };
+    if constexpr (CS > 0) {
+        constexpr int KS = 27 * CS, CH = KS >= 64 ? 16 : 8;
+#pragma unroll
+        for (int w = 0; w < CH; w++) {
+            // always taken (chains_ = CH), but the compiler does not know it: chains in one
+            // basic block are interleaved, whose accumulators would not fit the registers
+            if (w >= chains_) break;
+#pragma unroll
+            for (int t = w; t < KS; t += CH) {
+                const int tap = t / CS, c0 = (t % CS) * 16;
+                step((((tap / 9) * HY + (tap / 3) % 3) * HX + tap % 3) * (CS * 32 + 16) + c0 * 2, t * N16 * 32);
+            }
+            end_chain();
+        }
+    } else {
+        int2 en = tab[0];
+        for (int s = 0; s < ksteps; s++) {
+            const int2 cur = en;
+            if (s + 1 < ksteps) en = tab[s + 1];
+            step(cur.x & ~1, cur.y);
+            if (cur.x & 1) end_chain();
         }
     }
     const int gid = lane >> 2, tig = lane & 3, co0 = blockIdx.y * NC;
     double loss = 0.0;
 #pragma unroll
-    for (int m = 0; m < 2; m++)
+    for (int m = 0; m < MG; m++)
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-            const int r = warp * 32 + m * 16 + gid + 8 * h;
+            const int r = (warp * MG + m) * 16 + gid + 8 * h;
             const int x = x0 + (r & (TX - 1)), y = y0 + ((r >> LX) & (TY - 1)), z = z0 + (r >> (LX + LY));
             if (x >= d.W || y >= d.H || z >= d.D) continue;
             const long long vox = ((long long)z * d.H + y) * d.W + x;
@@ -419,7 +407,7 @@ __global__ void __launch_bounds__(256) k_conv_tile(Dims d, Src in, const uint4* 
         __syncthreads();
         if (tid == 0) {
             double s = 0.0;
-            for (int w = 0; w < 8; w++) s += sl[w];
+            for (int w = 0; w < NWARP; w++) s += sl[w];
             atomicAdd(e.loss, s / ((double)d.D * d.H * d.W));
         }
     }
@@ -439,23 +427,45 @@ TileShape tile_shape(const Dims& d)
 }
 int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
-template <int LX, int LY, int NC>
+template <int LX, int LY, int NWARP, int MG, int NC, int CS, int N16>
 void tile_launch(const Dims& d, const Src& in, const uint4* Wp, int Cin, int Cout, const Epi& e, int chains, cudaStream_t s)
 {
-    constexpr int LZ = 8 - LX - LY;
-    const int ntx = ceil_div(d.W, 1 << LX), nty = ceil_div(d.H, 1 << LY), ntz = ceil_div(d.D, 1 << LZ);
-    const size_t halo = (size_t)((1 << LX) + 2) * ((1 << LY) + 2) * ((1 << LZ) + 2);
-    const size_t smem = halo * (Cin * 2 + 16) + sizeof(int2) * 27 * (Cin / 16);
-    launch_pdl(k_conv_tile<LX, LY, NC>, dim3((unsigned)(ntx * nty * ntz), (unsigned)(Cout / NC)), 256, smem, s, d, in, Wp,
-               Cin, Cout, e, chains, ntx, nty, stop_flag());
+    constexpr int TX = 1 << LX, TY = 1 << LY, TZ = (16 * NWARP * MG) >> (LX + LY);
+    const int ntx = ceil_div(d.W, TX), nty = ceil_div(d.H, TY), ntz = ceil_div(d.D, TZ);
+    const size_t smem = (size_t)(TX + 2) * (TY + 2) * (TZ + 2) * (Cin * 2 + 16) + (CS ? 0 : sizeof(int2) * 27 * (Cin / 16));
+    launch_pdl(k_conv_tile<LX, LY, NWARP, MG, NC, CS, N16>, dim3((unsigned)(ntx * nty * ntz), (unsigned)(Cout / NC)),
+               32 * NWARP, smem, s, d, in, Wp, Cin, Cout, e, chains, ntx, nty, stop_flag());
 }
 
 template <int LX, int LY>
-void tile_nc(const Dims& d, const Src& in, const uint4* Wp, int Cin, int Cout, const Epi& e, int chains, cudaStream_t s)
+void tile_any(const Dims& d, const Src& in, const uint4* Wp, int Cin, int Cout, const Epi& e, int chains, cudaStream_t s)
 {
-    if (Cout % 48 == 0) tile_launch<LX, LY, 48>(d, in, Wp, Cin, Cout, e, chains, s);
-    else if (Cout % 32 == 0) tile_launch<LX, LY, 32>(d, in, Wp, Cin, Cout, e, chains, s);
-    else tile_launch<LX, LY, 16>(d, in, Wp, Cin, Cout, e, chains, s);
+    if (Cout % 48 == 0) tile_launch<LX, LY, 8, 2, 48, 0, 0>(d, in, Wp, Cin, Cout, e, chains, s);
+    else if (Cout % 32 == 0) tile_launch<LX, LY, 8, 2, 32, 0, 0>(d, in, Wp, Cin, Cout, e, chains, s);
+    else tile_launch<LX, LY, 8, 2, 16, 0, 0>(d, in, Wp, Cin, Cout, e, chains, s);
+}
+
+// The 16-wide tiles of the default network's layers (channels 16/32/64), else any.
+void tile_wide(const Dims& d, const Src& in, const uint4* Wp, int Cin, int Cout, const Epi& e, int chains, cudaStream_t s)
+{
+    const bool fills = (long long)d.D * d.H * d.W >= 512LL * sm_count();   // 512-voxel tiles for every SM
+    switch (Cin * 100 + Cout) {
+    case 1616: tile_launch<4, 3, 8, 4, 16, 1, 1>(d, in, Wp, Cin, Cout, e, chains, s); break;
+    case 1632: tile_launch<4, 2, 8, 2, 32, 1, 2>(d, in, Wp, Cin, Cout, e, chains, s); break;
+    case 1648: tile_launch<4, 2, 8, 2, 48, 1, 3>(d, in, Wp, Cin, Cout, e, chains, s); break;
+    case 3216: tile_launch<4, 2, 8, 2, 16, 2, 1>(d, in, Wp, Cin, Cout, e, chains, s); break;
+    case 3232: tile_launch<4, 2, 8, 2, 32, 2, 2>(d, in, Wp, Cin, Cout, e, chains, s); break;
+    case 3264: tile_launch<4, 2, 8, 2, 32, 2, 4>(d, in, Wp, Cin, Cout, e, chains, s); break;
+    case 3296: tile_launch<4, 2, 8, 2, 48, 2, 6>(d, in, Wp, Cin, Cout, e, chains, s); break;
+    case 4816: tile_launch<4, 2, 8, 2, 16, 3, 1>(d, in, Wp, Cin, Cout, e, chains, s); break;
+    case 6432: tile_launch<4, 2, 8, 2, 32, 4, 2>(d, in, Wp, Cin, Cout, e, chains, s); break;
+    case 6464: tile_launch<4, 2, 8, 2, 32, 4, 4>(d, in, Wp, Cin, Cout, e, chains, s); break;
+    case 9632:   // 135 KB a tile leaves one block per SM: sixteen warps of it where the grid has the tiles
+        if (fills) tile_launch<4, 3, 16, 2, 32, 6, 2>(d, in, Wp, Cin, Cout, e, chains, s);
+        else tile_launch<4, 2, 8, 2, 32, 6, 2>(d, in, Wp, Cin, Cout, e, chains, s);
+        break;
+    default: tile_any<4, 2>(d, in, Wp, Cin, Cout, e, chains, s); break;
+    }
 }
 
 template <int KIND>
@@ -466,21 +476,35 @@ void small_launch(const Dims& d, const Src& in, const uint4* Wp, int Cin, int Co
     else launch_pdl(k_conv_small<8, KIND>, grid, 256, 0, s, d, in, Wp, Cin, Cout, e, stop_flag());
 }
 
-template <int LX, int LY>
-cudaError_t allow_smem()
+cudaError_t allow_smem(std::initializer_list<const void*> kernels)
 {
     cudaError_t e = cudaSuccess;
-    for (const void* k : {(const void*)k_conv_tile<LX, LY, 16>, (const void*)k_conv_tile<LX, LY, 32>,
-                          (const void*)k_conv_tile<LX, LY, 48>})
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+    for (const void* k : kernels)
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
     return e;
+}
+template <int LX, int LY>
+cudaError_t allow_smem_any()
+{
+    return allow_smem({(const void*)k_conv_tile<LX, LY, 8, 2, 16, 0, 0>, (const void*)k_conv_tile<LX, LY, 8, 2, 32, 0, 0>,
+                       (const void*)k_conv_tile<LX, LY, 8, 2, 48, 0, 0>});
+}
+cudaError_t allow_smem_wide()
+{
+    return allow_smem(
+        {(const void*)k_conv_tile<4, 3, 8, 4, 16, 1, 1>, (const void*)k_conv_tile<4, 2, 8, 2, 32, 1, 2>,
+         (const void*)k_conv_tile<4, 2, 8, 2, 48, 1, 3>, (const void*)k_conv_tile<4, 2, 8, 2, 16, 2, 1>,
+         (const void*)k_conv_tile<4, 2, 8, 2, 32, 2, 2>, (const void*)k_conv_tile<4, 2, 8, 2, 32, 2, 4>,
+         (const void*)k_conv_tile<4, 2, 8, 2, 48, 2, 6>, (const void*)k_conv_tile<4, 2, 8, 2, 16, 3, 1>,
+         (const void*)k_conv_tile<4, 2, 8, 2, 32, 4, 2>, (const void*)k_conv_tile<4, 2, 8, 2, 32, 4, 4>,
+         (const void*)k_conv_tile<4, 2, 8, 2, 32, 6, 2>, (const void*)k_conv_tile<4, 3, 16, 2, 32, 6, 2>});
 }
 
 }  // namespace
 
 // Tiles of 256 voxels from which the tile kernel is the faster one (blocks of it that
 // a launch needs to beat 16 times as many small ones).
-constexpr int CONV_TILES_MIN = 64;
+constexpr int CONV_TILES_MIN = 32;
 
 void conv(const Dims& d, const Src& in, const bf16* Wpacked, int Cin, int Cout, const Epi& e, cudaStream_t s)
 {
@@ -489,16 +513,14 @@ void conv(const Dims& d, const Src& in, const bf16* Wpacked, int Cin, int Cout, 
     const TileShape t = tile_shape(d);
     const long long tiles = (long long)ceil_div(d.W, 1 << t.lx) * ceil_div(d.H, 1 << t.ly) * ceil_div(d.D, 1 << t.lz);
     if (tiles >= CONV_TILES_MIN) {
-        if (t.lx == 4) tile_nc<4, 2>(d, in, Wp, Cin, Cout, e, chains, s);
-        else if (t.lx == 3) tile_nc<3, 3>(d, in, Wp, Cin, Cout, e, chains, s);
-        else tile_nc<2, 3>(d, in, Wp, Cin, Cout, e, chains, s);
+        if (t.lx == 4) tile_wide(d, in, Wp, Cin, Cout, e, chains, s);
+        else if (t.lx == 3) tile_any<3, 3>(d, in, Wp, Cin, Cout, e, chains, s);
+        else tile_any<2, 3>(d, in, Wp, Cin, Cout, e, chains, s);
     } else {
         switch (in.kind) {
         case SRC_PLAIN: small_launch<SRC_PLAIN>(d, in, Wp, Cin, Cout, e, chains, s); break;
         case SRC_DENSE: small_launch<SRC_DENSE>(d, in, Wp, Cin, Cout, e, chains, s); break;
         case SRC_UP: small_launch<SRC_UP>(d, in, Wp, Cin, Cout, e, chains, s); break;
-        case SRC_POOL: small_launch<SRC_POOL>(d, in, Wp, Cin, Cout, e, chains, s); break;
-        case SRC_CHILDREN: small_launch<SRC_CHILDREN>(d, in, Wp, Cin, Cout, e, chains, s); break;
         default: small_launch<SRC_SKIP>(d, in, Wp, Cin, Cout, e, chains, s); break;
         }
     }
@@ -633,6 +655,53 @@ void wgrad(WgTable& T, cudaStream_t s)
 }
 
 // ---------------------------------------------------------------------------
+// Sums over the 8 fine voxels of a coarse one: out[v][c] = BF16(scale * sum), kept where
+// mask > 0.  scale 1/8: average pooling; scale 1: the gradient of a nearest upsampling.
+// One thread per 8 channels.  (Folded into the convolution's loads instead, every
+// output voxel repeats the 8 loads for each tap: 17 us for a 4^3 level against 3.)
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) k_gather8(Dims d, const bf16* __restrict__ X, int ld, int C, float scale,
+                                                 const bf16* __restrict__ mask, bf16* __restrict__ out,
+                                                 const int* __restrict__ stop)
+{
+    pdl_enter();
+    if (stop && *(volatile const int*)stop) return;
+    const int nch = C / 8;
+    const long long n = (long long)d.D * d.H * d.W * nch;
+    const long long Hf = 2LL * d.H, Wf = 2LL * d.W;
+    for (long long q = blockIdx.x * 256LL + threadIdx.x; q < n; q += gridDim.x * 256LL) {
+        const long long v = q / nch;
+        const int c = (int)(q - v * nch) * 8;
+        const int x = (int)(v % d.W), y = (int)((v / d.W) % d.H), z = (int)(v / ((long long)d.W * d.H));
+        Words<4> w[8], r, m;
+#pragma unroll
+        for (int o = 0; o < 8; o++)
+            w[o] = ld_words<4>(X + (((2LL * z + (o >> 2)) * Hf + 2 * y + ((o >> 1) & 1)) * Wf + 2 * x + (o & 1)) * ld + c);
+        if (mask) m = ld_words<4>(mask + q * 8);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            float a = 0.0f, b = 0.0f;
+#pragma unroll
+            for (int o = 0; o < 8; o++) {
+                a += lo_f(w[o].w[k]);
+                b += hi_f(w[o].w[k]);
+            }
+            r.w[k] = pack_bf(scale * a, scale * b);
+            if (mask) r.w[k] = relu_mask(r.w[k], m.w[k]);
+        }
+        *reinterpret_cast<uint4*>(out + q * 8) = make_uint4(r.w[0], r.w[1], r.w[2], r.w[3]);
+    }
+}
+
+void gather8(const Dims& d, const bf16* X, int ld, int C, float scale, const bf16* mask, bf16* out, cudaStream_t s)
+{
+    const long long n = (long long)d.D * d.H * d.W * (C / 8);
+    launch_pdl(k_gather8, (unsigned)std::min<long long>((n + 255) / 256, 16LL * sm_count()), 256, 0, s, d, X, ld, C, scale,
+               mask, out, stop_flag());
+    launches_counter_add(1);
+}
+
+// ---------------------------------------------------------------------------
 // Parameters
 // ---------------------------------------------------------------------------
 
@@ -763,9 +832,10 @@ void rms(long long n, const float* a, float* out, RmsScratch* scratch, cudaStrea
 
 cudaError_t conv_prepare()
 {
-    cudaError_t e = allow_smem<4, 2>();
-    if (e == cudaSuccess) e = allow_smem<3, 3>();
-    if (e == cudaSuccess) e = allow_smem<2, 3>();
+    cudaError_t e = allow_smem_any<4, 2>();
+    if (e == cudaSuccess) e = allow_smem_any<3, 3>();
+    if (e == cudaSuccess) e = allow_smem_any<2, 3>();
+    if (e == cudaSuccess) e = allow_smem_wide();
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, WG_SMEM);
     return e;
 }

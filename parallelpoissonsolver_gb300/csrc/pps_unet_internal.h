@@ -29,9 +29,7 @@ enum SrcKind : int {
     SRC_PLAIN = 0,      // X, leading dimension ld, channels from c0
     SRC_DENSE = 1,      // channel 0 = BF16(dense / (*rms)) (rms null: dense itself), zeros elsewhere
     SRC_UP = 2,         // channels [0, c_up): nearest 2x upsampling of `up`; the others: X at c0 + c
-    SRC_POOL = 3,       // mean of the 8 fine voxels of X
-    SRC_CHILDREN = 4,   // sum of the 8 fine voxels of X (upsampling backward), kept where mask > 0
-    SRC_SKIP = 5        // X + up/8 at the coarse voxel (pooling backward onto a skip gradient), kept where mask > 0
+    SRC_SKIP = 3        // X + up/8 at the coarse voxel (pooling backward onto a skip gradient), kept where mask > 0
 };
 struct Src {
     int kind = SRC_PLAIN;
@@ -66,6 +64,10 @@ struct Epi {
 // 3x3x3 zero-padded convolution on tensor cores (Cin, Cout multiples of 16, at most
 // 96), weights packed by pack().
 void conv(const Dims& d, const Src& in, const bf16* Wpacked, int Cin, int Cout, const Epi& e, cudaStream_t s);
+
+// out = BF16(scale * sum over the 8 fine voxels of X), kept where mask > 0 (null: everywhere);
+// d: the coarse grid, X: channels [0, C) of a fine tensor, out and mask dense.
+void gather8(const Dims& d, const bf16* X, int ld, int C, float scale, const bf16* mask, bf16* out, cudaStream_t s);
 
 // Weight and bias gradients of up to 11 layers in one launch (dW, db are added to).
 struct WgLayer {
