@@ -120,12 +120,11 @@ extern "C" pps_status pps_apply_operator_noalloc(const pps_grid* grid, const dou
     DevState* st = (DevState*)(base + kStateOffset);
     unsigned* counter = (unsigned*)(base + kCounterOffset);
     double* partials = (double*)(base + kPartialsOffset);
-    // The array keeps the previous call's contents: reset the scalar block (done = 0)
-    // and the completion counter, which the kernel needs at zero.
+    // One launch: the scratch starts as zeros, the kernel's last block resets the
+    // completion counter, and a reduction that only stores never sets the stop flag, so
+    // no call has anything to reset (a state kernel, a fill and a copy of the energy
+    // around the stencil took 17 of 39 us on a 64 x 48 x 80 box).
     const unsigned long long failures = launch_failures();
-    state_init(st, nullptr, 0, 0.0, 0.0, 0, 0, 1.0, 0, s);
-    e = cudaMemsetAsync(counter, 0, sizeof(unsigned), s);
-    if (e != cudaSuccess) return fail(PPS_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
 
     RedCtx rc;
     rc.partials = partials;
@@ -133,6 +132,7 @@ extern "C" pps_status pps_apply_operator_noalloc(const pps_grid* grid, const dou
     rc.st = st;
     rc.hist = nullptr;
     rc.kind = FIN_STORE;
+    rc.store = energy_dev;
     Coef a;
     const double ix = 1.0 / (g.ds[0] * g.ds[0]), iy = 1.0 / (g.ds[1] * g.ds[1]), iz = 1.0 / (g.ds[2] * g.ds[2]);
     a.cc = -2.0 * (ix + iy + iz);
@@ -141,12 +141,10 @@ extern "C" pps_status pps_apply_operator_noalloc(const pps_grid* grid, const dou
     a.cz = iz;
     a.cb = a.cw = 0.0;
     a.scale = 1.0;
-    // out = A u at the unknowns; sum u * (A u) over the unknowns into st->sums[0]
+    // out = A u at the unknowns; sum u * (A u) over the unknowns into *energy_dev
     fast_stencil_dot<double>(g, sh, u_dev, u_dev, out_dev, a, rc, s);
     e = cudaGetLastError();
     if (e != cudaSuccess) return fail(PPS_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
     if (launch_failures() != failures) return PPS_ERR_CUDA;   // the message is set already
-    e = cudaMemcpyAsync(energy_dev, &st->sums[0], sizeof(double), cudaMemcpyDeviceToDevice, s);
-    if (e != cudaSuccess) return fail(PPS_ERR_CUDA, std::string("cudaMemcpyAsync: ") + cudaGetErrorString(e));
     return PPS_OK;
 }

@@ -188,6 +188,9 @@ static __device__ void finalize(const RedCtx& rc, const double* tot)
         }
         break;
     }
+    case FIN_STORE:
+        if (rc.store) *rc.store = tot[0];
+        break;
     default:
         break;
     }
