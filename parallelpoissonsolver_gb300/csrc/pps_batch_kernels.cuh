@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(256) bk_cheb_s01(BatchDev B, const float* __re
     const CT<float> cf = coef[(size_t)q.p * cstride + ci];
     const Geo& g = q.P->g;
     if (q.cx == 4) {   // the block's rows are whole warps: all lanes reach the shuffles
-        cheb_v4_march<0>(g, q.i, q.k0, q.k1, q.c, Bf, nullptr, nullptr, Y, cf);
+        cheb_v4_march<0>(g, q.i, q.j, q.k0, q.k1, q.c, Bf, nullptr, nullptr, Y, cf);
         return;
     }
     const long long sj = g.sj, sk = g.sk;
@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(256) bk_cheb_sweep(BatchDev B, const float* __
     const CT<float> cf = coef[(size_t)q.p * cstride + ci];
     const Geo& g = q.P->g;
     if (q.cx == 4) {
-        cheb_v4_march<HAS_Z ? 2 : 1>(g, q.i, q.k0, q.k1, q.c, Y, Bf, Z, W, cf);
+        cheb_v4_march<HAS_Z ? 2 : 1>(g, q.i, q.j, q.k0, q.k1, q.c, Y, Bf, Z, W, cf);
         return;
     }
     const long long sj = g.sj, sk = g.sk;

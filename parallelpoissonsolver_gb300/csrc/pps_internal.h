@@ -270,9 +270,11 @@ template <typename T>
 void neumann_fill(const Geo& g, T* field, Faces f, int field_mode, double normb, cudaStream_t s);
 
 // Fast kernels, T = float or double storage.
-// Y = s1 (pre-folded coefficients; scale -1 gives X = -s1 directly).
+// Y = s1 (pre-folded coefficients; scale -1 gives X = -s1 directly).  mirror: the
+// kernel also fills the output's ghost points at Neumann faces (neumann_fill's mirror copy).
 template <typename T>
-void fast_cheb_s01(const Geo& g, const Shape& sh, const T* B, T* Y, const Coef& cy, const int* done, cudaStream_t s);
+void fast_cheb_s01(const Geo& g, const Shape& sh, const T* B, T* Y, const Coef& cy, const int* done, cudaStream_t s,
+                   bool mirror = true);
 // One sweep; Z == nullptr for the first sweep (s0 folded into the B coefficient).
 // s1..s_nsteps of the Chebyshev recurrence in one pass (nsteps 2 or 3): c[0] makes
 // s1 from B, c[t-1] step t (the last one's scale is the output's -1); X = the last
@@ -281,7 +283,7 @@ template <typename T>
 void fast_cheb_fused(const Geo& g, int nsteps, const T* B, T* X, const Coef* c, const int* done, cudaStream_t s);
 template <typename T>
 void fast_cheb_sweep(const Geo& g, const Shape& sh, const T* Y, const T* B, const T* Z, T* W, const Coef& c,
-                     const int* done, cudaStream_t s);
+                     const int* done, cudaStream_t s, bool mirror = true);
 template <typename T>
 void fast_scale_copy(const Geo& g, const Shape& sh, const T* B, T* X, double a, const int* done, cudaStream_t s);
 template <typename T>

@@ -425,10 +425,17 @@ void seq_dot2(const Geo& g, const double* a1, const double* b1, const double* a2
 // Neumann ghost fill (both families; the arithmetic matches the reference order)
 // ---------------------------------------------------------------------------
 
+struct FaceList {
+    int n, face[6];
+};
+
+// All Neumann faces of a grid in one launch (blockIdx.y picks the face): a face reads
+// data nodes and writes its own ghost layer, so the faces do not depend on each other.
 template <typename T>
-__global__ void k_neumann_fill(Geo g, T* __restrict__ field, Faces f, int face, int field_mode, double normb)
+__global__ void k_neumann_fill(Geo g, T* __restrict__ field, Faces f, FaceList fl, int field_mode, double normb)
 {
     pdl_enter();
+    const int face = fl.face[blockIdx.y];
     const int dir = face / 2, side = face % 2;
     const int a0 = dir == 0 ? 1 : 0;          // first remaining axis
     const int a1 = dir == 2 ? 1 : 2;          // second remaining axis
@@ -458,15 +465,18 @@ __global__ void k_neumann_fill(Geo g, T* __restrict__ field, Faces f, int face, 
 template <typename T>
 void neumann_fill(const Geo& g, T* field, Faces f, int field_mode, double normb, cudaStream_t s)
 {
+    FaceList fl{};
+    long long most = 0;
     for (int face = 0; face < 6; face++) {
         if (g.bcs[face] != 1) continue;
         const int dir = face / 2;
-        const long long total = (long long)g.n[dir == 0 ? 1 : 0] * g.n[dir == 2 ? 1 : 2];
-        unsigned blocks = (unsigned)((total + 255) / 256);
-        if (blocks > 1024) blocks = 1024;
-        launch_pdl(k_neumann_fill<T>, blocks, 256, 0, s, g, field, f, face, field_mode, normb);
-        PPS_COUNT_LAUNCH();
+        fl.face[fl.n++] = face;
+        most = std::max(most, (long long)g.n[dir == 0 ? 1 : 0] * g.n[dir == 2 ? 1 : 2]);
     }
+    if (fl.n == 0) return;
+    const unsigned blocks = (unsigned)std::min<long long>((most + 255) / 256, 1024);
+    launch_pdl(k_neumann_fill<T>, dim3(blocks, (unsigned)fl.n), 256, 0, s, g, field, f, fl, field_mode, normb);
+    PPS_COUNT_LAUNCH();
 }
 template void neumann_fill<double>(const Geo&, double*, Faces, int, double, cudaStream_t);
 template void neumann_fill<float>(const Geo&, float*, Faces, int, double, cudaStream_t);
@@ -677,12 +687,37 @@ __device__ __forceinline__ Col column_cx(const Geo& g, const Shape& sh, int cxw)
     return q;
 }
 
+static bool has_neumann(const Geo& g)
+{
+    for (int f = 0; f < 6; f++)
+        if (g.bcs[f] == 1) return true;
+    return false;
+}
+
+// W[c] = w at unknown (i, j, k); with NEU also into the ghost point that mirrors it
+// across a Neumann face one node away, so that the next stencil on W needs no fill of
+// its own (neumann_fill after each of the 9 steps of a degree-11 application was 18 %
+// of a solve on 128 x 128 x 256 with three Neumann faces).
+template <bool NEU, typename T>
+__device__ __forceinline__ void store_mirrored(const Geo& g, T* W, long long c, T w, int i, int j, int k)
+{
+    W[c] = w;
+    if (NEU) {
+        if (g.bcs[0] == 1 && i == 2) W[c - 2] = w;
+        if (g.bcs[1] == 1 && i == g.n[0] - 1) W[c + 2] = w;
+        if (g.bcs[2] == 1 && j == 2) W[c - 2 * g.sj] = w;
+        if (g.bcs[3] == 1 && j == g.n[1] - 1) W[c + 2 * g.sj] = w;
+        if (g.bcs[4] == 1 && k == 2) W[c - 2 * g.sk] = w;
+        if (g.bcs[5] == 1 && k == g.n[2] - 1) W[c + 2 * g.sk] = w;
+    }
+}
+
 // s1 of the preconditioner (chebyshevIteration.hpp:79-90) in pre-folded form:
 //   Y = cc*B + cx*(Bx pair) + cy*(By pair) + cz*(Bz pair)
 // s0 = B/theta is never stored: the first sweep folds it into its B coefficient.
 // With the output scale -1 folded into the coefficients this also writes X = -s1
 // directly (degree 3).
-template <typename T, int CX>
+template <typename T, int CX, bool NEU>
 __global__ void __launch_bounds__(256) k_cheb_s01(Geo g, Shape sh, const T* __restrict__ B, T* __restrict__ Y,
                                                   CT<T> cf, const int* done)
 {
@@ -714,7 +749,7 @@ __global__ void __launch_bounds__(256) k_cheb_s01(Geo g, Shape sh, const T* __re
             y = fmx(cf.cx, sx, y);
             y = fmx(cf.cy, sy, y);
             y = fmx(cf.cz, bm[u] + bp, y);
-            Y[c] = y;
+            store_mirrored<NEU>(g, Y, c, y, q.i + 32 * u, q.j, k);
             bm[u] = bc[u];
             bc[u] = bp;
         }
@@ -725,7 +760,7 @@ __global__ void __launch_bounds__(256) k_cheb_s01(Geo g, Shape sh, const T* __re
 // One sweep (chebyshevIteration.hpp:110) in pre-folded form:
 //   W = cc*Y + cx*(Yx pair) + cy*(Yy pair) + cz*(Yz pair) + cb*B [+ cw*Z]
 // HAS_Z = false for the first sweep, whose Z = s0 = B/theta is folded into cb.
-template <typename T, int CX, bool HAS_Z>
+template <typename T, int CX, bool HAS_Z, bool NEU>
 __global__ void __launch_bounds__(256) k_cheb_sweep(Geo g, Shape sh, const T* __restrict__ Y,
                                                     const T* __restrict__ B, const T* __restrict__ Z,
                                                     T* __restrict__ W, CT<T> cf, const int* done)
@@ -760,7 +795,7 @@ __global__ void __launch_bounds__(256) k_cheb_sweep(Geo g, Shape sh, const T* __
             w = fmx(cf.cz, ym[u] + yp, w);
             w = fmx(cf.cb, B[c], w);
             if (HAS_Z) w = fmx(cf.cw, Z[c], w);
-            W[c] = w;
+            store_mirrored<NEU>(g, W, c, w, q.i + 32 * u, q.j, k);
             ym[u] = yc[u];
             yc[u] = yp;
         }
@@ -807,8 +842,8 @@ __device__ __forceinline__ float4 add4(float4 a, float4 b)
 // (k_cheb_s01); 1: a sweep without Z; 2: a sweep with Z.  Every lane of the warp must
 // call it (the x neighbours come by shuffle); lanes whose float4 holds no unknown
 // compute on zeros and store nothing.
-template <int MODE>
-__device__ __forceinline__ void cheb_v4_march(const Geo& g, int i0, int k0, int k1, long long c,
+template <int MODE, bool NEU = false>
+__device__ __forceinline__ void cheb_v4_march(const Geo& g, int i0, int j, int k0, int k1, long long c,
                                               const float* __restrict__ U, const float* __restrict__ B,
                                               const float* __restrict__ Z, float* __restrict__ W, const CT<float>& cf)
 {
@@ -847,13 +882,13 @@ __device__ __forceinline__ void cheb_v4_march(const Geo& g, int i0, int k0, int 
             w.w = fmx(cf.cw, zv.w, w.w);
         }
         if (act) {
-            if (all4) {
+            if (all4 && !NEU) {
                 *reinterpret_cast<float4*>(W + c) = w;
             } else {
-                if (m0) W[c] = w.x;
-                if (m1) W[c + 1] = w.y;
-                if (m2) W[c + 2] = w.z;
-                if (m3) W[c + 3] = w.w;
+                if (m0) store_mirrored<NEU>(g, W, c, w.x, i0, j, k);
+                if (m1) store_mirrored<NEU>(g, W, c + 1, w.y, i0 + 1, j, k);
+                if (m2) store_mirrored<NEU>(g, W, c + 2, w.z, i0 + 2, j, k);
+                if (m3) store_mirrored<NEU>(g, W, c + 3, w.w, i0 + 3, j, k);
             }
         }
         um = uc;
@@ -862,7 +897,7 @@ __device__ __forceinline__ void cheb_v4_march(const Geo& g, int i0, int k0, int 
     }
 }
 
-template <int MODE>
+template <int MODE, bool NEU>
 __global__ void __launch_bounds__(256) k_cheb_v4(Geo g, Shape sh, const float* __restrict__ U,
                                                  const float* __restrict__ B, const float* __restrict__ Z,
                                                  float* __restrict__ W, CT<float> cf, const int* done)
@@ -871,7 +906,7 @@ __global__ void __launch_bounds__(256) k_cheb_v4(Geo g, Shape sh, const float* _
     EARLY_EXIT(done);
     const Col4 q = column4(g, sh);
     if (q.j >= g.hi[1]) return;   // a warp shares its row, so its lanes leave together
-    cheb_v4_march<MODE>(g, q.i0, q.k0, q.k1, q.c, U, B, Z, W, cf);
+    cheb_v4_march<MODE, NEU>(g, q.i0, q.j, q.k0, q.k1, q.c, U, B, Z, W, cf);
 }
 
 // The vectorised kernels take FP32 fields whose rows start on 16-byte boundaries.
@@ -1956,7 +1991,7 @@ __device__ __forceinline__ bool nsum6(const MI& a, const MI& b, const MI& c, con
 //   MODE 2: W = cc U + cx (six-neighbour sum) + cb B + cw Z          (later sweeps)
 // with the coefficients of k_cheb_s01 / k_cheb_sweep: 3, 4 or 5 FP64 operations per
 // unknown instead of 8 or 9.
-template <int MODE>
+template <int MODE, bool NEU>
 __global__ void __launch_bounds__(256) k_cheb_iso64(Geo g, Shape sh, const double* __restrict__ U,
                                                     const double* __restrict__ B, const double* __restrict__ Z,
                                                     double* __restrict__ W, CT<double> cf, const int* done)
@@ -1985,7 +2020,7 @@ __global__ void __launch_bounds__(256) k_cheb_iso64(Geo g, Shape sh, const doubl
         }
         if (MODE >= 1) w = fmx(cf.cb, B[c], w);
         if (MODE == 2) w = fmx(cf.cw, Z[c], w);
-        W[c] = w;
+        store_mirrored<NEU>(g, W, c, w, q.i, q.j, k);
         um = uc;
         uc = up;
         mm = mc;
@@ -2370,67 +2405,82 @@ __global__ void k_state_init(DevState* st, double* hist, int maxit, double tol_a
 
 // ---- wrappers ----
 
-template <typename T>
-void fast_cheb_s01(const Geo& g, const Shape& sh, const T* B, T* Y, const Coef& cy, const int* done, cudaStream_t s)
+template <typename T, bool NEU>
+static void cheb_s01_launch(const Geo& g, const Shape& sh, const T* B, T* Y, const Coef& cy, const int* done, cudaStream_t s)
 {
     const CT<T> c = cast_coef<T>(cy);
     if (sh.cx == 4) {
         if constexpr (std::is_same<T, float>::value) {
             if (v4_ok<T>(g, B, Y, nullptr, nullptr)) {
-                launch_pdl(k_cheb_v4<0>, grid_of(sh), block_of(sh), 0, s, g, sh, B, nullptr, nullptr, Y, c, done);
+                launch_pdl(k_cheb_v4<0, NEU>, grid_of(sh), block_of(sh), 0, s, g, sh, B, nullptr, nullptr, Y, c, done);
                 PPS_COUNT_LAUNCH();
                 return;
             }
         }
-        fast_cheb_s01<T>(g, make_shape(g, sh.ty, (int)sh.nblocks(), 1), B, Y, cy, done, s);   // scalar tiles
+        cheb_s01_launch<T, NEU>(g, make_shape(g, sh.ty, (int)sh.nblocks(), 1), B, Y, cy, done, s);   // scalar tiles
         return;
     }
     if constexpr (std::is_same<T, double>::value) {
         if (iso_coef(cy)) {   // equal spacings: the neighbour sum on the integer pipe
             const Shape c1 = sh.cx == 1 ? sh : make_shape(g, sh.ty, (int)sh.nblocks(), 1);
-            launch_pdl(k_cheb_iso64<0>, grid_of(c1), block_of(c1), 0, s, g, c1, B, nullptr, nullptr, Y, c, done);
+            launch_pdl(k_cheb_iso64<0, NEU>, grid_of(c1), block_of(c1), 0, s, g, c1, B, nullptr, nullptr, Y, c, done);
             PPS_COUNT_LAUNCH();
             return;
         }
     }
-    if (sh.cx == 2) launch_pdl(k_cheb_s01<T, 2>, grid_of(sh), block_of(sh), 0, s, g, sh, B, Y, c, done);
-    else launch_pdl(k_cheb_s01<T, 1>, grid_of(sh), block_of(sh), 0, s, g, sh, B, Y, c, done);
+    if (sh.cx == 2) launch_pdl(k_cheb_s01<T, 2, NEU>, grid_of(sh), block_of(sh), 0, s, g, sh, B, Y, c, done);
+    else launch_pdl(k_cheb_s01<T, 1, NEU>, grid_of(sh), block_of(sh), 0, s, g, sh, B, Y, c, done);
     PPS_COUNT_LAUNCH();
 }
 template <typename T>
-void fast_cheb_sweep(const Geo& g, const Shape& sh, const T* Y, const T* B, const T* Z, T* W, const Coef& cf,
-                     const int* done, cudaStream_t s)
+void fast_cheb_s01(const Geo& g, const Shape& sh, const T* B, T* Y, const Coef& cy, const int* done, cudaStream_t s,
+                   bool mirror)
+{
+    if (mirror && has_neumann(g)) cheb_s01_launch<T, true>(g, sh, B, Y, cy, done, s);
+    else cheb_s01_launch<T, false>(g, sh, B, Y, cy, done, s);
+}
+
+template <typename T, bool NEU>
+static void cheb_sweep_launch(const Geo& g, const Shape& sh, const T* Y, const T* B, const T* Z, T* W, const Coef& cf,
+                              const int* done, cudaStream_t s)
 {
     const CT<T> c = cast_coef<T>(cf);
     if (sh.cx == 4) {
         if constexpr (std::is_same<T, float>::value) {
             if (v4_ok<T>(g, Y, B, Z, W)) {
-                if (Z) launch_pdl(k_cheb_v4<2>, grid_of(sh), block_of(sh), 0, s, g, sh, Y, B, Z, W, c, done);
-                else launch_pdl(k_cheb_v4<1>, grid_of(sh), block_of(sh), 0, s, g, sh, Y, B, Z, W, c, done);
+                if (Z) launch_pdl(k_cheb_v4<2, NEU>, grid_of(sh), block_of(sh), 0, s, g, sh, Y, B, Z, W, c, done);
+                else launch_pdl(k_cheb_v4<1, NEU>, grid_of(sh), block_of(sh), 0, s, g, sh, Y, B, Z, W, c, done);
                 PPS_COUNT_LAUNCH();
                 return;
             }
         }
-        fast_cheb_sweep<T>(g, make_shape(g, sh.ty, (int)sh.nblocks(), 1), Y, B, Z, W, cf, done, s);   // scalar tiles
+        cheb_sweep_launch<T, NEU>(g, make_shape(g, sh.ty, (int)sh.nblocks(), 1), Y, B, Z, W, cf, done, s);   // scalar tiles
         return;
     }
     if constexpr (std::is_same<T, double>::value) {
         if (iso_coef(cf)) {   // equal spacings: the neighbour sum on the integer pipe
             const Shape c1 = sh.cx == 1 ? sh : make_shape(g, sh.ty, (int)sh.nblocks(), 1);
-            if (Z) launch_pdl(k_cheb_iso64<2>, grid_of(c1), block_of(c1), 0, s, g, c1, Y, B, Z, W, c, done);
-            else launch_pdl(k_cheb_iso64<1>, grid_of(c1), block_of(c1), 0, s, g, c1, Y, B, Z, W, c, done);
+            if (Z) launch_pdl(k_cheb_iso64<2, NEU>, grid_of(c1), block_of(c1), 0, s, g, c1, Y, B, Z, W, c, done);
+            else launch_pdl(k_cheb_iso64<1, NEU>, grid_of(c1), block_of(c1), 0, s, g, c1, Y, B, Z, W, c, done);
             PPS_COUNT_LAUNCH();
             return;
         }
     }
     if (Z) {
-        if (sh.cx == 2) launch_pdl(k_cheb_sweep<T, 2, true>, grid_of(sh), block_of(sh), 0, s, g, sh, Y, B, Z, W, c, done);
-        else launch_pdl(k_cheb_sweep<T, 1, true>, grid_of(sh), block_of(sh), 0, s, g, sh, Y, B, Z, W, c, done);
+        if (sh.cx == 2) launch_pdl(k_cheb_sweep<T, 2, true, NEU>, grid_of(sh), block_of(sh), 0, s, g, sh, Y, B, Z, W, c, done);
+        else launch_pdl(k_cheb_sweep<T, 1, true, NEU>, grid_of(sh), block_of(sh), 0, s, g, sh, Y, B, Z, W, c, done);
     } else {
-        if (sh.cx == 2) launch_pdl(k_cheb_sweep<T, 2, false>, grid_of(sh), block_of(sh), 0, s, g, sh, Y, B, Z, W, c, done);
-        else launch_pdl(k_cheb_sweep<T, 1, false>, grid_of(sh), block_of(sh), 0, s, g, sh, Y, B, Z, W, c, done);
+        if (sh.cx == 2) launch_pdl(k_cheb_sweep<T, 2, false, NEU>, grid_of(sh), block_of(sh), 0, s, g, sh, Y, B, Z, W, c, done);
+        else launch_pdl(k_cheb_sweep<T, 1, false, NEU>, grid_of(sh), block_of(sh), 0, s, g, sh, Y, B, Z, W, c, done);
     }
     PPS_COUNT_LAUNCH();
+}
+template <typename T>
+void fast_cheb_sweep(const Geo& g, const Shape& sh, const T* Y, const T* B, const T* Z, T* W, const Coef& cf,
+                     const int* done, cudaStream_t s, bool mirror)
+{
+    if (mirror && has_neumann(g)) cheb_sweep_launch<T, true>(g, sh, Y, B, Z, W, cf, done, s);
+    else cheb_sweep_launch<T, false>(g, sh, Y, B, Z, W, cf, done, s);
 }
 template <typename T>
 void fast_cheb_fused(const Geo& g, int nsteps, const T* B, T* X, const Coef* c, const int* done, cudaStream_t s)
@@ -2831,9 +2881,9 @@ void state_init(DevState* st, double* hist, int maxit, double tol_abs, double to
 
 #define PPS_INST(T)                                                                                              \
     template void fast_cheb_s01<T>(const Geo&, const Shape&, const T*, T*, const Coef&, const int*,               \
-                                   cudaStream_t);                                                                \
+                                   cudaStream_t, bool);                                                              \
     template void fast_cheb_sweep<T>(const Geo&, const Shape&, const T*, const T*, const T*, T*, const Coef&,    \
-                                     const int*, cudaStream_t);                                                  \
+                                     const int*, cudaStream_t, bool);                                            \
     template void fast_scale_copy<T>(const Geo&, const Shape&, const T*, T*, double, const int*, cudaStream_t); \
     template void fast_stencil_dot<T>(const Geo&, const Shape&, const T*, const T*, T*, const Coef&, RedCtx,     \
                                       cudaStream_t);                                                             \

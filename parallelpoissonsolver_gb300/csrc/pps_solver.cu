@@ -666,8 +666,10 @@ struct Launcher {
 // One preconditioner application X = M^{-1} B in storage type T.  The two last
 // sweeps of the reference are dead (its output is s_{n-2}, chebyshevIteration.hpp:
 // 114-125), so sweeps run for i = 2..n-2 and the last one writes X = -s_{n-2}.
+// mirror: X's ghost points at Neumann faces are filled as well (the stencil that follows
+// reads them; CG's do not, and its z keeps the ghosts it has).
 template <typename T>
-void fast_cheb(pps_solver* s, Fields<T>& F, T* B, T* X, Launcher& L, const ChebP& p);
+void fast_cheb(pps_solver* s, Fields<T>& F, T* B, T* X, Launcher& L, const ChebP& p, bool mirror = false);
 
 template <typename T>
 void fast_inner_precond(pps_solver* s, T* B, T* X, Launcher& L, bool cg);
@@ -675,9 +677,14 @@ void fast_inner_precond(pps_solver* s, T* B, T* X, Launcher& L, bool cg);
 // The preconditioner s->prec_kind names: the identity, the Chebyshev polynomial,
 // or the inner BiCGSTAB solve.
 template <typename T>
-void fast_precond(pps_solver* s, Fields<T>& F, T* B, T* X, Launcher& L)
+void fast_precond(pps_solver* s, Fields<T>& F, T* B, T* X, Launcher& L, bool mirror = false)
 {
     const Geo& g = s->geo;
+    if (mirror && s->has_neumann && s->prec_kind != PPS_PREC_CHEBYSHEV) {
+        fast_precond<T>(s, F, B, X, L, false);
+        neumann_fill<T>(g, X, faces_of(s), 0, 1.0, s->stream);
+        return;
+    }
     if (s->prec_kind == PPS_PREC_NONE) {
         CK(cudaMemcpyAsync(X, B, sizeof(T) * (size_t)g.ntot, cudaMemcpyDeviceToDevice, s->stream));
         L.bytes += bytes_of<T>(g.ntot, 2);
@@ -687,12 +694,12 @@ void fast_precond(pps_solver* s, Fields<T>& F, T* B, T* X, Launcher& L)
         fast_inner_precond<T>(s, B, X, L, s->prec_kind == PPS_PREC_CG);
         return;
     }
-    fast_cheb<T>(s, F, B, X, L, cheb_of(s));
+    fast_cheb<T>(s, F, B, X, L, cheb_of(s), mirror);
 }
 
 // X = -s_{n-2} of the Chebyshev recurrence p on B (the preconditioner, or a smoother).
 template <typename T>
-void fast_cheb(pps_solver* s, Fields<T>& F, T* B, T* X, Launcher& L, const ChebP& p)
+void fast_cheb(pps_solver* s, Fields<T>& F, T* B, T* X, Launcher& L, const ChebP& p, bool mirror)
 {
     const Geo& g = s->geo;
     cudaStream_t st = s->stream;
@@ -700,7 +707,7 @@ void fast_cheb(pps_solver* s, Fields<T>& F, T* B, T* X, Launcher& L, const ChebP
     const int* done = &s->d_st->done;
     if (s->has_neumann) {
         neumann_fill<T>(g, B, faces_of(s), 0, 1.0, st);
-        L.launches += 2;
+        L.launches++;
     }
     const Coef a = op_coef(g);
     const int n = p.n;
@@ -708,13 +715,14 @@ void fast_cheb(pps_solver* s, Fields<T>& F, T* B, T* X, Launcher& L, const ChebP
     double rhoOld = 1 / sigma;
     double rhoCurr = 1 / (2 * sigma - rhoOld);
     if (n == 1) {
-        fill_field<T>(X, g.ntot, (T)(-0.0), st);
+        fill_field<T>(X, g.ntot, (T)(-0.0), st);   // its ghost points too
         L.bytes += bytes_of<T>(g.ntot, 1);
         L.launches++;
         return;
     }
     if (n == 2) {
         fast_scale_copy<T>(g, s->shape, B, X, -1.0 / p.theta, done, st);
+        if (mirror && s->has_neumann) neumann_fill<T>(g, X, faces_of(s), 0, 1.0, st);
         L.bytes += bytes_of<T>(N, 2);
         L.launches++;
         return;
@@ -723,7 +731,7 @@ void fast_cheb(pps_solver* s, Fields<T>& F, T* B, T* X, Launcher& L, const ChebP
     Coef c01 = cheb_s01_coef(a, p, rhoCurr);
     if (n == 3) {
         c01.scale = -1.0;
-        fast_cheb_s01<T>(g, shc, B, X, c01, done, st);
+        fast_cheb_s01<T>(g, shc, B, X, c01, done, st, mirror);
         L.bytes += bytes_of<T>(N, 2);
         L.launches++;
         return;
@@ -766,10 +774,6 @@ void fast_cheb(pps_solver* s, Fields<T>& F, T* B, T* X, Launcher& L, const ChebP
     for (int it = 2; it <= n - 2; it++) {
         rhoOld = rhoCurr;
         rhoCurr = 1 / (2 * sigma - rhoOld);
-        if (s->has_neumann) {
-            neumann_fill<T>(g, Y, faces_of(s), 0, 1.0, st);
-            L.launches += 2;
-        }
         const bool last = (it == n - 2);
         Coef c = cheb_sweep_coef(a, p, rhoCurr, rhoOld, last ? -1.0 : 1.0);
         const bool first = (it == 2);
@@ -778,7 +782,7 @@ void fast_cheb(pps_solver* s, Fields<T>& F, T* B, T* X, Launcher& L, const ChebP
             c.cb += c.cw / p.theta;
             c.cw = 0.0;
         }
-        fast_cheb_sweep<T>(g, shc, Y, B, first ? nullptr : Z, last ? X : W, c, done, st);
+        fast_cheb_sweep<T>(g, shc, Y, B, first ? nullptr : Z, last ? X : W, c, done, st, !last || mirror);
         const int words = first ? 3 : 4;
         L.bytes += bytes_of<T>(N, words);
         L.launches++;
@@ -1037,14 +1041,12 @@ void fast_bicgstab_iteration(pps_solver* s, Fields<T>& F, T* xacc, Launcher& L)
     cudaStream_t st = s->stream;
     const long long N = s->n_unknowns;
     const Coef a = op_coef(g);
-    fast_precond<T>(s, F, F.p, F.Mp, L);
-    if (s->has_neumann) neumann_fill<T>(g, F.Mp, faces_of(s), 0, 1.0, st);
+    fast_precond<T>(s, F, F.p, F.Mp, L, true);
     // the stencils run on the Chebyshev tiles (x-vectorised for FP32); the updates
     // are flat 16-byte vector passes on Dirichlet grids
     fast_stencil_dot<T>(g, s->shape_cheb, F.Mp, F.r0, F.AMp, a, red_c(s, FIN_ALPHA), st);
     fast_axpy_alpha<T>(g, sh, F.r, F.AMp, s->d_st, st);
-    fast_precond<T>(s, F, F.r, F.z, L);
-    if (s->has_neumann) neumann_fill<T>(g, F.z, faces_of(s), 0, 1.0, st);
+    fast_precond<T>(s, F, F.r, F.z, L, true);
     fast_stencil_dot2<T>(g, s->shape_cheb, F.z, F.r, F.Az, a, red_c(s, FIN_OMEGA), st);
     fast_update_xr<T>(g, sh, xacc, F.Mp, F.z, F.r, F.Az, F.r0, red_c(s, FIN_CONV), st);
     fast_update_p<T>(g, sh, F.p, F.r, F.AMp, s->d_st, st);
