@@ -71,11 +71,11 @@ struct pps_batch {
     float *p = nullptr, *r = nullptr, *r0 = nullptr, *Mp = nullptr, *AMp = nullptr, *z = nullptr, *Az = nullptr;
     float *Y = nullptr, *Z = nullptr, *W = nullptr, *e = nullptr;
     BProb* dprob = nullptr;
-    unsigned* dblk = nullptr;
+    BItem* dblk = nullptr;
     unsigned blk_cap = 0;
     // the Chebyshev kernels' table (v4 tiles where chosen)
     BProb* dprob4 = nullptr;
-    unsigned* dblk4 = nullptr;
+    BItem* dblk4 = nullptr;
     unsigned blk_cap4 = 0;
     double* partials = nullptr;
     unsigned* counters = nullptr;
@@ -117,16 +117,38 @@ BProb make_prob(const Geo& g, long long off, const SizeTile& t, bool cheb)
     P.nchunks = (uz + P.kchunk - 1) / P.kchunk;
     P.nblocks = (unsigned)P.ntx * P.nty * P.nchunks;
     P.first_block = 0;
+    const double ix = 1.0 / (g.ds[0] * g.ds[0]), iy = 1.0 / (g.ds[1] * g.ds[1]), iz = 1.0 / (g.ds[2] * g.ds[2]);
+    const double a[4] = {-2.0 * (ix + iy + iz), ix, iy, iz};
+    for (int q = 0; q < 4; q++) {
+        P.a64[q] = a[q];
+        P.a32[q] = (float)a[q];
+    }
     return P;
 }
 
-// Builds the problem table and the block -> problem map for the problems in
+// Planes per z-chunk before any tuning: the longest of 32, 16, 8, 4 that gives the
+// batch 6 blocks per SM (8 fit).  24 problems of 17-63 per axis: chunks of 32 / 8 / 4
+// solve in 17.9 / 14.3 / 16.4 ms; 40 of 47-71 in 62 ms with any of 16 to 64.
+int default_kchunk(const pps_batch* s)
+{
+    int kc = 32;
+    for (; kc > 4; kc /= 2) {
+        long long blocks = 0;
+        for (const Geo& g : s->geo)
+            blocks += (long long)((g.hi[0] - g.lo[0] + 31) / 32) * ((g.hi[1] - g.lo[1] + 7) / 8) *
+                      ((g.hi[2] - g.lo[2] + kc - 1) / kc);
+        if (blocks >= 6LL * sm_count()) break;
+    }
+    return kc;
+}
+
+// Builds the problem table and the block -> work table for the problems in
 // `which` (biggest first, so the longest items start first), uploads them: the
 // table of every kernel, or (cheb) the Chebyshev kernels' own.
 BatchDev build_table(pps_batch* s, const std::vector<int>& which, bool cheb = false)
 {
     BProb*& dprob = cheb ? s->dprob4 : s->dprob;
-    unsigned*& dblk = cheb ? s->dblk4 : s->dblk;
+    BItem*& dblk = cheb ? s->dblk4 : s->dblk;
     unsigned& cap = cheb ? s->blk_cap4 : s->blk_cap;
     const BatchDev& previous = cheb ? s->B4 : s->B;
     std::vector<int> order = which;
@@ -138,13 +160,18 @@ BatchDev build_table(pps_batch* s, const std::vector<int>& which, bool cheb = fa
         return na > nc;
     });
     std::vector<BProb> hp((size_t)s->nprob);
-    std::vector<unsigned> blk;
+    std::vector<BItem> blk;
     for (int p = 0; p < s->nprob; p++)
         hp[(size_t)p] = make_prob(s->geo[(size_t)p], s->off[(size_t)p], s->tiles[key_of(s->geo[(size_t)p])], cheb);
     for (int p : order) {
         BProb& P = hp[(size_t)p];
         P.first_block = (unsigned)blk.size();
-        for (unsigned q = 0; q < P.nblocks; q++) blk.push_back((unsigned)p);
+        for (int k = 0; k < P.nchunks; k++)
+            for (int t = 0; t < P.ntx * P.nty; t++) {
+                const int bx = t % P.ntx, by = t / P.ntx;
+                blk.push_back(BItem{p, P.cx == 4 ? bx * 128 : P.g.lo[0] + bx * 32 * P.cx, P.g.lo[1] + by * 8,
+                                    P.g.lo[2] + k * P.kchunk});
+            }
     }
     if (blk.size() > cap) {
         if (s->gexec) {   // a captured graph holds the old table pointers
@@ -153,18 +180,18 @@ BatchDev build_table(pps_batch* s, const std::vector<int>& which, bool cheb = fa
         }
         if (dblk) cudaFree(dblk);
         cap = (unsigned)blk.size();
-        BK(cudaMalloc((void**)&dblk, sizeof(unsigned) * cap));
+        BK(cudaMalloc((void**)&dblk, sizeof(BItem) * cap));
         if (!cheb) {   // block partials of the reductions (the Chebyshev kernels reduce nothing)
             if (s->partials) cudaFree(s->partials);
             BK(cudaMalloc((void**)&s->partials, sizeof(double) * 4 * (size_t)cap));
         }
     }
     BK(cudaMemcpyAsync(dprob, hp.data(), sizeof(BProb) * hp.size(), cudaMemcpyHostToDevice, s->stream));
-    BK(cudaMemcpyAsync(dblk, blk.data(), sizeof(unsigned) * blk.size(), cudaMemcpyHostToDevice, s->stream));
+    BK(cudaMemcpyAsync(dblk, blk.data(), sizeof(BItem) * blk.size(), cudaMemcpyHostToDevice, s->stream));
     BK(cudaStreamSynchronize(s->stream));
     BatchDev B;
     B.prob = dprob;
-    B.blk2prob = dblk;
+    B.item = dblk;
     B.nprob = s->nprob;
     B.total_blocks = (unsigned)blk.size();
     if (s->gexec && B.total_blocks != previous.total_blocks) {   // the graph was captured for another table
@@ -527,8 +554,10 @@ pps_status pps_batch_create(int nprob, const pps_grid* grids, const pps_config* 
             s->theta[(size_t)p] = th;
             s->delta[(size_t)p] = de;
             s->sigma[(size_t)p] = th / de;
-            s->tiles[key_of(g)] = SizeTile();
         }
+        SizeTile def;
+        def.kchunk = default_kchunk(s);
+        for (const Geo& g : s->geo) s->tiles[key_of(g)] = def;
         s->pool = pool;
         BK(cudaMalloc((void**)&s->x, sizeof(double) * (size_t)pool));
         BK(cudaMalloc((void**)&s->b, sizeof(double) * (size_t)pool));

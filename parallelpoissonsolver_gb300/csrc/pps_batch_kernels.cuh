@@ -2,9 +2,11 @@
 // Included by pps_kernels.cu (same translation unit: shares Acc, finalize, CT).
 //
 // Every field of every problem lives in one pooled array at the problem's offset.
-// A launch has one thread block per (problem, tile, z-chunk) work item; the
-// block -> problem table `blk2prob` maps a block to its problem, whose own tile
-// shape (columns per thread cx, z-chunk) the autotuner picked for its grid size.
+// A launch has one thread block per (problem, tile, z-chunk) work item; the table
+// `item` maps a block to its problem, first column and plane (one load; the problem's
+// geometry, stop flag and coefficients are then fetched together: on small problems a
+// block's time is this chain of dependent loads).  The tile shape (columns per thread
+// cx, z-chunk) is the problem's, by its grid size.
 // Reductions are per problem: block partials in launch order, a per-problem
 // completion counter, and the problem's last block sums its partials in block
 // order and advances that problem's scalars.  A problem whose stop flag is set is
@@ -21,18 +23,15 @@ struct BCol {
 __device__ __forceinline__ BCol bcolumn(const BatchDev& B)
 {
     BCol q;
-    q.p = B.blk2prob[blockIdx.x];
+    const int4 it = __ldg(reinterpret_cast<const int4*>(B.item) + blockIdx.x);
+    q.p = it.x;
     q.P = &B.prob[q.p];
     const BProb& P = *q.P;
-    const unsigned local = blockIdx.x - P.first_block;
-    const unsigned tiles = (unsigned)P.ntx * (unsigned)P.nty;
-    const unsigned tile = local % tiles, chunk = local / tiles;
-    const int bx = (int)(tile % (unsigned)P.ntx), by = (int)(tile / (unsigned)P.ntx);
     q.cx = P.cx;
     // cx 4: the x-vectorised Chebyshev tiles, a float4 per thread from x = 0
-    q.i = P.cx == 4 ? bx * 128 + threadIdx.x * 4 : P.g.lo[0] + bx * 32 * P.cx + threadIdx.x;
-    q.j = P.g.lo[1] + by * (int)blockDim.y + threadIdx.y;
-    q.k0 = P.g.lo[2] + (int)chunk * P.kchunk;
+    q.i = it.y + threadIdx.x * (P.cx == 4 ? 4 : 1);
+    q.j = it.z + threadIdx.y;
+    q.k0 = it.w;
     q.k1 = min(q.k0 + P.kchunk, P.g.hi[2]);
     q.active = q.j < P.g.hi[1];
     q.c = P.off + q.i + P.g.sj * q.j + P.g.sk * q.k0;
@@ -197,8 +196,7 @@ __global__ void __launch_bounds__(256) bk_residual(BatchDev B, const double* __r
     const BCol q = bcolumn(B);
     BSKIP_FINISHED(bst, q);
     const Geo& g = q.P->g;
-    const double ix = 1.0 / (g.ds[0] * g.ds[0]), iy = 1.0 / (g.ds[1] * g.ds[1]), iz = 1.0 / (g.ds[2] * g.ds[2]);
-    const double cc = -2.0 * (ix + iy + iz);
+    const double cc = q.P->a64[0], ix = q.P->a64[1], iy = q.P->a64[2], iz = q.P->a64[3];
     double s = 0.0;
     if (q.active) {
         for (int u = 0; u < q.cx; u++) {
@@ -262,9 +260,9 @@ __global__ void __launch_bounds__(256) bk_cheb_s01(BatchDev B, const float* __re
 {
     pdl_enter();
     const BCol q = bcolumn(B);
+    const CT<float> cf = coef[(size_t)q.p * cstride + ci];
     BSKIP_INNER(bst, q);
     if (!q.active) return;
-    const CT<float> cf = coef[(size_t)q.p * cstride + ci];
     const Geo& g = q.P->g;
     if (q.cx == 4) {   // the block's rows are whole warps: all lanes reach the shuffles
         cheb_v4_march<0>(g, q.i, q.j, q.k0, q.k1, q.c, Bf, nullptr, nullptr, Y, cf);
@@ -298,9 +296,9 @@ __global__ void __launch_bounds__(256) bk_cheb_sweep(BatchDev B, const float* __
 {
     pdl_enter();
     const BCol q = bcolumn(B);
+    const CT<float> cf = coef[(size_t)q.p * cstride + ci];
     BSKIP_INNER(bst, q);
     if (!q.active) return;
-    const CT<float> cf = coef[(size_t)q.p * cstride + ci];
     const Geo& g = q.P->g;
     if (q.cx == 4) {
         cheb_v4_march<HAS_Z ? 2 : 1>(g, q.i, q.j, q.k0, q.k1, q.c, Y, Bf, Z, W, cf);
@@ -338,10 +336,7 @@ __global__ void __launch_bounds__(256) bk_stencil_dot(BatchDev B, const float* _
     const BCol q = bcolumn(B);
     BSKIP_INNER(bst, q);
     const Geo& g = q.P->g;
-    const float ix = (float)(1.0 / (g.ds[0] * g.ds[0])), iy = (float)(1.0 / (g.ds[1] * g.ds[1])),
-                iz = (float)(1.0 / (g.ds[2] * g.ds[2]));
-    const float cc = (float)(-2.0 * (1.0 / (g.ds[0] * g.ds[0]) + 1.0 / (g.ds[1] * g.ds[1]) +
-                                    1.0 / (g.ds[2] * g.ds[2])));
+    const float cc = q.P->a32[0], ix = q.P->a32[1], iy = q.P->a32[2], iz = q.P->a32[3];
     Acc<float> a1, a2;
     if (q.active) {
         const long long sj = g.sj, sk = g.sk;

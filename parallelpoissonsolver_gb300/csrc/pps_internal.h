@@ -194,11 +194,20 @@ struct BProb {
     long long off;
     unsigned first_block, nblocks;
     int ntx, nty, nchunks, kchunk, cx;
+    // the operator's weights: centre, x, y, z (formed on the host: six FP64 divisions in
+    // every thread cost more than the rest of a small problem's pass)
+    double a64[4];
+    float a32[4];
+};
+
+// One launch block's work: its problem, first column and first plane.
+struct alignas(16) BItem {
+    int p, i0, j0, k0;
 };
 
 struct BatchDev {
     const BProb* prob;
-    const unsigned* blk2prob;   // launch block -> problem
+    const BItem* item;   // launch block -> work
     int nprob;
     unsigned total_blocks;
 };
