@@ -361,6 +361,9 @@ template <typename T>
 void fast_bicg_start(const Geo& g, const Shape& sh, const T* B, T* r, T* r0, T* p, RedCtx rc, cudaStream_t s);
 // out = (float)in over a whole field.
 void cast_field_f32(const double* in, float* out, long long n, cudaStream_t s);
+// out = r - A z at the unknowns on equal spacings (false, and nothing done, on others).
+bool fast_field_residual_iso64(const Geo& g, const double* r, const double* z, double* out, const Coef& a, const int* stop,
+                               cudaStream_t s);
 template <typename T>
 void fill_field(T* p, long long n, T v, cudaStream_t s);
 // Zero the boundary nodes and guard layers of a padded field.

@@ -1714,6 +1714,31 @@ __global__ void __launch_bounds__(256) k_fcg_update_xr_flat(long long n, T* __re
     reduce_finalize<1>(v, rc);
 }
 
+// FCG's direction alone: p_out = z + beta p_in (z on a restart, beta = 0).
+template <typename T>
+__global__ void __launch_bounds__(256) k_fcg_p_flat(long long n, const T* __restrict__ z, const T* __restrict__ pin,
+                                                    T* __restrict__ pout, const DevState* st)
+{
+    pdl_enter();
+    EARLY_EXIT(&st->done);
+    typedef Vec16<T> VT;
+    typedef typename VT::type V;
+    const bool restart = st->beta == 0.0;
+    const T be = (T)st->beta;
+    const long long nv = n / VT::n, stride = (long long)gridDim.x * blockDim.x;
+    const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    for (long long i = t0; i < nv; i += stride) {
+        V zv = reinterpret_cast<const V*>(z)[i];
+        if (!restart) {
+            V pv = reinterpret_cast<const V*>(pin)[i];
+#pragma unroll
+            for (int e = 0; e < VT::n; e++) VT::at(zv, e) = fmx(be, VT::at(pv, e), VT::at(zv, e));
+        }
+        reinterpret_cast<V*>(pout)[i] = zv;
+    }
+    for (long long i = nv * VT::n + t0; i < n; i += stride) pout[i] = restart ? z[i] : fmx(be, pin[i], z[i]);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256) k_fcg_dot_flat(long long n, const T* __restrict__ r, const T* __restrict__ z,
                                                       const T* __restrict__ Ap, RedCtx rc)
@@ -2074,6 +2099,51 @@ __global__ void __launch_bounds__(256, 4) k_stencil_dots_iso64(Geo g, Shape sh, 
     v[0] = a1.value();
     if (NS == 2) v[NS - 1] = a2.value();
     reduce_emit<NS>(v, rc, sh);
+}
+
+// out = r - A z at the unknowns (equal spacings, the neighbour sum on the integer pipe).
+__global__ void __launch_bounds__(256) k_field_residual_iso64(Geo g, Shape sh, const double* __restrict__ r,
+                                                              const double* __restrict__ z, double* __restrict__ out,
+                                                              Coef cf, const int* __restrict__ stop)
+{
+    pdl_enter();
+    EARLY_EXIT(stop);
+    const Col q = column(g, sh);
+    if (!q.active) return;
+    const long long sj = g.sj, sk = g.sk;
+    long long c = q.c;
+    double um = z[c - sk], uc = z[c];
+    MI mm = msplit(um), mc = msplit(uc);
+#pragma unroll 2
+    for (int k = q.k0; k < q.k1; k++) {
+        const double up = z[c + sk];
+        const double xw = z[c - 1], xe = z[c + 1], ys = z[c - sj], yn = z[c + sj];
+        const MI mp = msplit(up);
+        double s6, a;
+        if (nsum6<true>(msplit(xw), msplit(xe), msplit(ys), msplit(yn), mm, mp, s6)) {
+            a = fmx(cf.cx, s6, cf.cc * uc);
+        } else {
+            a = cf.cc * uc;
+            a = fmx(cf.cx, xw + xe, a);
+            a = fmx(cf.cy, ys + yn, a);
+            a = fmx(cf.cz, um + up, a);
+        }
+        out[c] = r[c] - a;
+        um = uc;
+        uc = up;
+        mm = mc;
+        mc = mp;
+        c += sk;
+    }
+}
+bool fast_field_residual_iso64(const Geo& g, const double* r, const double* z, double* out, const Coef& a, const int* stop,
+                               cudaStream_t s)
+{
+    if (!iso_coef(a)) return false;
+    const Shape sh = make_shape(g, 8, sm_count() * 16);
+    launch_pdl(k_field_residual_iso64, grid_of(sh), block_of(sh), 0, s, g, sh, r, z, out, a, stop);
+    PPS_COUNT_LAUNCH();
+    return true;
 }
 
 // Counts the entries of a whole field (guard layers included) whose bit pattern is
@@ -2601,6 +2671,16 @@ static bool flat_ok(const Geo& g, std::initializer_list<const void*> ptrs)
         if (((uintptr_t)p & 15u) != 0) return false;
     return true;
 }
+// Blocks of a flat pass that ends in a reduction: at most the shape's, each with 8
+// vectors per thread or more.  Every block pays a shuffle tree and a chain of FP64
+// additions (2 lanes per clock and SM on GB300) for its sums: on 128^3 doubles one
+// vector per thread, 4096 blocks, took 68 us for z.r, z.Ap, r.r against 26 us with 561.
+template <typename T>
+static unsigned flat_red_blocks(const Geo& g, const Shape& sh)
+{
+    const long long vecs = g.ntot / Vec16<T>::n, per = 8LL * 32 * sh.ty;
+    return (unsigned)std::max(1LL, std::min((long long)sh.nblocks(), (vecs + per - 1) / per));
+}
 template <typename T>
 void fast_axpy_alpha(const Geo& g, const Shape& sh, T* r, const T* v, const DevState* st, cudaStream_t s)
 {
@@ -2625,7 +2705,7 @@ void fast_update_xr(const Geo& g, const Shape& sh, T* x, const T* Mp, const T* z
         return;
     }
     if (flat_ok(g, {x, Mp, z, r, Az, r0})) {
-        launch_pdl(k_update_xr_flat<T>, sh.nblocks(), 32 * sh.ty, 0, s, g.ntot, x, Mp, z, r, Az, r0, rc);
+        launch_pdl(k_update_xr_flat<T>, flat_red_blocks<T>(g, sh), 32 * sh.ty, 0, s, g.ntot, x, Mp, z, r, Az, r0, rc);
         PPS_COUNT_LAUNCH();
         return;
     }
@@ -2702,13 +2782,13 @@ template <typename T>
 void fast_fcg_update_xr_flat(const Geo& g, const Shape& sh, T* x, const T* p, T* r, const T* Ap, RedCtx rc,
                              cudaStream_t s)
 {
-    launch_pdl(k_fcg_update_xr_flat<T>, sh.nblocks(), 32 * sh.ty, 0, s, g.ntot, x, p, r, Ap, rc);
+    launch_pdl(k_fcg_update_xr_flat<T>, flat_red_blocks<T>(g, sh), 32 * sh.ty, 0, s, g.ntot, x, p, r, Ap, rc);
     PPS_COUNT_LAUNCH();
 }
 template <typename T>
 void fast_fcg_dot_flat(const Geo& g, const Shape& sh, const T* r, const T* z, const T* Ap, RedCtx rc, cudaStream_t s)
 {
-    launch_pdl(k_fcg_dot_flat<T>, sh.nblocks(), 32 * sh.ty, 0, s, g.ntot, r, z, Ap, rc);
+    launch_pdl(k_fcg_dot_flat<T>, flat_red_blocks<T>(g, sh), 32 * sh.ty, 0, s, g.ntot, r, z, Ap, rc);
     PPS_COUNT_LAUNCH();
 }
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -2775,6 +2855,17 @@ void fast_fcg_p_stencil(const Geo& g, const Shape& sh, const T* z, const T* pin,
         }
         fast_fcg_p_stencil<T>(g, make_shape(g, sh.ty, (int)sh.nblocks(), 1), z, pin, pout, Ap, a, rc, s, staged);
         return;
+    }
+    if constexpr (std::is_same<T, double>::value) {
+        if (iso_coef(a) && flat_ok(g, {z, pin, pout})) {
+            // FP64 on equal spacings: forming p at every tap costs 7 FP64 operations per
+            // unknown and the plain stencil 8 more; p stored by a pass of its own leaves
+            // 3 to the stencil on the integer pipe (128^3: 82 -> 44 us for both)
+            launch_pdl(k_fcg_p_flat<T>, sm_count() * 8, 256, 0, s, g.ntot, z, pin, pout, rc.st);
+            PPS_COUNT_LAUNCH();
+            fast_stencil_dot<T>(g, make_shape(g, sh.ty, sm_count() * 8, 1), pout, pout, Ap, a, rc, s);
+            return;
+        }
     }
     launch_pdl(k_fcg_p_stencil<T>, grid_of(sh), block_of(sh), 0, s, g, sh, z, pin, pout, Ap, a, rc);
     PPS_COUNT_LAUNCH();

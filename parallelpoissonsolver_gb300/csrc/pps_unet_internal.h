@@ -120,6 +120,8 @@ template <typename T>
 void field_axpy(const Geo& g, const Shape& sh, T* x, const T* y, cudaStream_t s);
 template <typename T>
 void field_residual_restrict(const Geo& g, const T* r, const T* z, const Dims& dc, float* coarse, cudaStream_t s);
+// coarse = R f of a stored FP64 field (the weights and sums of field_residual_restrict)
+void field_restrict(const Geo& g, const double* f, const Dims& dc, float* coarse, cudaStream_t s);
 // f += P coarse at the unknowns.  With `dots` (flexible CG's z = M r finished by this
 // prolongation) the FP32 float4 kernel also runs the z.r, z.Ap reduction `dots`
 // describes over the unknowns and the call returns true; otherwise (FP64, unaligned
