@@ -919,6 +919,420 @@ static bool v4_ok(const Geo& g, const void* a, const void* b, const void* c, con
     return true;
 }
 
+// Three Chebyshev steps in one pass over FP32 fields on a Dirichlet grid (temporal
+// blocking).  One step per launch is bound by HBM: 8, 12 or 16 bytes per unknown and
+// step, 132 for the nine of a degree-11 application; three at a time they move 48.
+// MODE 0: s1..s3 from B; 1: from Y = s1 without Z; 2: from Y, Z and B.  X = the third
+// step; TWO: X2 = the second, which the next pass reads as its Z.
+//
+// A block marches along z over a tile of 12 warps x 2 rows a thread, lw lanes of 4
+// points to a row, in a wavefront: when plane k of the input arrives, step t is computed
+// on plane k - t.  The z neighbours are the thread's own last two planes of step t-1 and
+// the one just computed, the x neighbours come by shuffle, the y neighbours from the
+// thread's other row or through shared memory (each thread stores its two rows of steps
+// 0..2 once and reads two), so one barrier per plane orders everything.  Rows within 3 of
+// the tile's edge, and the quad at an interior edge along x, are computed for their
+// neighbours only.  Values off the unknowns are zero, as the work fields' guard cells
+// are, and the input is read as stored, its guard layer included.  Per point the
+// arithmetic is k_cheb_v4's in the same order (two points an instruction), so the
+// results are bit-identical.
+//
+// What bounds it: the shared-memory path (about 110 wavefronts a warp and plane) and
+// the issue slots, with half the work on halo points.  256^3, MODE 0 / 2 / 2: 100, 115,
+// 99 us against 118, 138, 138 for three launches of k_cheb_v4; a BiCGSTAB iteration
+// 1296 -> 1104 us, at 512^3 8.09 -> 6.13 ms.  One row a thread with 20 warps read the
+// shared memory half as often again (1284 us); fewer warps hide less latency (8: 1596
+// us); without the L2 prefetch the loads' latency shows (1281 us).
+constexpr int CHEB3_AHEAD = 2;   // planes brought into L2 ahead of the loads
+constexpr int CHEB3_WARPS = 12, CHEB3_R = 2;
+constexpr int CHEB3_THREADS = 32 * CHEB3_WARPS;
+constexpr int CHEB3_PITCH = CHEB3_THREADS + 64;   // 32 spare slots at either end
+constexpr int CHEB3_SMEM = 2 * 3 * 2 * CHEB3_PITCH * 16;
+
+struct Cheb3Tile {
+    int lw, lwlog;   // lanes of a row: 8, 16 or 32
+    int f0, f_own0, f_own1;   // first float4 of the tile along x; those it stores are [f_own0, f_own1)
+    int j0, j1;      // rows stored
+    int kb, ke;      // planes stored
+};
+// The steps' coefficients, each twice for the packed operations.
+struct Cheb3Coef {
+    struct {
+        float2 cc, cx, cy, cz, cb, cw;
+    } c[3];
+};
+
+// Two FP32 operations an instruction, each rounded as the single one.
+__device__ __forceinline__ float2 add2(float2 a, float2 b)
+{
+    float2 r;
+    asm("add.rn.f32x2 %0, %1, %2;"
+        : "=l"(*reinterpret_cast<unsigned long long*>(&r))
+        : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)));
+    return r;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b)
+{
+    float2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;"
+        : "=l"(*reinterpret_cast<unsigned long long*>(&r))
+        : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)));
+    return r;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
+{
+    float2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(*reinterpret_cast<unsigned long long*>(&r))
+        : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)),
+          "l"(*reinterpret_cast<unsigned long long*>(&c)));
+    return r;
+}
+__device__ __forceinline__ float2 lo2f(const float4& v) { return make_float2(v.x, v.y); }
+__device__ __forceinline__ float2 hi2f(const float4& v) { return make_float2(v.z, v.w); }
+
+// Loads of the next plane: volatile, so that they stay where they are issued, an
+// iteration before their use.
+template <bool A16>
+__device__ __forceinline__ float4 ld_quad(const float* p)
+{
+    float4 v;
+    if constexpr (A16) {
+        asm volatile("ld.global.nc.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    } else {
+        asm volatile("ld.global.nc.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+        asm volatile("ld.global.nc.v2.f32 {%0,%1}, [%2];" : "=f"(v.z), "=f"(v.w) : "l"(p + 2));
+    }
+    return v;
+}
+__device__ __forceinline__ void prefetch_l2(const float* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+__device__ __forceinline__ float keep(float v, unsigned ma, unsigned mb) { return __uint_as_float(__float_as_uint(v) & ma & mb); }
+
+template <int MODE, bool A16, bool TWO>
+__device__ __forceinline__ void cheb3_march(const Geo& g, const Cheb3Tile& T, const float* __restrict__ U,
+                                            const float* __restrict__ B, const float* __restrict__ Z,
+                                            float* __restrict__ X, float* __restrict__ X2, const Cheb3Coef& cs,
+                                            float4* sm)
+{
+    constexpr int NS = 3, R = CHEB3_R, PITCH = CHEB3_PITCH;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int tid = threadIdx.x, lw = T.lw;
+    const int l = tid & (lw - 1), trow = tid >> T.lwlog;
+    const int xlo = g.lo[0], xhi = g.hi[0], lo2 = g.lo[2];
+    const int f = T.f0 + l, x = (A16 ? 0 : xlo) + 4 * f, j = T.j0 - NS + trow * R;
+    const long long sk = g.sk;
+    const unsigned uz = (unsigned)(g.hi[2] - lo2);
+    // unknowns of the quad (x >= lo is implied without A16), and of each row
+    const unsigned mx0 = x >= xlo && x < xhi ? ~0u : 0u, mx1 = x + 1 >= xlo && x + 1 < xhi ? ~0u : 0u,
+                   mx2 = x + 2 < xhi ? ~0u : 0u, mx3 = x + 3 < xhi ? ~0u : 0u;
+    unsigned mrow[R], off[R];
+    bool own[R];
+    // Offset in a plane.  Threads beyond the grid load the nearest point of its guard
+    // layer instead: what they hold reaches no unknown but through the guard point itself
+    // (rows lo-1 and hi, x = hi), which is read as stored.
+    const int xc = A16 ? min(x, xhi & ~3) : min(x, xhi & ~1);
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const int jr = j + r;
+        mrow[r] = jr >= g.lo[1] && jr < g.hi[1] ? ~0u : 0u;
+        // a quad of even x holds an unknown when its first or third point is one
+        own[r] = mrow[r] && (mx0 | mx2) && f >= T.f_own0 && f < T.f_own1 && jr >= T.j0 && jr < T.j1;
+        off[r] = (unsigned)(xc + g.sj * min(max(jr, g.lo[1] - 1), g.hi[1]));
+    }
+    bool own4[R], own1[R];   // rows whose quad is stored whole, and in part
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        own4[r] = own[r] && (mx0 & mx1 & mx2 & mx3);
+        own1[r] = own[r] && !own4[r];
+    }
+    float4* slot = sm + 32 + tid;   // + ((buffer * 3 + step) * 2 + {0: the thread's first row, 1: its last}) * PITCH
+    for (int q = tid; q < 2 * NS * 2 * 64; q += CHEB3_THREADS) {
+        const int b = q / 64, e = q % 64;
+        sm[b * PITCH + (e < 32 ? e : CHEB3_THREADS + e)] = zero;
+    }
+    // the input just outside a row's ends, where no lane holds it (MODE 0: stored guard
+    // values; a work field's are zero)
+    const bool el = MODE == 0 && !A16 && f == 0, er = MODE == 0 && l == lw - 1 && x + 4 == xhi;
+    float4 m[NS][R], c[NS][R];   // steps 0..2 on their planes k-t-2 and k-t-1
+    float4 b1[R], b2[R], b3[R];  // B on planes k-1, k-2, k-3
+    float lc[R], rc[R];          // input outside the row's ends on plane k-1
+    float4 pu[R], pb[R], pz[R];
+    float pl[R], pr[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+#pragma unroll
+        for (int t = 0; t < NS; t++) m[t][r] = c[t][r] = zero;
+        b1[r] = b2[r] = b3[r] = pu[r] = pb[r] = pz[r] = zero;
+        lc[r] = rc[r] = pl[r] = pr[r] = 0.f;
+    }
+    const int k0 = T.kb - NS, k1 = T.ke + NS;
+    // the input's plane k; B and Z on plane k-1.  FAST: all of them in the grid
+    auto fetch = [&](int k, auto fast) {
+        constexpr bool FAST = decltype(fast)::value;
+        if (FAST || (unsigned)(k - lo2 + 1) < uz + 2) {
+            const float* P = U + sk * k;
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                pu[r] = ld_quad<A16>(P + off[r]);
+                if (el) pl[r] = P[off[r] - 1];
+                if (er) pr[r] = P[off[r] + 4];
+            }
+        } else {
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                pu[r] = zero;
+                pl[r] = pr[r] = 0.f;
+            }
+        }
+        if (k + CHEB3_AHEAD < g.hi[2]) {   // bring the planes after that into L2
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                prefetch_l2(U + sk * (k + CHEB3_AHEAD) + off[r]);
+                if (MODE >= 1) prefetch_l2(B + sk * (k + CHEB3_AHEAD - 1) + off[r]);
+                if (MODE == 2) prefetch_l2(Z + sk * (k + CHEB3_AHEAD - 1) + off[r]);
+            }
+        }
+        if (MODE >= 1 && (FAST || (unsigned)(k - 1 - lo2) < uz)) {
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                pb[r] = ld_quad<A16>(B + sk * (k - 1) + off[r]);
+                if (MODE == 2) pz[r] = ld_quad<A16>(Z + sk * (k - 1) + off[r]);
+            }
+        }
+    };
+    float4 *rd = slot, *wr = slot + NS * 2 * PITCH;
+    // Plane k arrives.  FAST: planes k-3 .. k+1 are unknowns or (k+1) the guard layer, and
+    // both stores are due, so the body has no branches but the stores of ragged quads.
+    auto plane = [&](int k, auto fast) {
+        constexpr bool FAST = decltype(fast)::value;
+        float4 up[R], z1[R], m0_old[R], m1_old[R];
+        float nl[R], nr[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            up[r] = pu[r];
+            z1[r] = pz[r];
+            nl[r] = pl[r];
+            nr[r] = pr[r];
+            m0_old[r] = m[0][r];
+            m1_old[r] = m[1][r];
+            if (MODE >= 1) {
+                b3[r] = b2[r];
+                b2[r] = b1[r];
+                b1[r] = pb[r];
+            }
+        }
+        fetch(k + 1, fast);   // in flight while this plane's steps run
+#pragma unroll
+        for (int t = 1; t <= NS; t++) {
+            const auto& cf = cs.c[t - 1];
+            const int p = k - t;
+            const bool on = FAST || (unsigned)(p - lo2) < uz;   // uniform
+            const bool st = (t == NS || (t == NS - 1 && TWO)) && (FAST || (unsigned)(p - T.kb) < (unsigned)(T.ke - T.kb));
+            float* o = (t == NS ? X : X2) + sk * p;
+            const float4 above = rd[(t - 1) * 2 * PITCH + PITCH - lw], below = rd[(t - 1) * 2 * PITCH + lw];
+            float4 w[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const float4 u = c[t - 1][r], um = m[t - 1][r], un = up[r];   // step t-1 on planes k-t, k-t-1, k-t+1
+                const float4 ya = r == 0 ? above : c[t - 1][r > 0 ? r - 1 : 0];
+                const float4 yb = r == R - 1 ? below : c[t - 1][r < R - 1 ? r + 1 : r];
+                float left = __shfl_up_sync(0xffffffffu, u.w, 1, lw), right = __shfl_down_sync(0xffffffffu, u.x, 1, lw);
+                if (l == 0) left = MODE == 0 && t == 1 ? lc[r] : 0.f;
+                if (l == lw - 1) right = MODE == 0 && t == 1 ? rc[r] : 0.f;
+                float2 va = mul2(cf.cc, lo2f(u)), vb = mul2(cf.cc, hi2f(u));
+                va = fma2(cf.cx, make_float2(left + u.y, u.x + u.z), va);
+                vb = fma2(cf.cx, make_float2(u.y + u.w, u.z + right), vb);
+                va = fma2(cf.cy, add2(lo2f(ya), lo2f(yb)), va);
+                vb = fma2(cf.cy, add2(hi2f(ya), hi2f(yb)), vb);
+                va = fma2(cf.cz, add2(lo2f(um), lo2f(un)), va);
+                vb = fma2(cf.cz, add2(hi2f(um), hi2f(un)), vb);
+                if (MODE >= 1 || t >= 2) {
+                    // MODE 0 keeps B as step 0: its planes k-2 and k-3
+                    const float4 bv = MODE == 0 ? (t == 2 ? m0_old[r] : b3[r]) : t == 1 ? b1[r] : t == 2 ? b2[r] : b3[r];
+                    va = fma2(cf.cb, lo2f(bv), va);
+                    vb = fma2(cf.cb, hi2f(bv), vb);
+                }
+                if ((MODE == 2 && t == 1) || (MODE >= 1 && t == 2) || t == 3) {
+                    const float4 zv = t == 1 ? z1[r] : t == 2 ? m0_old[r] : m1_old[r];
+                    va = fma2(cf.cw, lo2f(zv), va);
+                    vb = fma2(cf.cw, hi2f(zv), vb);
+                }
+                const unsigned mr = on ? mrow[r] : 0u;
+                const float4 v = make_float4(keep(va.x, mx0, mr), keep(va.y, mx1, mr), keep(vb.x, mx2, mr), keep(vb.y, mx3, mr));
+                w[r] = v;
+                if (st) {
+                    float* q = o + off[r];
+                    if (own4[r]) {
+                        if constexpr (A16) {
+                            *reinterpret_cast<float4*>(q) = v;
+                        } else {
+                            *reinterpret_cast<float2*>(q) = make_float2(v.x, v.y);
+                            *reinterpret_cast<float2*>(q + 2) = make_float2(v.z, v.w);
+                        }
+                    }
+                    if (own1[r]) {
+                        if (mx0) q[0] = v.x;
+                        if (mx1) q[1] = v.y;
+                        if (mx2) q[2] = v.z;
+                        if (mx3) q[3] = v.w;
+                    }
+                }
+            }
+            // step t-1 on the plane the next iteration centres on, for the rows around
+            wr[(t - 1) * 2 * PITCH] = up[0];
+            wr[(t - 1) * 2 * PITCH + PITCH] = up[R - 1];
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                m[t - 1][r] = c[t - 1][r];
+                c[t - 1][r] = up[r];
+                up[r] = w[r];
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            if (MODE == 0) b3[r] = m0_old[r];   // B on the next iteration's plane k-3
+            lc[r] = nl[r];
+            rc[r] = nr[r];
+        }
+        float4* sw = rd;
+        rd = wr;
+        wr = sw;
+        __syncthreads();
+    };
+    const std::false_type slow{};
+    const std::true_type quick{};
+    fetch(k0, slow);
+    __syncthreads();
+    int k = k0;
+    const int ka = min(T.kb + NS, k1), kz = min(T.ke + NS - 1, g.hi[2]);
+    for (; k < ka; k++) plane(k, slow);
+#pragma unroll 1
+    for (; k < kz; k++) plane(k, quick);
+    for (; k < k1; k++) plane(k, slow);
+}
+
+// Tiles of a grid along x, y and z.
+struct Cheb3Grid {
+    int lwlog, nf, ntx, rows, nty, kc, nz;
+    bool a16;   // quads from x = 0 on 16-byte boundaries, else from the first unknown on 8-byte ones
+};
+__device__ __forceinline__ void cheb3_tile(const Geo& g, const Cheb3Grid& G, int tx, int ty, int tz, Cheb3Tile& T)
+{
+    // one tile along x: all quads of a row; more: lw - 2 each, the first lane of the
+    // first and the last lane of the last included
+    T.lwlog = G.lwlog;
+    T.lw = 1 << G.lwlog;
+    T.f0 = tx * (T.lw - 2);
+    T.f_own0 = tx == 0 ? 0 : T.f0 + 1;
+    T.f_own1 = tx == G.ntx - 1 ? G.nf : T.f0 + T.lw - 1;
+    T.j0 = g.lo[1] + ty * G.rows;
+    T.j1 = min(T.j0 + G.rows, g.hi[1]);
+    T.kb = g.lo[2] + tz * G.kc;
+    T.ke = min(T.kb + G.kc, g.hi[2]);
+}
+
+template <int MODE, bool A16, bool TWO>
+__global__ void __launch_bounds__(CHEB3_THREADS, 1) k_cheb3(Geo g, Cheb3Grid G, const float* __restrict__ U,
+                                                            const float* __restrict__ B, const float* __restrict__ Z,
+                                                            float* __restrict__ X, float* __restrict__ X2,
+                                                            const __grid_constant__ Cheb3Coef cs, const int* done)
+{
+    pdl_enter();
+    EARLY_EXIT(done);
+    extern __shared__ __align__(16) unsigned char cheb3_smem[];
+    Cheb3Tile T;
+    cheb3_tile(g, G, blockIdx.x % G.ntx, blockIdx.x / G.ntx, blockIdx.y, T);
+    cheb3_march<MODE, A16, TWO>(g, T, U, B, Z, X, X2, cs, reinterpret_cast<float4*>(cheb3_smem));
+}
+
+static Cheb3Grid cheb3_grid(const Geo& g, bool a16)
+{
+    Cheb3Grid G;
+    const int uy = g.hi[1] - g.lo[1], uz = g.hi[2] - g.lo[2];
+    auto along_x = [&](bool a) {
+        G.a16 = a;
+        G.nf = (g.hi[0] - (a ? 0 : g.lo[0]) + 3) / 4;
+        G.lwlog = G.nf <= 8 ? 3 : G.nf <= 16 ? 4 : 5;
+        const int lw = 1 << G.lwlog;
+        G.ntx = G.nf <= lw ? 1 : (G.nf - 2 + lw - 3) / (lw - 2);
+        return G.ntx * lw;
+    };
+    // the 16-byte quads where they take no more lanes (an edge of 128 is 32 quads from
+    // its first unknown and 33 from x = 0)
+    const int wide = along_x(false);
+    if (a16 && along_x(true) > wide) along_x(false);
+    G.rows = (CHEB3_THREADS >> G.lwlog) * CHEB3_R - 6;
+    G.nty = (uy + G.rows - 1) / G.rows;
+    G.rows = (uy + G.nty - 1) / G.nty;
+    // one block per SM at a time: z chunks whose rounds of blocks, each chunk with its 6
+    // extra planes and a start of about 4, come to the fewest planes
+    const long long xy = (long long)G.ntx * G.nty;
+    double best = 1e300;
+    for (int nz = 1; nz <= std::min(uz, 64); nz++) {
+        const int kc = (uz + nz - 1) / nz;
+        const double cost = (double)((xy * ((uz + kc - 1) / kc) + sm_count() - 1) / sm_count()) * (kc + 10);
+        if (cost < best) {
+            best = cost;
+            G.kc = kc;
+            G.nz = (uz + kc - 1) / kc;
+        }
+    }
+    return G;
+}
+
+bool cheb3_ok(const Geo& g, std::initializer_list<const void*> ptrs)
+{
+    // offsets within a plane are 32-bit
+    if (has_neumann(g) || g.sj % 2 != 0 || g.sk >= (1LL << 31)) return false;
+    for (const void* p : ptrs)
+        if (p && ((uintptr_t)p & 7u) != 0) return false;
+    return true;
+}
+
+template <bool A16, bool TWO>
+static const void* cheb3_kernel(int mode)
+{
+    return mode == 0 ? (const void*)k_cheb3<0, A16, TWO> : mode == 1 ? (const void*)k_cheb3<1, A16, TWO> : (const void*)k_cheb3<2, A16, TWO>;
+}
+cudaError_t cheb3_prepare()
+{
+    cudaError_t e = cudaSuccess;
+    for (int mode = 0; mode < 3; mode++)
+        for (const void* k : {cheb3_kernel<false, false>(mode), cheb3_kernel<false, true>(mode), cheb3_kernel<true, false>(mode),
+                              cheb3_kernel<true, true>(mode)})
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, CHEB3_SMEM);
+    return e;
+}
+
+template <bool A16, bool TWO>
+static void cheb3_launch(const Geo& g, const Cheb3Grid& G, int mode, const float* U, const float* B, const float* Z,
+                         float* X, float* X2, const Cheb3Coef& cs, const int* done, cudaStream_t s)
+{
+    const dim3 grid((unsigned)(G.ntx * G.nty), (unsigned)G.nz);
+    if (mode == 0) launch_pdl(k_cheb3<0, A16, TWO>, grid, CHEB3_THREADS, CHEB3_SMEM, s, g, G, U, B, Z, X, X2, cs, done);
+    else if (mode == 1) launch_pdl(k_cheb3<1, A16, TWO>, grid, CHEB3_THREADS, CHEB3_SMEM, s, g, G, U, B, Z, X, X2, cs, done);
+    else launch_pdl(k_cheb3<2, A16, TWO>, grid, CHEB3_THREADS, CHEB3_SMEM, s, g, G, U, B, Z, X, X2, cs, done);
+    PPS_COUNT_LAUNCH();
+}
+
+void fast_cheb3(const Geo& g, int mode, const float* U, const float* B, const float* Z, float* X, float* X2,
+                const Coef* c, const int* done, cudaStream_t s)
+{
+    Cheb3Coef cs;
+    for (int t = 0; t < 3; t++) {
+        const CT<float> f = cast_coef<float>(c[t]);
+        cs.c[t] = {{f.cc, f.cc}, {f.cx, f.cx}, {f.cy, f.cy}, {f.cz, f.cz}, {f.cb, f.cb}, {f.cw, f.cw}};
+    }
+    bool a16 = g.sj % 4 == 0;
+    for (const void* p : {(const void*)U, (const void*)B, (const void*)Z, (const void*)X, (const void*)X2})
+        a16 = a16 && ((uintptr_t)p & 15u) == 0;
+    const Cheb3Grid G = cheb3_grid(g, a16);
+    if (G.a16) X2 ? cheb3_launch<true, true>(g, G, mode, U, B, Z, X, X2, cs, done, s)
+                  : cheb3_launch<true, false>(g, G, mode, U, B, Z, X, X2, cs, done, s);
+    else X2 ? cheb3_launch<false, true>(g, G, mode, U, B, Z, X, X2, cs, done, s)
+            : cheb3_launch<false, false>(g, G, mode, U, B, Z, X, X2, cs, done, s);
+}
+
 // Several Chebyshev steps in one pass (temporal blocking).  The steps s1..s_NS of
 // the recurrence above (s1 from B, then sweeps; the last writes X = -s_NS) run as a
 // wavefront along z over a tile of 32 x 16 columns: when B plane j is loaded, step t

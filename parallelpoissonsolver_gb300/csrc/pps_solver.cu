@@ -82,6 +82,7 @@ template <typename T>
 struct Fields {
     T *p = nullptr, *r = nullptr, *r0 = nullptr, *Mp = nullptr, *AMp = nullptr, *z = nullptr, *Az = nullptr;
     T *Y = nullptr, *Z = nullptr, *W = nullptr, *e = nullptr;
+    T* V = nullptr;   // FP32: the Chebyshev passes' fourth buffer
 };
 
 }  // namespace
@@ -270,6 +271,10 @@ void alloc_fields(Fields<T>& F, long long ntot, bool with_e, bool with_cheb = tr
         CK(cudaMalloc((void**)q, sizeof(T) * (size_t)ntot));
         CK(cudaMemset(*q, 0, sizeof(T) * (size_t)ntot));
     }
+    if (with_cheb && sizeof(T) == 4) {
+        CK(cudaMalloc((void**)&F.V, sizeof(T) * (size_t)ntot));
+        CK(cudaMemset(F.V, 0, sizeof(T) * (size_t)ntot));
+    }
     if (with_e) {
         CK(cudaMalloc((void**)&F.e, sizeof(T) * (size_t)ntot));
         CK(cudaMemset(F.e, 0, sizeof(T) * (size_t)ntot));
@@ -279,7 +284,7 @@ void alloc_fields(Fields<T>& F, long long ntot, bool with_e, bool with_cheb = tr
 template <typename T>
 void free_fields(Fields<T>& F)
 {
-    T* all[] = {F.p, F.r, F.r0, F.Mp, F.AMp, F.z, F.Az, F.Y, F.Z, F.W, F.e};
+    T* all[] = {F.p, F.r, F.r0, F.Mp, F.AMp, F.z, F.Az, F.Y, F.Z, F.W, F.e, F.V};
     for (T* q : all)
         if (q) cudaFree(q);
     F = Fields<T>();
@@ -766,33 +771,60 @@ void fast_cheb(pps_solver* s, Fields<T>& F, T* B, T* X, Launcher& L, const ChebP
     T* Y = F.Y;
     T* Z = F.Z;
     T* W = F.W;
-    fast_cheb_s01<T>(g, shc, B, Y, c01, done, st);
-    L.bytes += bytes_of<T>(N, 2);
-    L.launches++;
-    const bool prof = L.profile && s->sweep_ev_used + 2 <= (int)s->sweep_ev.size();
-    if (prof) CK(cudaEventRecord(s->sweep_ev[s->sweep_ev_used], st));
-    for (int it = 2; it <= n - 2; it++) {
+    // coefficients of step it (2..n-2); the first step's Z = s0 = B/theta is folded into B's
+    auto next_coef = [&](int it) {
         rhoOld = rhoCurr;
         rhoCurr = 1 / (2 * sigma - rhoOld);
-        const bool last = (it == n - 2);
-        Coef c = cheb_sweep_coef(a, p, rhoCurr, rhoOld, last ? -1.0 : 1.0);
-        const bool first = (it == 2);
-        if (first) {
-            // Z = s0 = B/theta: fold it into the B coefficient instead of storing s0
+        Coef c = cheb_sweep_coef(a, p, rhoCurr, rhoOld, it == n - 2 ? -1.0 : 1.0);
+        if (it == 2) {
             c.cb += c.cw / p.theta;
             c.cw = 0.0;
         }
-        fast_cheb_sweep<T>(g, shc, Y, B, first ? nullptr : Z, last ? X : W, c, done, st, !last || mirror);
-        const int words = first ? 3 : 4;
+        return c;
+    };
+    // FP32: three steps a pass (k_cheb3), the steps that do not divide by three first.
+    // Below 64 K unknowns a pass's 6 extra planes and rows cost more than two launches
+    // (BiCGSTAB iteration: 32^3 106 us alone, 115 in passes; 48 x 40 x 64 137, 125).
+    int lead = n - 2;
+    if constexpr (std::is_same<T, float>::value) {
+        if (N >= 65536 && n >= 5 && F.V && cheb3_ok(g, {B, X, Y, Z, W, F.V})) lead = (n - 2) % 3;
+    }
+    if (lead > 0) {
+        fast_cheb_s01<T>(g, shc, B, Y, c01, done, st);
+        L.bytes += bytes_of<T>(N, 2);
+        L.launches++;
+    }
+    const bool prof = L.profile && s->sweep_ev_used + 2 <= (int)s->sweep_ev.size();
+    if (prof) CK(cudaEventRecord(s->sweep_ev[s->sweep_ev_used], st));
+    auto count = [&](int words) {
         L.bytes += bytes_of<T>(N, words);
         L.launches++;
         s->sweep_bytes_acc += bytes_of<T>(N, words);
         s->sweep_launch_acc++;
+    };
+    for (int it = 2; it <= lead; it++) {
+        const bool last = (it == n - 2);
+        const Coef c = next_coef(it);
+        fast_cheb_sweep<T>(g, shc, Y, B, it == 2 ? nullptr : Z, last ? X : W, c, done, st, !last || mirror);
+        count(it == 2 ? 3 : 4);
         if (!last) {
             T* t = Z;   // (Y, Z, W) <- (W, Y, Z)
             Z = Y;
             Y = W;
             W = t;
+        }
+    }
+    if constexpr (std::is_same<T, float>::value) {
+        T* V = F.V;
+        for (int it = lead + 1; it <= n - 2; it += 3) {   // steps it, it+1, it+2
+            Coef c[3];
+            for (int q = 0; q < 3; q++) c[q] = it + q == 1 ? c01 : next_coef(it + q);
+            const bool last = it + 2 == n - 2;
+            const int mode = it == 1 ? 0 : it == 2 ? 1 : 2;
+            fast_cheb3(g, mode, mode == 0 ? B : Y, B, Z, last ? X : W, last ? nullptr : V, c, done, st);
+            count(1 + mode + (last ? 1 : 2));
+            std::swap(Y, W);   // the step just made is the next pass's Y, the one before it its Z
+            std::swap(Z, V);
         }
     }
     if (prof) {
@@ -2012,6 +2044,7 @@ pps_status pps_create(const pps_grid* grid, const pps_config* cfg, pps_solver** 
         CK(cudaMalloc((void**)&s->d_b, fb));
         if (cfg->form == PPS_FORM_MIXED) {
             alloc_fields<float>(s->f32, g.ntot, true);
+            CK(cheb3_prepare());
         } else {
             alloc_fields<double>(s->f64, g.ntot, false);
         }
