@@ -565,8 +565,9 @@ pps_status pps_batch_create(int nprob, const pps_grid* grids, const pps_config* 
         BK(cudaMemsetAsync(s->b, 0, sizeof(double) * (size_t)pool, s->stream));
         float** f32[] = {&s->p, &s->r, &s->r0, &s->Mp, &s->AMp, &s->z, &s->Az, &s->Y, &s->Z, &s->W, &s->e};
         for (float** q : f32) {
-            BK(cudaMalloc((void**)q, sizeof(float) * (size_t)pool));
-            BK(cudaMemsetAsync(*q, 0, sizeof(float) * (size_t)pool, s->stream));
+            // 32 floats of slack: the persistent batch shifts its fields by two
+            BK(cudaMalloc((void**)q, sizeof(float) * (size_t)(pool + 32)));
+            BK(cudaMemsetAsync(*q, 0, sizeof(float) * (size_t)(pool + 32), s->stream));
         }
         BK(cudaMalloc((void**)&s->dprob, sizeof(BProb) * (size_t)nprob));
         BK(cudaMalloc((void**)&s->dprob4, sizeof(BProb) * (size_t)nprob));

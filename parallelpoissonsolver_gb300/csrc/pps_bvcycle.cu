@@ -45,6 +45,7 @@ namespace bvc {
 constexpr int MAXLEV = 6;          // levels 0..5
 constexpr int NT = 256;            // threads per block: 32 x 8 columns of a tile
 constexpr int EX_MAX = 32;         // coarsest level: at most 32 unknowns per axis
+constexpr int KZ0 = 128, KZ1 = 16, WAVES = 8;   // longest z chunks of work items; items per resident block
 constexpr double RATIO = 8.0;      // smoothing interval [lmax/RATIO, lmax]
 
 struct Prob {
@@ -53,7 +54,7 @@ struct Prob {
     long long coff[MAXLEV];        // pooled offset of level l >= 1 (dense n_l^3)
     int n[MAXLEV];                 // unknowns per axis on level l
     int kz[MAXLEV];                // planes per work item on level l
-    int ntx[MAXLEV], nty[MAXLEV], nch[MAXLEV];
+    int lwlog;                     // level 0 in quads of 4 points: log2 of the lanes of a row; 0: one column per thread
     double ih2;                    // 1/h^2 (FP64 residual)
     float fcc[3], fcn[3], fcb[3], fcz[3];   // fine Chebyshev steps: W = cc Y + cn sum(Y nbrs) + cb B + cz Z
     float lih2[MAXLEV], lastm[MAXLEV], lastc[MAXLEV];   // level operators (l >= 1)
@@ -65,12 +66,17 @@ struct State {
     double rho, alpha, beta;
     int mode;                      // 0: refinement step next, 1: FCG iteration
     int done, status, skip, par;
+    int xnz;                       // the initial x holds a non-zero value the residual reads
     int inner_it, total_it, refinements;
 };
 
-struct Barrier {
-    unsigned count, gen;
-    int error, pad;
+// The arrivals' counter and the generation the blocks poll lie on lines of their own.
+struct alignas(128) Barrier {
+    unsigned count;
+    unsigned pad0[31];
+    unsigned gen;
+    int error;
+    unsigned pad1[30];
 };
 
 enum : int { PH_NORM = 0, PH_A, PH_B, PH_C1, PH_C2, PH_C3, PH_R0, PH_RS, PH_D1, PH_D2, PH_DR, PH_EX, PH_UP, PH_UR,
@@ -84,6 +90,7 @@ struct Dev {
     const Prob* prob;
     int nprob;
     const long long* toff;         // toff[l * (nprob + 1) + q]: first work item of problem q on level l
+    const int4* items[MAXLEV];     // level l's work items: problem, first column along x, y, first plane
     const Phase* phases;
     int nphases;
     State* st;
@@ -129,12 +136,11 @@ __device__ bool grid_barrier(const Dev& D)
             atomicAdd(&D.bar->gen, 1u);
         } else {
             const unsigned long long t0 = now_ns();
-            while (*gen == g) {
-                if (*err != 0 || now_ns() - t0 > D.limit_ns) {
+            for (unsigned spin = 1; *gen == g; spin++) {
+                if (spin % 16 == 1 && (*err != 0 || now_ns() - t0 > D.limit_ns)) {
                     atomicExch(&D.bar->error, 1);
                     break;
                 }
-                __nanosleep(64);
             }
         }
         __threadfence();
@@ -148,36 +154,33 @@ __device__ bool grid_barrier(const Dev& D)
 
 struct Item {
     int q;
-    int i, j, k0, k1;              // this thread's column (0-based unknown indices) and planes
+    int i, j, k0, k1;              // this thread's column (0-based unknown indices; a quad's first) and planes
+    int l, lw;                     // quads: this thread's lane of its row, lanes of a row
     bool on;                       // the column lies inside the level
     long long item;                // item index within the phase
 };
 
-__device__ __forceinline__ int find_problem(const long long* row, int nprob, long long item)
-{
-    int lo = 0, hi = nprob - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (row[mid] <= item) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
-
-__device__ __forceinline__ Item decode(const Dev& D, int lev, long long item)
+// quads: level 0 of a problem with lwlog > 0 (a row's quads on 1 << lwlog lanes)
+__device__ __forceinline__ Item decode(const Dev& D, int lev, long long item, bool quads)
 {
     Item it;
-    const long long* row = D.toff + (long long)lev * (D.nprob + 1);
-    it.q = find_problem(row, D.nprob, item);
+    const int4 w = __ldg(D.items[lev] + item);
+    it.q = w.x;
     it.item = item;
     const Prob& P = D.prob[it.q];
-    const long long t = item - row[it.q];
-    const int ntx = P.ntx[lev], nty = P.nty[lev];
-    const int bx = (int)(t % ntx), by = (int)((t / ntx) % nty), ch = (int)(t / ((long long)ntx * nty));
     const int n = P.n[lev];
-    it.i = bx * 32 + (int)(threadIdx.x & 31);
-    it.j = by * 8 + (int)(threadIdx.x >> 5);
-    it.k0 = ch * P.kz[lev];
+    const int lwlog = quads ? P.lwlog : 0;
+    if (lwlog > 0) {
+        it.lw = 1 << lwlog;
+        it.l = (int)threadIdx.x & (it.lw - 1);
+        it.i = w.y + 4 * it.l;
+        it.j = w.z + (int)(threadIdx.x >> lwlog);
+    } else {
+        it.lw = it.l = 0;
+        it.i = w.y + (int)(threadIdx.x & 31);
+        it.j = w.z + (int)(threadIdx.x >> 5);
+    }
+    it.k0 = w.w;
     it.k1 = min(it.k0 + P.kz[lev], n);
     it.on = it.i < n && it.j < n;
     return it;
@@ -327,52 +330,42 @@ __device__ __forceinline__ float nsum(const float* f, long long c, long long sj,
 
 // ---- levels >= 1: dense n^3, the upper wall one fine spacing above the last unknown ----
 
-__device__ __forceinline__ float lvl_apply(const float* u, long long base, int n, int i, int j, int k, float ih2,
-                                           float lm, float lc, float uc)
-{
-    const long long sj = n, sk = (long long)n * n;
-    const long long c = base + i + sj * j + sk * k;
-    float a = 0.f;
-    const int t[3] = {i, j, k};
-    const long long s[3] = {1, sj, sk};
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-        const float um = t[d] > 0 ? u[c - s[d]] : 0.f;
-        if (t[d] < n - 1) a += ih2 * ((um + u[c + s[d]]) - 2.f * uc);
-        else a += lm * um + lc * uc;
-    }
-    return a;
-}
-
-__device__ __forceinline__ float lvl_dinv(int n, int i, int j, int k, float ih2, float lc)
-{
-    float d = 0.f;
-    d += i < n - 1 ? 2.f * ih2 : -lc;
-    d += j < n - 1 ? 2.f * ih2 : -lc;
-    d += k < n - 1 ? 2.f * ih2 : -lc;
-    return 1.f / d;
-}
-
 // ---- phase bodies ----
 
-// ||b_adj||^2: b minus the Dirichlet nodes' contributions (x on the boundary nodes)
-__device__ void ph_norm(const Dev& D, const Item& it, double& acc)
+// ||b_adj||^2: b minus the Dirichlet nodes' contributions (x on the boundary nodes);
+// nz: whether x holds a non-zero value at an unknown or a node next to one
+__device__ void ph_norm(const Dev& D, const Item& it, double& acc, unsigned long long& nz)
 {
     const Prob& P = D.prob[it.q];
     if (!it.on) return;
     const long long sj = P.m + 4, sk = sj * sj;
     const int m = P.m;
-    for (int k = it.k0; k < it.k1; k++) {
-        const long long c = idx0(P, it.i, it.j, k);
-        double bd = 0.0;
-        if (it.i == 0) bd += D.x[c - 1];
-        if (it.i == m - 1) bd += D.x[c + 1];
-        if (it.j == 0) bd += D.x[c - sj];
-        if (it.j == m - 1) bd += D.x[c + sj];
-        if (k == 0) bd += D.x[c - sk];
-        if (k == m - 1) bd += D.x[c + sk];
-        const double v = D.b[c] - bd * P.ih2;
-        acc = fma(v, v, acc);
+    auto bits = [](double v) { return (unsigned long long)__double_as_longlong(v) << 1; };
+    for (int u = 0; u < (it.lw ? 4 : 1); u++) {
+        const int i = it.i + u;
+        const bool rim = i == 0 || i == m - 1 || it.j == 0 || it.j == m - 1;
+        long long c = idx0(P, i, it.j, it.k0);
+        for (int k = it.k0; k < it.k1; k++, c += sk) {
+            double v = D.b[c];
+            nz |= bits(D.x[c]);
+            if (rim || k == 0 || k == m - 1) {
+                double bd = 0.0;
+                auto node = [&](bool at, long long o) {
+                    if (!at) return;
+                    const double xv = D.x[c + o];
+                    nz |= bits(xv);
+                    bd += xv;
+                };
+                node(i == 0, -1);
+                node(i == m - 1, 1);
+                node(it.j == 0, -sj);
+                node(it.j == m - 1, sj);
+                node(k == 0, -sk);
+                node(k == m - 1, sk);
+                v -= bd * P.ih2;
+            }
+            acc = fma(v, v, acc);
+        }
     }
 }
 
@@ -422,10 +415,11 @@ __device__ void ph_a_refine(const Dev& D, const Item& it)
 {
     const Prob& P = D.prob[it.q];
     if (!it.on) return;
+    const bool first = D.st[it.q].refinements == 0;   // no correction yet
     for (int k = it.k0; k < it.k1; k++) {
         const long long c = idx0(P, it.i, it.j, k);
         const float ev = D.e[c];
-        if (ev != 0.f) D.x[c] += (double)ev;
+        if (!first && ev != 0.f) D.x[c] += (double)ev;
         D.e[c] = 0.f;
     }
 }
@@ -446,6 +440,9 @@ __device__ void ph_b_fcg(const Dev& D, const Item& it, Acc<float>& acc)
     }
 }
 
+// The first residual of a solve that starts from x = 0 is b.
+__device__ __forceinline__ bool from_b(const State& S) { return S.refinements == 0 && S.xnz == 0; }
+
 // refinement residual r = b - A x in FP64, stored in FP32; sum of its FP64 squares
 __device__ void ph_b_refine(const Dev& D, const Item& it, double& acc)
 {
@@ -454,6 +451,14 @@ __device__ void ph_b_refine(const Dev& D, const Item& it, double& acc)
     const long long sj = P.m + 4, sk = sj * sj;
     const double* x = D.x;
     long long c = idx0(P, it.i, it.j, it.k0);
+    if (from_b(D.st[it.q])) {
+        for (int k = it.k0; k < it.k1; k++, c += sk) {
+            const double rv = D.b[c];
+            D.r[c] = (float)rv;
+            acc = fma(rv, rv, acc);
+        }
+        return;
+    }
     double xm = x[c - sk], xc = x[c];   // the planes below and above carried along the march
     for (int k = it.k0; k < it.k1; k++, c += sk) {
         const double xp = x[c + sk];
@@ -507,35 +512,71 @@ __device__ void ph_r0(const Dev& D, const Item& it)
 }
 
 // full-weighting restriction onto level lc (its unknown c on the finer level's 2c+1),
-// from t0 (lc = 1) or the finer level's residual ct
+// from t0 (lc = 1) or the finer level's residual ct.  A thread marches its coarse
+// column: the weighted 3 x 3 sum of a fine plane serves the coarse planes on either side,
+// and the third point of a fine row is the next lane's first.
 __device__ void ph_restrict(const Dev& D, const Item& it, int lc)
 {
     const Prob& P = D.prob[it.q];
-    if (!it.on) return;
-    const int nf = P.n[lc - 1];
-    const float w[3] = {0.25f, 0.5f, 0.25f};
-    for (int k = it.k0; k < it.k1; k++) {
+    const int nf = P.n[lc - 1], n = P.n[lc], lane = threadIdx.x & 31;
+    const float* f = lc == 1 ? D.t0 : D.ct;
+    const long long sj = lc == 1 ? P.m + 4 : nf, sk = sj * sj;
+    const long long base = lc == 1 ? idx0(P, 2 * it.i, 2 * it.j, 0) : P.coff[lc - 1] + 2 * it.i + sj * (2 * it.j);
+    const bool x2 = 2 * it.i + 2 < nf, y2 = 2 * it.j + 2 < nf;
+    auto plane = [&](int k) -> float {
         float s = 0.f;
-        for (int a = 0; a < 3; a++) {
-            const int fk = 2 * k + a;
-            if (fk >= nf) continue;
-            for (int bb = 0; bb < 3; bb++) {
-                const int fj = 2 * it.j + bb;
-                if (fj >= nf) continue;
-                float row = 0.f;
-                for (int cc = 0; cc < 3; cc++) {
-                    const int fi = 2 * it.i + cc;
-                    if (fi >= nf) continue;
-                    const float v = lc == 1 ? D.t0[idx0(P, fi, fj, fk)]
-                                            : D.ct[P.coff[lc - 1] + fi + (long long)nf * (fj + (long long)nf * fk)];
-                    row = fmaf(w[cc], v, row);
-                }
-                s = fmaf(w[bb] * w[a], row, s);
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+            const bool in = it.on && k < nf && (b < 2 || y2);
+            float u = 0.f, v = 0.f;
+            const long long c = base + sj * b + sk * k;
+            if (in) {
+                const float2 t = *reinterpret_cast<const float2*>(f + c);   // nf and c are even
+                u = t.x;
+                v = t.y;
             }
+            float w = __shfl_down_sync(0xffffffffu, u, 1);
+            if (lane == 31) w = in && x2 ? f[c + 2] : 0.f;
+            if (!x2) w = 0.f;
+            s = fmaf(b == 1 ? 0.5f : 0.25f, fmaf(0.25f, w, fmaf(0.5f, v, 0.25f * u)), s);
         }
-        const int n = P.n[lc];
-        D.cr[P.coff[lc] + it.i + (long long)n * (it.j + (long long)n * k)] = s;
+        return s;
+    };
+    float below = plane(2 * it.k0);
+    for (int k = it.k0; k < it.k1; k++) {
+        const float mid = plane(2 * k + 1), above = plane(2 * k + 2);
+        if (it.on)
+            D.cr[P.coff[lc] + it.i + (long long)n * (it.j + (long long)n * k)] = fmaf(0.25f, above, fmaf(0.5f, mid, 0.25f * below));
+        below = above;
     }
+}
+
+// The weights of a level's 7-point operator in one column: a neighbour's is zero where
+// it is the wall; the lower neighbour's and the centre's differ at the last unknown of an
+// axis.  [e]: e = 1 on the level's last plane.  dinv: 1 / -diag.
+struct LCol {
+    float xm, xp, ym, yp, zm[2], ndg[2], dinv[2];
+};
+__device__ __forceinline__ float lvl_ndiag(const Prob& P, int l, bool lx, bool ly, bool lz)
+{
+    return (lx ? -P.lastc[l] : 2.f * P.lih2[l]) + (ly ? -P.lastc[l] : 2.f * P.lih2[l]) + (lz ? -P.lastc[l] : 2.f * P.lih2[l]);
+}
+__device__ __forceinline__ LCol lvl_col(const Prob& P, int l, int i, int j)
+{
+    const int n = P.n[l];
+    const bool lx = i == n - 1, ly = j == n - 1;
+    LCol C;
+    C.xm = i > 0 ? (lx ? P.lastm[l] : P.lih2[l]) : 0.f;
+    C.xp = lx ? 0.f : P.lih2[l];
+    C.ym = j > 0 ? (ly ? P.lastm[l] : P.lih2[l]) : 0.f;
+    C.yp = ly ? 0.f : P.lih2[l];
+    C.zm[0] = P.lih2[l];
+    C.zm[1] = P.lastm[l];
+    for (int e = 0; e < 2; e++) {
+        C.ndg[e] = lvl_ndiag(P, l, lx, ly, e);
+        C.dinv[e] = 1.f / C.ndg[e];
+    }
+    return C;
 }
 
 // Jacobi-scaled Chebyshev on level l, on the interval [2/RATIO, 2] of D^-1 A_l:
@@ -548,41 +589,60 @@ __device__ void ph_jcheb(const Dev& D, const Item& it, int l, int step, bool up)
     const Prob& P = D.prob[it.q];
     if (!it.on) return;
     const int n = P.n[l];
-    const long long base = P.coff[l];
-    const float* bsrc = up ? D.ct : D.cr;
-    const float ih2 = P.lih2[l], lm = P.lastm[l], lc = P.lastc[l];
+    const float* b = up ? D.ct : D.cr;
+    const float ih2 = P.lih2[l];
     const long long sj = n, sk = (long long)n * n;
-    for (int k = it.k0; k < it.k1; k++) {
-        const long long c = base + it.i + sj * it.j + sk * k;
-        const float dinv = lvl_dinv(n, it.i, it.j, k, ih2, lc);
-        const float bv = bsrc[c];
-        const float s0 = dinv * bv * D.jt;
-        if (step == 1) {
-            // A s0 needs s0 at the neighbours: D^-1 b / theta there
-            float as0 = 0.f;
-            const int t[3] = {it.i, it.j, k};
-            const long long s[3] = {1, sj, sk};
-            for (int d = 0; d < 3; d++) {
-                int ti[3] = {it.i, it.j, k};
-                float um = 0.f;
-                if (t[d] > 0) {
-                    ti[d] = t[d] - 1;
-                    um = lvl_dinv(n, ti[0], ti[1], ti[2], ih2, lc) * bsrc[c - s[d]] * D.jt;
-                }
-                if (t[d] < n - 1) {
-                    ti[d] = t[d] + 1;
-                    const float upv = lvl_dinv(n, ti[0], ti[1], ti[2], ih2, lc) * bsrc[c + s[d]] * D.jt;
-                    as0 += ih2 * ((um + upv) - 2.f * s0);
-                } else {
-                    as0 += lm * um + lc * s0;
-                }
-            }
-            D.cc1[c] = fmaf(D.ja1, s0, D.jb1 * dinv * (bv + as0));
-        } else {
-            const float s1 = D.cc1[c];
-            const float as1 = lvl_apply(D.cc1, base, n, it.i, it.j, k, ih2, lm, lc, s1);
-            const float X = -(fmaf(D.ja2, s1, D.jb2 * dinv * (bv + as1)) - D.jc2 * s0);
+    const LCol C = lvl_col(P, l, it.i, it.j);
+    long long c = P.coff[l] + it.i + sj * it.j + sk * it.k0;
+    if (step == 1) {
+        // A s0 needs s0 = D^-1 b / theta at the neighbours, whose D differ where they are
+        // the last unknown of an axis: one factor per neighbour and plane kind
+        const bool lx = it.i == n - 1, ly = it.j == n - 1;
+        float fc[2], fxm[2], fxp[2], fym[2], fyp[2];
+        for (int e = 0; e < 2; e++) {
+            fc[e] = C.dinv[e] * D.jt;
+            fxm[e] = it.i > 0 ? D.jt / lvl_ndiag(P, l, false, ly, e) * C.xm : 0.f;
+            fxp[e] = !lx ? D.jt / lvl_ndiag(P, l, it.i + 1 == n - 1, ly, e) * C.xp : 0.f;
+            fym[e] = it.j > 0 ? D.jt / lvl_ndiag(P, l, lx, false, e) * C.ym : 0.f;
+            fyp[e] = !ly ? D.jt / lvl_ndiag(P, l, lx, it.j + 1 == n - 1, e) * C.yp : 0.f;
+        }
+        const long long xm = it.i > 0 ? -1 : 0, xp = lx ? 0 : 1, ym = it.j > 0 ? -sj : 0, yp = ly ? 0 : sj;
+        float bv = b[c];
+        float sm = it.k0 > 0 ? b[c - sk] * fc[0] : 0.f, s0 = bv * fc[it.k0 == n - 1];
+        for (int k = it.k0; k < it.k1; k++, c += sk) {
+            const int e = k == n - 1;
+            const float bn = e ? 0.f : b[c + sk];
+            const float sp = bn * fc[k + 1 == n - 1];   // zero above the last plane
+            float as = -C.ndg[e] * s0;
+            as = fmaf(fxm[e], b[c + xm], as);
+            as = fmaf(fxp[e], b[c + xp], as);
+            as = fmaf(fym[e], b[c + ym], as);
+            as = fmaf(fyp[e], b[c + yp], as);
+            as = fmaf(C.zm[e], sm, as);
+            as = fmaf(ih2, sp, as);
+            D.cc1[c] = fmaf(D.ja1, s0, D.jb1 * C.dinv[e] * (bv + as));
+            sm = s0;
+            s0 = sp;
+            bv = bn;
+        }
+    } else {
+        const float* u = D.cc1;
+        const long long xm = it.i > 0 ? -1 : 0, xp = it.i == n - 1 ? 0 : 1, ym = it.j > 0 ? -sj : 0, yp = it.j == n - 1 ? 0 : sj;
+        float um = it.k0 > 0 ? u[c - sk] : 0.f, uc = u[c];
+        for (int k = it.k0; k < it.k1; k++, c += sk) {
+            const int e = k == n - 1;
+            const float un = e ? 0.f : u[c + sk], bv = b[c];
+            float as = -C.ndg[e] * uc;
+            as = fmaf(C.xm, u[c + xm], as);
+            as = fmaf(C.xp, u[c + xp], as);
+            as = fmaf(C.ym, u[c + ym], as);
+            as = fmaf(C.yp, u[c + yp], as);
+            as = fmaf(C.zm[e], um, as);
+            as = fmaf(ih2, un, as);
+            const float X = -(fmaf(D.ja2, uc, D.jb2 * C.dinv[e] * (bv + as)) - D.jc2 * (C.dinv[e] * bv * D.jt));
             D.cz[c] = up ? D.cz[c] + X : X;
+            um = uc;
+            uc = un;
         }
     }
 }
@@ -593,60 +653,76 @@ __device__ void ph_lres(const Dev& D, const Item& it, int l)
     const Prob& P = D.prob[it.q];
     if (!it.on) return;
     const int n = P.n[l];
-    const long long base = P.coff[l];
-    for (int k = it.k0; k < it.k1; k++) {
-        const long long c = base + it.i + (long long)n * (it.j + (long long)n * k);
-        D.ct[c] = D.cr[c] - lvl_apply(D.cz, base, n, it.i, it.j, k, P.lih2[l], P.lastm[l], P.lastc[l], D.cz[c]);
+    const long long sj = n, sk = (long long)n * n;
+    const LCol C = lvl_col(P, l, it.i, it.j);
+    const float* u = D.cz;
+    const long long xm = it.i > 0 ? -1 : 0, xp = it.i == n - 1 ? 0 : 1, ym = it.j > 0 ? -sj : 0, yp = it.j == n - 1 ? 0 : sj;
+    long long c = P.coff[l] + it.i + sj * it.j + sk * it.k0;
+    float um = it.k0 > 0 ? u[c - sk] : 0.f, uc = u[c];
+    for (int k = it.k0; k < it.k1; k++, c += sk) {
+        const int e = k == n - 1;
+        const float un = e ? 0.f : u[c + sk];
+        float a = -C.ndg[e] * uc;
+        a = fmaf(C.xm, u[c + xm], a);
+        a = fmaf(C.xp, u[c + xp], a);
+        a = fmaf(C.ym, u[c + ym], a);
+        a = fmaf(C.yp, u[c + yp], a);
+        a = fmaf(C.zm[e], um, a);
+        a = fmaf(P.lih2[l], un, a);
+        D.ct[c] = D.cr[c] - a;
+        um = uc;
+        uc = un;
     }
 }
 
-// trilinear prolongation weights of fine unknown f from the coarse line: f = 2c+1
-// takes z_c; f = 2c takes (z_{c-1} + z_c) / 2 (z_{-1} = 0, the wall)
-__device__ __forceinline__ int pro_taps(int f, int nc, int (&c)[2], float (&w)[2])
+// One column's coarse line in (x, y): fine i odd takes coarse i/2, even the mean of i/2 - 1
+// and i/2 (the wall's zero below the first).  The column's value on coarse plane cz.
+struct PCol {
+    long long aa, ab, ba, bb;
+    float waa, wab, wba, wbb;
+};
+__device__ __forceinline__ PCol pro_col(int nc, int i, int j)
 {
-    if (f & 1) {
-        c[0] = f >> 1;
-        w[0] = 1.f;
-        return c[0] < nc ? 1 : 0;
-    }
-    const int hc = f >> 1;
-    int n = 0;
-    if (hc - 1 >= 0) {
-        c[n] = hc - 1;
-        w[n++] = 0.5f;
-    }
-    if (hc < nc) {
-        c[n] = hc;
-        w[n++] = 0.5f;
-    }
-    return n;
+    PCol C;
+    const int xb = i >> 1, xa = (i & 1) || xb == 0 ? xb : xb - 1, yb = j >> 1, ya = (j & 1) || yb == 0 ? yb : yb - 1;
+    const float wxb = i & 1 ? 1.f : 0.5f, wxa = i & 1 || i == 0 ? 0.f : 0.5f;
+    const float wyb = j & 1 ? 1.f : 0.5f, wya = j & 1 || j == 0 ? 0.f : 0.5f;
+    C.aa = xa + (long long)nc * ya;
+    C.ab = xb + (long long)nc * ya;
+    C.ba = xa + (long long)nc * yb;
+    C.bb = xb + (long long)nc * yb;
+    C.waa = wxa * wya;
+    C.wab = wxb * wya;
+    C.wba = wxa * wyb;
+    C.wbb = wxb * wyb;
+    return C;
 }
-
-__device__ __forceinline__ float prolong_at(const float* zc, long long base, int nc, int fi, int fj, int fk)
+__device__ __forceinline__ float pro_plane(const float* zc, const PCol& C)
 {
-    int ci[2], cj[2], ck[2];
-    float wi[2], wj[2], wk[2];
-    const int ni = pro_taps(fi, nc, ci, wi), nj = pro_taps(fj, nc, cj, wj), nk = pro_taps(fk, nc, ck, wk);
-    float s = 0.f;
-    for (int a = 0; a < nk; a++)
-        for (int bb = 0; bb < nj; bb++) {
-            float row = 0.f;
-            for (int cc = 0; cc < ni; cc++)
-                row = fmaf(wi[cc], zc[base + ci[cc] + (long long)nc * (cj[bb] + (long long)nc * ck[a])], row);
-            s = fmaf(wk[a] * wj[bb], row, s);
-        }
-    return s;
+    return fmaf(C.waa, zc[C.aa], fmaf(C.wab, zc[C.ab], fmaf(C.wba, zc[C.ba], C.wbb * zc[C.bb])));
 }
 
-// z_l += P z_{l+1} on level l >= 1
+// z_l += P z_{l+1} on level l >= 1: a coarse plane is interpolated once for the two fine
+// planes it covers
 __device__ void ph_up(const Dev& D, const Item& it, int l)
 {
     const Prob& P = D.prob[it.q];
     if (!it.on) return;
     const int n = P.n[l], nc = P.n[l + 1];
-    for (int k = it.k0; k < it.k1; k++) {
-        const long long c = P.coff[l] + it.i + (long long)n * (it.j + (long long)n * k);
-        D.cz[c] += prolong_at(D.cz, P.coff[l + 1], nc, it.i, it.j, k);
+    const long long sk = (long long)n * n, sc = (long long)nc * nc;
+    const PCol C = pro_col(nc, it.i, it.j);
+    const float* zc = D.cz + P.coff[l + 1];
+    long long c = P.coff[l] + it.i + (long long)n * it.j + sk * it.k0;
+    int h = it.k0 >> 1;
+    float below = !(it.k0 & 1) && h > 0 ? pro_plane(zc + sc * (h - 1), C) : 0.f;
+    float cur = pro_plane(zc + sc * h, C);
+    for (int k = it.k0; k < it.k1; k++, c += sk) {
+        D.cz[c] += k & 1 ? cur : 0.5f * (below + cur);
+        if (k & 1) {
+            below = cur;
+            h++;
+            if (k + 1 < it.k1) cur = pro_plane(zc + sc * h, C);
+        }
     }
 }
 
@@ -656,59 +732,321 @@ __device__ void ph_p0(const Dev& D, const Item& it, Acc<float>& a1, Acc<float>& 
     const Prob& P = D.prob[it.q];
     if (!it.on) return;
     const int nc = P.n[1];
-    for (int k = it.k0; k < it.k1; k++) {
-        const long long c = idx0(P, it.i, it.j, k);
-        const float zv = D.z[c] + prolong_at(D.cz, P.coff[1], nc, it.i, it.j, k);
+    const long long sk = (long long)(P.m + 4) * (P.m + 4), sc = (long long)nc * nc;
+    const PCol C = pro_col(nc, it.i, it.j);
+    const float* zc = D.cz + P.coff[1];
+    long long c = idx0(P, it.i, it.j, it.k0);
+    int h = it.k0 >> 1;
+    float below = !(it.k0 & 1) && h > 0 ? pro_plane(zc + sc * (h - 1), C) : 0.f;
+    float cur = pro_plane(zc + sc * h, C);
+    for (int k = it.k0; k < it.k1; k++, c += sk) {
+        const float zv = D.z[c] + (k & 1 ? cur : 0.5f * (below + cur));
         D.z[c] = zv;
         a1.add(zv, D.r[c]);
         a2.add(zv, D.ap[c]);
+        if (k & 1) {
+            below = cur;
+            h++;
+            if (k + 1 < it.k1) cur = pro_plane(zc + sc * h, C);
+        }
+    }
+}
+
+// ---- level 0 in quads ----
+// Edges that are a multiple of 4: a thread owns four consecutive points of a row, 8, 16 or
+// 32 lanes a row (the FP32 pools are shifted so that the first unknown of a row lies on
+// a 16-byte boundary).  The x neighbours come by shuffle within the row's lanes, the
+// others are quad loads, z carried along the march.  Lanes off the grid take part in
+// the shuffles and touch no memory.  (No pointer here is __restrict__: what one phase
+// writes the next reads in the same launch, which the read-only load path does not see.)  One column per thread spent 14 scalar loads a point
+// on the direction phase alone and was bound by the L1 path.
+
+__device__ __forceinline__ float4 ldq(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ void stq(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ float4 operator+(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+__device__ __forceinline__ float4 fma4(float s, float4 a, float4 b)
+{
+    return make_float4(fmaf(s, a.x, b.x), fmaf(s, a.y, b.y), fmaf(s, a.z, b.z), fmaf(s, a.w, b.w));
+}
+__device__ __forceinline__ float4 scale4(float s, float4 a) { return make_float4(s * a.x, s * a.y, s * a.z, s * a.w); }
+__device__ __forceinline__ void add4(Acc<float>& acc, float4 a, float4 b)
+{
+    acc.add(a.x, b.x);
+    acc.add(a.y, b.y);
+    acc.add(a.z, b.z);
+    acc.add(a.w, b.w);
+}
+// sums of the x neighbours of quad u; beyond the row's lanes: `left` and `right`, read by
+// the end lanes (a guard cell's zero, or the next tile of a row longer than 32 quads)
+__device__ __forceinline__ float4 xsum4(const Item& it, float4 u, float left, float right)
+{
+    const float a = __shfl_up_sync(0xffffffffu, u.w, 1, it.lw), b = __shfl_down_sync(0xffffffffu, u.x, 1, it.lw);
+    if (it.l != 0) left = a;
+    if (it.l != it.lw - 1) right = b;
+    return make_float4(left + u.y, u.x + u.z, u.y + u.w, u.z + right);
+}
+
+// FCG direction p_out = z + beta p_in, Ap = A p_out, sum p_out.Ap
+__device__ void pq_a_fcg(const Dev& D, const Item& it, Acc<float>& acc)
+{
+    const Prob& P = D.prob[it.q];
+    const State& S = D.st[it.q];
+    const long long sj = P.m + 4, sk = sj * sj;
+    const float* z = D.z;
+    const float* pin = S.par ? D.pb : D.pa;
+    float* pout = S.par ? D.pa : D.pb;
+    const float be = (float)S.beta, ih2 = (float)P.ih2;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const bool on = it.on, plain = be == 0.f;
+    const bool el = on && it.l == 0 && it.i > 0, er = on && it.l == it.lw - 1 && it.i + 4 < P.m;
+    auto dir = [&](long long c) { return !on ? zero : plain ? ldq(z + c) : fma4(be, ldq(pin + c), ldq(z + c)); };
+    auto dir1 = [&](long long c) { return plain ? z[c] : fmaf(be, pin[c], z[c]); };
+    long long c = idx0(P, it.i, it.j, it.k0);
+    float4 pm = dir(c - sk), pc = dir(c);
+    for (int k = it.k0; k < it.k1; k++, c += sk) {
+        const float4 pp = dir(c + sk);
+        const float4 ya = dir(c - sj), yb = dir(c + sj);
+        const float4 s = (xsum4(it, pc, el ? dir1(c - 1) : 0.f, er ? dir1(c + 4) : 0.f) + (ya + yb)) + (pm + pp);
+        const float4 a = scale4(ih2, fma4(-6.f, pc, s));
+        if (on) {
+            stq(pout + c, pc);
+            stq(D.ap + c, a);
+            add4(acc, pc, a);
+        }
+        pm = pc;
+        pc = pp;
+    }
+}
+
+__device__ void pq_b_fcg(const Dev& D, const Item& it, Acc<float>& acc)
+{
+    const Prob& P = D.prob[it.q];
+    const State& S = D.st[it.q];
+    if (!it.on) return;
+    const long long sk = (long long)(P.m + 4) * (P.m + 4);
+    const float* p = S.par ? D.pb : D.pa;   // the direction phase A wrote (its parity flipped since)
+    const float* ap = D.ap;
+    float* e = D.e;
+    float* r = D.r;
+    const float al = (float)S.alpha;
+    long long c = idx0(P, it.i, it.j, it.k0);
+#pragma unroll 2
+    for (int k = it.k0; k < it.k1; k++, c += sk) {
+        const float4 ev = fma4(al, ldq(p + c), ldq(e + c)), rn = fma4(-al, ldq(ap + c), ldq(r + c));
+        stq(e + c, ev);
+        stq(r + c, rn);
+        add4(acc, rn, rn);
+    }
+}
+
+__device__ void pq_a_refine(const Dev& D, const Item& it)
+{
+    const Prob& P = D.prob[it.q];
+    if (!it.on) return;
+    const long long sk = (long long)(P.m + 4) * (P.m + 4);
+    long long c = idx0(P, it.i, it.j, it.k0);
+    const bool first = D.st[it.q].refinements == 0;   // no correction yet
+    for (int k = it.k0; k < it.k1; k++, c += sk) {
+        if (!first) {
+            const float4 ev = ldq(D.e + c);
+            double2* x = reinterpret_cast<double2*>(D.x + c);
+            double2 a = x[0], b = x[1];
+            if (ev.x != 0.f) a.x += (double)ev.x;
+            if (ev.y != 0.f) a.y += (double)ev.y;
+            if (ev.z != 0.f) b.x += (double)ev.z;
+            if (ev.w != 0.f) b.y += (double)ev.w;
+            x[0] = a;
+            x[1] = b;
+        }
+        stq(D.e + c, make_float4(0.f, 0.f, 0.f, 0.f));
+    }
+}
+
+// refinement residual in FP64, two columns at a time
+__device__ void pq_b_refine(const Dev& D, const Item& it, double& acc)
+{
+    const Prob& P = D.prob[it.q];
+    if (!it.on) return;
+    const long long sj = P.m + 4, sk = sj * sj;
+    const double* x = D.x;
+    const double* b = D.b;
+    const bool fb = from_b(D.st[it.q]);
+    auto ld2 = [](const double* p) { return *reinterpret_cast<const double2*>(p); };
+    for (int h = 0; h < 2; h++) {
+        long long c = idx0(P, it.i + 2 * h, it.j, it.k0);
+        double2 xm = make_double2(0.0, 0.0), xc = xm;
+        if (!fb) {
+            xm = ld2(x + c - sk);
+            xc = ld2(x + c);
+        }
+        for (int k = it.k0; k < it.k1; k++, c += sk) {
+            double2 rv = ld2(b + c);
+            if (!fb) {
+                const double2 xp = ld2(x + c + sk), ya = ld2(x + c - sj), yb = ld2(x + c + sj);
+                const double s0 = ((x[c - 1] + xc.y) + (ya.x + yb.x)) + (xm.x + xp.x);
+                const double s1 = ((xc.x + x[c + 2]) + (ya.y + yb.y)) + (xm.y + xp.y);
+                rv.x -= (s0 - 6.0 * xc.x) * P.ih2;
+                rv.y -= (s1 - 6.0 * xc.y) * P.ih2;
+                xm = xc;
+                xc = xp;
+            }
+            *reinterpret_cast<float2*>(D.r + c) = make_float2((float)rv.x, (float)rv.y);
+            acc = fma(rv.x, rv.x, acc);
+            acc = fma(rv.y, rv.y, acc);
+        }
+    }
+}
+
+// fine Chebyshev step t (ph_cheb0), or, t = 3, the fine residual t0 = r - A z (ph_r0)
+template <int t>
+__device__ void pq_cheb0(const Dev& D, const Item& it)
+{
+    const Prob& P = D.prob[it.q];
+    const long long sj = P.m + 4, sk = sj * sj;
+    const float* Y = t == 0 ? D.r : t == 1 ? D.y1 : t == 2 ? D.y2 : D.z;
+    const float* B = D.r;
+    const float* Z = D.y1;
+    float* W = t == 0 ? D.y1 : t == 1 ? D.y2 : t == 2 ? D.z : D.t0;
+    const float cc = t < 3 ? P.fcc[t < 3 ? t : 0] : 6.f * (float)P.ih2, cn = t < 3 ? P.fcn[t < 3 ? t : 0] : -(float)P.ih2;
+    const float cb = t < 3 ? P.fcb[t < 3 ? t : 0] : 1.f, cz = t < 3 ? P.fcz[t < 3 ? t : 0] : 0.f;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const bool on = it.on;
+    const bool el = on && it.l == 0 && it.i > 0, er = on && it.l == it.lw - 1 && it.i + 4 < P.m;
+    auto ld = [&](long long c) { return on ? ldq(Y + c) : zero; };
+    long long c = idx0(P, it.i, it.j, it.k0);
+    float4 ym = ld(c - sk), yc = ld(c);
+    for (int k = it.k0; k < it.k1; k++, c += sk) {
+        const float4 yp = ld(c + sk), ya = ld(c - sj), yb = ld(c + sj);
+        const float4 s = (xsum4(it, yc, el ? Y[c - 1] : 0.f, er ? Y[c + 4] : 0.f) + (ya + yb)) + (ym + yp);
+        float4 w = fma4(cn, s, scale4(cc, yc));
+        if (on) {
+            if (t > 0) w = fma4(cb, ldq(B + c), w);
+            if (t == 2) w = fma4(cz, ldq(Z + c), w);
+            stq(W + c, w);
+        }
+        ym = yc;
+        yc = yp;
+    }
+}
+
+// z += P z_1 and the sums z.r, z.Ap.  The quad at i = 4l takes coarse 2l - 1 .. 2l + 1:
+// two from one load, the first from the lane below.
+__device__ void pq_p0(const Dev& D, const Item& it, Acc<float>& a1, Acc<float>& a2)
+{
+    const Prob& P = D.prob[it.q];
+    const int nc = P.n[1];
+    const long long sk = (long long)(P.m + 4) * (P.m + 4), sc = (long long)nc * nc;
+    const bool on = it.on;
+    const int h0 = it.i >> 1, yb = it.j >> 1;
+    const float wb = it.j & 1 ? 1.f : 0.5f;
+    const bool two = !(it.j & 1) && yb > 0;
+    const float* zc = D.cz + P.coff[1] + h0 + (long long)nc * yb;
+    auto line = [&](int h) -> float4 {   // the quad on coarse plane h
+        float2 v = make_float2(0.f, 0.f);
+        float left = 0.f;
+        if (on) {
+            const float* p = zc + sc * h;
+            v = *reinterpret_cast<const float2*>(p);
+            if (it.l == 0 && h0 > 0) left = p[-1];
+            v.x *= wb;
+            v.y *= wb;
+            left *= wb;
+            if (two) {
+                const float2 u = *reinterpret_cast<const float2*>(p - nc);
+                v.x = fmaf(0.5f, u.x, v.x);
+                v.y = fmaf(0.5f, u.y, v.y);
+                if (it.l == 0 && h0 > 0) left = fmaf(0.5f, p[-nc - 1], left);
+            }
+        }
+        const float a = __shfl_up_sync(0xffffffffu, v.y, 1, it.lw);
+        if (it.l != 0) left = a;
+        return make_float4(0.5f * (left + v.x), v.x, 0.5f * (v.x + v.y), v.y);
+    };
+    const float* r = D.r;
+    const float* ap = D.ap;
+    float* z = D.z;
+    long long c = idx0(P, it.i, it.j, it.k0);
+    int h = it.k0 >> 1;
+    float4 below = make_float4(0.f, 0.f, 0.f, 0.f), cur = line(h);
+    if (!(it.k0 & 1) && h > 0) below = line(h - 1);
+    for (int k = it.k0; k < it.k1; k++, c += sk) {
+        if (on) {
+            const float4 zv = ldq(z + c) + (k & 1 ? cur : scale4(0.5f, below + cur));
+            stq(z + c, zv);
+            add4(a1, zv, ldq(r + c));
+            add4(a2, zv, ldq(ap + c));
+        }
+        if (k & 1) {
+            below = cur;
+            h++;
+            if (k + 1 < it.k1) cur = line(h);
+        }
     }
 }
 
 // z_k = A_k^-1 r_k on the coarsest level, the whole level in shared memory (one block):
 // passes along x, y, z with V^-1, the eigenvalue division, passes with V
-// (matrices as unet::level_exact_data lays them out)
-__device__ void ph_exact(const Dev& D, int q, float* sm)
+// (matrices as unet::level_exact_data lays them out).  A thread transforms whole lines,
+// held in registers (NM >= n; a run-time length left them in local memory); rows have
+// an odd pitch, so that lines along x start in different banks, and the matrices' rows a
+// multiple of 4, so that one load brings four weights (one a product was the limit).
+template <int NM>
+__device__ void exact_passes(float* cube, const float* M, int n, int px)
 {
-    const Prob& P = D.prob[q];
-    const int n = P.n[P.k];
-    const long long tot = (long long)n * n * n;
-    float* cube = sm;
-    float* M = sm + tot;
-    const int nm = 6 * n * n + 3 * n;
-    const float* src = D.mats + P.mats;
-    for (int i = threadIdx.x; i < nm; i += NT) M[i] = src[i];
-    const long long base = P.coff[P.k];
-    for (long long i = threadIdx.x; i < tot; i += NT) cube[i] = D.cr[base + i];
-    __syncthreads();
+    const int tot = n * n * n, pn = (n + 3) & ~3;
     for (int pass = 0; pass < 7; pass++) {
         if (pass == 3) {
-            const float* lam = M + 6 * n * n;
-            for (long long i = threadIdx.x; i < tot; i += NT) {
-                const int xi = (int)(i % n), yi = (int)((i / n) % n), zi = (int)(i / ((long long)n * n));
-                cube[i] = cube[i] / (lam[xi] + lam[n + yi] + lam[2 * n + zi]);
+            const float* lam = M + 6 * n * pn;
+            for (int i = threadIdx.x; i < tot; i += NT) {
+                const int xi = i % n, yi = (i / n) % n, zi = i / (n * n);
+                float* v = cube + xi + px * (yi + n * zi);
+                *v = *v / (lam[xi] + lam[n + yi] + lam[2 * n + zi]);
             }
         } else {
             const int axis = pass < 3 ? pass : pass - 4;
-            const float* Mat = M + (pass < 3 ? axis : 3 + axis) * n * n;
-            const long long stride = axis == 0 ? 1 : (axis == 1 ? n : (long long)n * n);
-            float v[EX_MAX];
+            const float* Mat = M + (pass < 3 ? axis : 3 + axis) * n * pn;
+            const int stride = axis == 0 ? 1 : axis == 1 ? px : px * n;
             for (int t = threadIdx.x; t < n * n; t += NT) {
-                long long b0;
-                if (axis == 0) b0 = (long long)t * n;
-                else if (axis == 1) b0 = (t % n) + (long long)(t / n) * n * n;
-                else b0 = t;
-                for (int mm = 0; mm < n; mm++) v[mm] = cube[b0 + mm * stride];
+                const int a = t % n, b = t / n;
+                float* line = cube + (axis == 0 ? px * t : axis == 1 ? a + px * n * b : a + px * b);
+                float v[NM];
+#pragma unroll
+                for (int m = 0; m < NM; m++) v[m] = m < n ? line[m * stride] : 0.f;
                 for (int i = 0; i < n; i++) {
                     float acc = 0.f;
-                    for (int mm = 0; mm < n; mm++) acc = fmaf(Mat[i * n + mm], v[mm], acc);
-                    cube[b0 + i * stride] = acc;
+#pragma unroll
+                    for (int m = 0; m < NM; m += 4)
+                        if (m < n) {   // the padding's weights and values are zero
+                            const float4 w = *reinterpret_cast<const float4*>(Mat + i * pn + m);
+                            acc = fmaf(w.x, v[m], acc);
+                            acc = fmaf(w.y, v[m + 1], acc);
+                            acc = fmaf(w.z, v[m + 2], acc);
+                            acc = fmaf(w.w, v[m + 3], acc);
+                        }
+                    line[i * stride] = acc;
                 }
             }
         }
         __syncthreads();
     }
-    for (long long i = threadIdx.x; i < tot; i += NT) D.cz[base + i] = cube[i];
+}
+__device__ void ph_exact(const Dev& D, int q, float* sm)
+{
+    const Prob& P = D.prob[q];
+    const int n = P.n[P.k], px = n | 1, tot = n * n * n;
+    float* cube = sm;
+    const int pn = (n + 3) & ~3;
+    float* M = sm + ((px * n * n + 3) & ~3);
+    const float* src = D.mats + P.mats;
+    for (int i = threadIdx.x; i < 6 * n * pn; i += NT) M[i] = i % pn < n ? src[i / pn * n + i % pn] : 0.f;
+    for (int i = threadIdx.x; i < 3 * n; i += NT) M[6 * n * pn + i] = src[6 * n * n + i];
+    const long long base = P.coff[P.k];
+    for (int i = threadIdx.x; i < tot; i += NT) cube[i % n + px * (i / n)] = D.cr[base + i];
+    __syncthreads();
+    if (n <= 8) exact_passes<8>(cube, M, n, px);
+    else if (n <= 16) exact_passes<16>(cube, M, n, px);
+    else exact_passes<32>(cube, M, n, px);
+    for (int i = threadIdx.x; i < tot; i += NT) D.cz[base + i] = cube[i % n + px * (i / n)];
     __syncthreads();
 }
 
@@ -754,24 +1092,30 @@ __device__ void run_phase(const Dev& D, const Phase& ph, float* sm)
     const long long* row = D.toff + (long long)lev * (D.nprob + 1);
     const long long total = row[D.nprob];
     for (long long item = blockIdx.x; item < total; item += gridDim.x) {
-        const Item it = decode(D, lev, item);
+        const Item it = decode(D, lev, item, ph.type != PH_RS && lev == 0);
         if (!takes_part(D, ph, it.q)) continue;
+        const bool quads = it.lw > 0;
         const State& S = D.st[it.q];
         const long long first = row[it.q], count = row[it.q + 1] - row[it.q];
         double tot[2];
         switch (ph.type) {
         case PH_NORM: {
             double v[1] = {0.0};
-            ph_norm(D, it, v[0]);
+            unsigned long long nz = 0;
+            ph_norm(D, it, v[0], nz);
+            if (__syncthreads_or(nz != 0) && threadIdx.x == 0) D.st[it.q].xnz = 1;
             if (item_reduce<1>(D, it, first, count, v, tot)) advance(D, it.q, PH_NORM, tot);
             break;
         }
         case PH_A:
             if (S.mode == 1) {
                 Acc<float> a;
-                ph_a_fcg(D, it, a);
+                if (quads) pq_a_fcg(D, it, a);
+                else ph_a_fcg(D, it, a);
                 double v[1] = {a.value()};
                 if (item_reduce<1>(D, it, first, count, v, tot)) advance(D, it.q, PH_A, tot);
+            } else if (quads) {
+                pq_a_refine(D, it);
             } else {
                 ph_a_refine(D, it);
             }
@@ -779,19 +1123,33 @@ __device__ void run_phase(const Dev& D, const Phase& ph, float* sm)
         case PH_B:
             if (S.mode == 1) {
                 Acc<float> a;
-                ph_b_fcg(D, it, a);
+                if (quads) pq_b_fcg(D, it, a);
+                else ph_b_fcg(D, it, a);
                 double v[1] = {a.value()};
                 if (item_reduce<1>(D, it, first, count, v, tot)) advance(D, it.q, PH_B, tot);
             } else {
                 double v[1] = {0.0};
-                ph_b_refine(D, it, v[0]);
+                if (quads) pq_b_refine(D, it, v[0]);
+                else ph_b_refine(D, it, v[0]);
                 if (item_reduce<1>(D, it, first, count, v, tot)) advance(D, it.q, PH_B, tot);
             }
             break;
-        case PH_C1: ph_cheb0(D, it, 0); break;
-        case PH_C2: ph_cheb0(D, it, 1); break;
-        case PH_C3: ph_cheb0(D, it, 2); break;
-        case PH_R0: ph_r0(D, it); break;
+        case PH_C1:
+            if (quads) pq_cheb0<0>(D, it);
+            else ph_cheb0(D, it, 0);
+            break;
+        case PH_C2:
+            if (quads) pq_cheb0<1>(D, it);
+            else ph_cheb0(D, it, 1);
+            break;
+        case PH_C3:
+            if (quads) pq_cheb0<2>(D, it);
+            else ph_cheb0(D, it, 2);
+            break;
+        case PH_R0:
+            if (quads) pq_cheb0<3>(D, it);
+            else ph_r0(D, it);
+            break;
         case PH_RS: ph_restrict(D, it, ph.level + 1); break;
         case PH_D1: ph_jcheb(D, it, ph.level, 1, false); break;
         case PH_D2: ph_jcheb(D, it, ph.level, 2, false); break;
@@ -802,7 +1160,8 @@ __device__ void run_phase(const Dev& D, const Phase& ph, float* sm)
         case PH_U2: ph_jcheb(D, it, ph.level, 2, true); break;
         case PH_P0: {
             Acc<float> a1, a2;
-            ph_p0(D, it, a1, a2);
+            if (quads) pq_p0(D, it, a1, a2);
+            else ph_p0(D, it, a1, a2);
             double v[2] = {a1.value(), a2.value()};
             if (item_reduce<2>(D, it, first, count, v, tot)) advance(D, it.q, PH_P0, tot);
             break;
@@ -816,10 +1175,10 @@ __device__ void run_phase(const Dev& D, const Phase& ph, float* sm)
 // The persistent solve: the norm phase, then rounds of the phase program until every
 // problem has finished (or max_rounds), a grid barrier after every phase.  All blocks
 // read `unfinished` after the same barrier, so they leave the loop together.
-__global__ void __launch_bounds__(NT, 6) k_bvc_solve(Dev D)
+__global__ void __launch_bounds__(NT, 4) k_bvc_solve(const __grid_constant__ Dev D)
 {
     pdl_enter();
-    extern __shared__ float sm_ex[];
+    extern __shared__ __align__(16) float sm_ex[];
     run_phase(D, Phase{PH_NORM, 0}, sm_ex);
     if (!grid_barrier(D)) return;
     for (int round = 0; round < D.max_rounds; round++) {
@@ -863,6 +1222,7 @@ struct Plan {
     long long max_items = 0;
     Prob* dprob = nullptr;
     long long* dtoff = nullptr;
+    int4* ditems = nullptr;
     Phase* dphases = nullptr;
     State* dst = nullptr;
     float *cr = nullptr, *cz = nullptr, *ct = nullptr, *cc1 = nullptr;
@@ -881,7 +1241,7 @@ struct Plan {
 void free_plan(Plan* p)
 {
     if (p->gexec) cudaGraphExecDestroy(p->gexec);
-    void* ptrs[] = {p->dprob, p->dtoff, p->dphases, p->dst, p->cr, p->cz, p->ct, p->cc1, p->dmats, p->partials,
+    void* ptrs[] = {p->dprob, p->dtoff, p->ditems, p->dphases, p->dst, p->cr, p->cz, p->ct, p->cc1, p->dmats, p->partials,
                     p->counters, p->bar, p->unfinished};
     for (void* q : ptrs)
         if (q) cudaFree(q);
@@ -963,18 +1323,11 @@ bool bvc_create(BvcPlan** out, int nprob, const Geo* geo, const long long* off, 
         pr.k = k;
         const double h = g.ds[0];
         pr.ih2 = 1.0 / (h * h);
+        pr.lwlog = m % 4 != 0 ? 0 : m <= 32 ? 3 : m <= 64 ? 4 : 5;
         fine_coefs(pr, h);
         for (int l = 0; l <= k; l++) {
             const int nl = m >> l;
             pr.n[l] = nl;
-            // planes per item: up to 128 on the solver's grid, where an item's fixed costs
-            // (locating its problem, the block sum) are worth amortising over long columns
-            // (256 problems of the batched workload: 119.9 ms with 16, 112.8 ms with 128);
-            // 16 on the coarse levels
-            pr.kz[l] = std::min(nl, l == 0 ? 128 : 16);
-            pr.ntx[l] = (nl + 31) / 32;
-            pr.nty[l] = (nl + 7) / 8;
-            pr.nch[l] = (nl + pr.kz[l] - 1) / pr.kz[l];
             if (l >= 1) {
                 const double H = h * (double)(1 << l);
                 pr.lih2[l] = (float)(1.0 / (H * H));
@@ -1002,7 +1355,7 @@ bool bvc_create(BvcPlan** out, int nprob, const Geo* geo, const long long* off, 
         }
         pr.mats = it->second;
         P->maxk = std::max(P->maxk, k);
-        P->ex_smem = std::max(P->ex_smem, sizeof(float) * ((size_t)n * n * n + 6 * (size_t)n * n + 3 * (size_t)n));
+        P->ex_smem = std::max(P->ex_smem, sizeof(float) * ((size_t)(n | 1) * n * n + 4 + 6 * (size_t)n * ((n + 3) & ~3) + 3 * (size_t)n));
     }
     // item order: largest problems first, so their items are handed out first
     std::vector<int> order((size_t)nprob);
@@ -1015,16 +1368,49 @@ bool bvc_create(BvcPlan** out, int nprob, const Geo* geo, const long long* off, 
         table[(size_t)t] = P->prob[(size_t)order[(size_t)t]];
         P->slot[(size_t)order[(size_t)t]] = t;
     }
+    // Work items of every level: a tile of columns (quads on level 0: 256 >> lwlog rows of
+    // 1 << lwlog quads; else 32 x 8 columns) by a chunk of planes.  The chunks are as long
+    // as KZ0 / KZ1 planes where that leaves 8 items for each of the 4 blocks of every
+    // SM, and shorter down to 4 planes where it does not: a phase of a small batch is
+    // one march long (8 problems of 32 and 64: 9.3 ms with 128 planes, 2.4 with 4; 256
+    // problems: 70.3 ms with 4 items a block, 66.7 with 8, 69.8 with 16).
     P->toff.assign((size_t)MAXLEV * (nprob + 1), 0);
+    std::vector<int4> items;
+    std::vector<size_t> items_at(MAXLEV + 1, 0);
     for (int l = 0; l < MAXLEV; l++) {
-        long long acc = 0;
-        for (int t = 0; t < nprob; t++) {
-            P->toff[(size_t)l * (nprob + 1) + t] = acc;
-            const Prob& pr = table[(size_t)t];
-            if (l <= pr.k) acc += (long long)pr.ntx[l] * pr.nty[l] * pr.nch[l];
+        auto tile = [&](const Prob& pr, int& w, int& hgt) {
+            const bool quads = l == 0 && pr.lwlog > 0;
+            w = quads ? 4 << pr.lwlog : 32;
+            hgt = quads ? NT >> pr.lwlog : 8;
+        };
+        auto count = [&](const Prob& pr, int kz) -> long long {
+            if (l > pr.k) return 0;
+            int w, hgt;
+            tile(pr, w, hgt);
+            const int n = pr.n[l];
+            return (long long)((n + w - 1) / w) * ((n + hgt - 1) / hgt) * ((n + kz - 1) / kz);
+        };
+        int kz = l == 0 ? KZ0 : KZ1;
+        for (; kz > 4; kz /= 2) {
+            long long total = 0;
+            for (const Prob& pr : table) total += count(pr, kz);
+            if (total >= (long long)WAVES * 4 * sm_count()) break;
         }
-        P->toff[(size_t)l * (nprob + 1) + nprob] = acc;
-        P->max_items = std::max(P->max_items, acc);
+        items_at[(size_t)l] = items.size();
+        for (int t = 0; t < nprob; t++) {
+            Prob& pr = table[(size_t)t];
+            P->toff[(size_t)l * (nprob + 1) + t] = (long long)(items.size() - items_at[(size_t)l]);
+            if (l > pr.k) continue;
+            int w, hgt;
+            tile(pr, w, hgt);
+            const int n = pr.n[l];
+            pr.kz[l] = std::min(n, kz);
+            for (int k0 = 0; k0 < n; k0 += pr.kz[l])
+                for (int j0 = 0; j0 < n; j0 += hgt)
+                    for (int i0 = 0; i0 < n; i0 += w) items.push_back(make_int4(t, i0, j0, k0));
+        }
+        P->toff[(size_t)l * (nprob + 1) + nprob] = (long long)(items.size() - items_at[(size_t)l]);
+        P->max_items = std::max(P->max_items, P->toff[(size_t)l * (nprob + 1) + nprob]);
     }
     // the phase program of one round
     auto add = [&](int type, int level) { P->phases.push_back(Phase{type, level}); };
@@ -1053,6 +1439,8 @@ bool bvc_create(BvcPlan** out, int nprob, const Geo* geo, const long long* off, 
     const size_t cbytes = sizeof(float) * (size_t)std::max(cpool, 32LL);
     VK(cudaMalloc((void**)&P->dprob, sizeof(Prob) * (size_t)nprob));
     VK(cudaMalloc((void**)&P->dtoff, sizeof(long long) * P->toff.size()));
+    VK(cudaMalloc((void**)&P->ditems, sizeof(int4) * std::max<size_t>(items.size(), 1)));
+    VK(cudaMemcpyAsync(P->ditems, items.data(), sizeof(int4) * items.size(), cudaMemcpyHostToDevice, s));
     VK(cudaMalloc((void**)&P->dphases, sizeof(Phase) * P->phases.size()));
     VK(cudaMalloc((void**)&P->dst, sizeof(State) * (size_t)nprob));
     for (float** f : {&P->cr, &P->cz, &P->ct, &P->cc1}) {
@@ -1078,20 +1466,22 @@ bool bvc_create(BvcPlan** out, int nprob, const Geo* geo, const long long* off, 
     D.prob = P->dprob;
     D.nprob = nprob;
     D.toff = P->dtoff;
+    for (int l = 0; l < MAXLEV; l++) D.items[l] = P->ditems + items_at[(size_t)l];
     D.phases = P->dphases;
     D.nphases = (int)P->phases.size();
     D.st = P->dst;
     D.x = pools.x;
     D.b = pools.b;
-    D.r = pools.r;
-    D.z = pools.z;
-    D.pa = pools.pa;
-    D.pb = pools.pb;
-    D.ap = pools.ap;
-    D.e = pools.e;
-    D.y1 = pools.y1;
-    D.y2 = pools.y2;
-    D.t0 = pools.t0;
+    // two floats in: the first unknown of a row (index 2) then lies on a 16-byte boundary
+    D.r = pools.r + 2;
+    D.z = pools.z + 2;
+    D.pa = pools.pa + 2;
+    D.pb = pools.pb + 2;
+    D.ap = pools.ap + 2;
+    D.e = pools.e + 2;
+    D.y1 = pools.y1 + 2;
+    D.y2 = pools.y2 + 2;
+    D.t0 = pools.t0 + 2;
     D.cr = P->cr;
     D.cz = P->cz;
     D.ct = P->ct;
@@ -1179,7 +1569,8 @@ pps_status bvc_solve(BvcPlan* plan, cudaStream_t s, cudaEvent_t ev0, cudaEvent_t
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ev0, ev1);
     std::vector<State> table((size_t)P->nprob);
-    Barrier bar{};
+    Barrier bar;
+    std::memset(&bar, 0, sizeof(bar));
     if (!ck(cudaMemcpyAsync(table.data(), P->dst, sizeof(State) * table.size(), cudaMemcpyDeviceToHost, s),
             "cudaMemcpyAsync") ||
         !ck(cudaMemcpyAsync(&bar, P->bar, sizeof(Barrier), cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync") ||

@@ -95,3 +95,33 @@ def test_persistent_vcycle_batch_rejects_what_it_does_not_run(gpu):
         pps.Batch([pps.BlockGrid(npglobal=(34, 34, 66), ds=(1 / 33, 1 / 33, 1 / 65))], method="vcycle")
     with pytest.raises(pps.PpsError):
         pps.Batch([pps.BlockGrid.cube(32)]).set_wait_limit(1.0)       # the per-phase batch has no barrier
+
+
+@pytest.mark.parametrize("start", ["zero", "nonzero"])
+@pytest.mark.parametrize("edges", [[18, 62],            # not a multiple of 4: one column per thread
+                                   [20, 32, 36],        # 8 and 16 lanes a row, ragged
+                                   [64, 68, 100],       # 16 lanes full, 32 lanes ragged
+                                   [136]])              # two tiles along x
+def test_persistent_vcycle_batch_at_tile_edges(gpu, oracle, edges, start):
+    """Edges where the level-0 tiles end raggedly, and a start whose unknowns and boundary
+    nodes are not zero (the first residual then reads x), against the oracle."""
+    grids = [pps.BlockGrid.cube(m) for m in edges]
+    rng = np.random.default_rng(sum(edges))
+    fields = []
+    for m in edges:
+        b = np.zeros((m + 4,) * 3)
+        b[2:-2, 2:-2, 2:-2] = rng.standard_normal((m,) * 3)
+        x = np.zeros_like(b)
+        if start == "nonzero":
+            x[1:-1, 1:-1, 1:-1] = rng.standard_normal((m + 2,) * 3)   # unknowns and boundary nodes
+        fields.append((x, b))
+    bt = loaded(grids, fields)
+    assert bt.solve() == pps.OK, pps.last_error()
+    for p, m in enumerate(edges):
+        x, ps = bt.get(p)
+        assert ps["err_true"] <= 1e-10
+        want = fields[p][0].copy()
+        oracle.solve(oracle.cube(m), oracle.Config(tol=1e-13, maxit=20000, threads=8), want, fields[p][1].copy())
+        sl = grids[p].unknowns()
+        assert rel_l2(x[sl], want[sl]) < 1e-7
+    bt.close()
