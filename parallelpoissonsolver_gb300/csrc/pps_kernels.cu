@@ -574,9 +574,11 @@ __global__ void __launch_bounds__(256) k_canon_finalize(RedCtx rc, const int* do
 #pragma unroll
         for (int q = 0; q < NS; q++) acc[q] += rc.cells[q * n + c];
     }
+    // a warp without cells sums zeros: skipped (a shuffle tree of FP64 additions holds the
+    // SM's FP64 pipe for 80 clocks a sum)
 #pragma unroll
     for (int q = 0; q < NS; q++) {
-        const double w = warp_sum(acc[q]);
+        const double w = c0 + warp * 32 < c1 ? warp_sum(acc[q]) : 0.0;
         if (lane == 0) sm[warp][q] = w;
     }
     __syncthreads();
@@ -598,7 +600,7 @@ __global__ void __launch_bounds__(256) k_canon_finalize(RedCtx rc, const int* do
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < NS; q++) {
-        const double w = warp_sum(acc[q]);
+        const double w = warp * 32 < CANON_BLOCKS ? warp_sum(acc[q]) : 0.0;
         if (lane == 0) sm[warp][q] = w;
     }
     __syncthreads();
@@ -616,6 +618,64 @@ __global__ void __launch_bounds__(256) k_canon_finalize(RedCtx rc, const int* do
     }
 }
 
+// The same tree in one block, for launches of few cells: the whole reduction then needs
+// no second phase, no fence and no counter.  The cells are read coalesced, each thread's
+// at once, into shared memory (rows of `per` on an odd stride, so that threads on
+// neighbouring rows meet no bank conflict); thread (q, b) adds block b's cells of sum q in
+// the order of warp_sum (offsets 16, 8, 4, 2, 1; an absent cell is the zero it is there),
+// and the block sums go through the shuffle trees of four warps a sum.  A warp that held
+// no cells added zeros: left out.
+static constexpr int CANON_ONE_THREADS = 1024, CANON_ONE_LOADS = 6;
+template <int NS>
+__global__ void __launch_bounds__(CANON_ONE_THREADS) k_canon_one(RedCtx rc, int n, int per, const int* done)
+{
+    pdl_enter();
+    const int stop = done != nullptr ? *(volatile const int*)done : 0;
+    extern __shared__ double cell[];
+    __shared__ double sm[NS][4];
+    const int tid = threadIdx.x, row = per | 1;
+    double in[CANON_ONE_LOADS];
+#pragma unroll
+    for (int u = 0; u < CANON_ONE_LOADS; u++) {
+        const int t = tid + u * CANON_ONE_THREADS;
+        in[u] = t < NS * n ? rc.cells[t] : 0.0;
+    }
+    if (stop) return;
+#pragma unroll
+    for (int u = 0; u < CANON_ONE_LOADS; u++) {
+        const int t = tid + u * CANON_ONE_THREADS, q = NS > 1 && t >= n, c = t - q * n;
+        if (t < NS * n) cell[(q * CANON_BLOCKS + c / per) * row + c % per] = in[u];
+    }
+    __syncthreads();
+    const int q = tid / CANON_BLOCKS, b = tid % CANON_BLOCKS;
+    if (q < NS) {
+        const double* v = cell + (size_t)tid * row;
+        const int m = max(0, min(per, n - b * per));
+        double a[16];
+#pragma unroll
+        for (int l = 0; l < 16; l++) {
+            a[l] = l < m ? v[l] : 0.0;
+            if (l + 16 < m) a[l] += v[l + 16];
+        }
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) {
+            if (o < per) {   // uniform; else the upper half is zeros
+#pragma unroll
+                for (int l = 0; l < o; l++) a[l] += a[l + o];
+            }
+        }
+        const double w = warp_sum(a[0]);
+        if ((tid & 31) == 0) sm[q][(tid >> 5) & 3] = w;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        double tot[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+        for (int s = 0; s < NS; s++) tot[s] = ((sm[s][0] + sm[s][1]) + sm[s][2]) + sm[s][3];
+        finalize(rc, tot);
+    }
+}
+
 // Equal weights on the three axes (equal spacings): the FP64 kernels then sum the six
 // neighbours on the integer pipe.
 static inline bool iso_coef(const Coef& c) { return c.cx == c.cy && c.cx == c.cz; }
@@ -623,7 +683,16 @@ static inline bool iso_coef(const Coef& c) { return c.cx == c.cy && c.cx == c.cz
 template <int NS>
 static void canon_finalize(const RedCtx& rc, const int* done, cudaStream_t s)
 {
-    launch_pdl(k_canon_finalize<NS>, CANON_BLOCKS, 256, 0, s, rc, done);
+    const long long per = (rc.cell_n + CANON_BLOCKS - 1) / CANON_BLOCKS;
+    // One block up to what its static limits hold (32 cells a block sum, 44 KB of cells, six
+    // loads a thread).  A BiCGSTAB solve at 24 x 21 x 30 takes 3.42 ms with the grid-wide
+    // sums and 3.15 ms with one block, 64^3 (16 cells a block sum) 7.93 and 7.80,
+    // 70 x 65 x 50 (20 cells) 8.27 and 8.28: the limits lie where it stops paying.
+    const size_t smem = sizeof(double) * NS * CANON_BLOCKS * (size_t)(per | 1);
+    if (per <= 32 && smem <= 44 * 1024 && NS * rc.cell_n <= CANON_ONE_THREADS * CANON_ONE_LOADS)
+        launch_pdl(k_canon_one<NS>, 1, CANON_ONE_THREADS, smem, s, rc, (int)rc.cell_n, (int)per, done);
+    else
+        launch_pdl(k_canon_finalize<NS>, CANON_BLOCKS, 256, 0, s, rc, done);
     PPS_COUNT_LAUNCH();
 }
 

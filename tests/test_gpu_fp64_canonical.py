@@ -95,3 +95,36 @@ def test_fp64_neumann_ragged_is_tile_independent(gpu, oracle):
     for x, it, h in outs[1:]:
         assert it == outs[0][1] and same_bits(h, outs[0][2]) and same_bits(x, outs[0][0])
     assert abs(outs[0][1] - int(gold["iterations"])) <= 1
+
+
+#        unknowns (x, y, z): 1 cell; 1, 2 and 13 cells a block; the last sizes that two
+#        sums and one sum take in one block, and the first ones beyond
+CELLS = [(3, 1, 1), (5, 8, 64), (33, 3, 64), (40, 52, 62), (5, 168, 64), (5, 169, 64), (5, 256, 64), (5, 257, 64)]
+
+
+@pytest.mark.parametrize("krylov", ["bicgstab", "cg"])
+@pytest.mark.parametrize("n", CELLS)
+def test_fp64_sums_count_every_cell_once(gpu, oracle, n, krylov):
+    """Small whole numbers sum without rounding, so ||b|| is exact in any order; the sums
+    of two steps (two at a time) follow the oracle's up to rounding, which two
+    well-conditioned steps carry from 1e-15 to far less than 1e-9."""
+    npg, ds = tuple(v + 2 for v in n), (0.03, 0.03, 0.03)
+    g = pps.BlockGrid(npglobal=npg, ds=ds)
+    rng = np.random.default_rng(5)
+    b = g.new_field()
+    sl = g.unknowns()
+    b[sl] = rng.integers(-8, 9, b[sl].shape)
+    want = np.sqrt(np.sum(b[sl] ** 2))
+    x = g.new_field()
+    cls = pps.BiCGSTAB if krylov == "bicgstab" else pps.BaseCG
+    s = cls(g, pps.ChebyshevIteration(11), tolerance=1e-14, max_iteration=2, form="fp64")
+    bo = b.copy()
+    s(x, b)
+    h, nb = s.history(), s.stats()["norm_b"]
+    s.close()
+    assert nb == want
+    cfg = oracle.Config(krylov=0 if krylov == "bicgstab" else 1, tol=1e-14, maxit=2)
+    ho = oracle.solve(oracle.Grid(npg, ds, (0.0, 0.0, 0.0), (0,) * 6), cfg, np.zeros_like(bo), bo).history
+    k = min(len(h), len(ho))
+    assert k >= 2
+    np.testing.assert_allclose(h[:k], ho[:k], rtol=1e-9, atol=1e-14)
