@@ -781,6 +781,13 @@ __device__ __forceinline__ void store_mirrored(const Geo& g, T* W, long long c, 
     }
 }
 
+// The stop flag of an iteration's kernel, read where the kernel begins and tested after the
+// first loads are under way: tested at once it puts one memory latency before them.  A
+// mixed solve on 40 x 33 x 60 with Neumann faces takes 8.04 ms with the test first and
+// 7.67 with this.  (The x-vectorised kernels and the BiCGSTAB updates gained nothing from it
+// or lost 2% to the registers of the longer-lived loads: they test first.)
+__device__ __forceinline__ int stop_of(const int* done) { return done != nullptr ? *(volatile const int*)done : 0; }
+
 // s1 of the preconditioner (chebyshevIteration.hpp:79-90) in pre-folded form:
 //   Y = cc*B + cx*(Bx pair) + cy*(By pair) + cz*(Bz pair)
 // s0 = B/theta is never stored: the first sweep folds it into its B coefficient.
@@ -791,7 +798,7 @@ __global__ void __launch_bounds__(256) k_cheb_s01(Geo g, Shape sh, const T* __re
                                                   CT<T> cf, const int* done)
 {
     pdl_enter();
-    EARLY_EXIT(done);
+    const int stop = stop_of(done);
     const Col q = column_cx(g, sh, CX);
     if (!q.active) return;
     const long long sj = g.sj, sk = g.sk;
@@ -814,6 +821,7 @@ __global__ void __launch_bounds__(256) k_cheb_s01(Geo g, Shape sh, const T* __re
             const T bp = B[c + sk];
             const T sx = B[c - 1] + B[c + 1];
             const T sy = B[c - sj] + B[c + sj];
+            if (stop) return;
             T y = cf.cc * bc[u];
             y = fmx(cf.cx, sx, y);
             y = fmx(cf.cy, sy, y);
@@ -835,7 +843,7 @@ __global__ void __launch_bounds__(256) k_cheb_sweep(Geo g, Shape sh, const T* __
                                                     T* __restrict__ W, CT<T> cf, const int* done)
 {
     pdl_enter();
-    EARLY_EXIT(done);
+    const int stop = stop_of(done);
     const Col q = column_cx(g, sh, CX);
     if (!q.active) return;
     const long long sj = g.sj, sk = g.sk;
@@ -858,12 +866,14 @@ __global__ void __launch_bounds__(256) k_cheb_sweep(Geo g, Shape sh, const T* __
             const T yp = Y[c + sk];
             const T sx = Y[c - 1] + Y[c + 1];
             const T sy = Y[c - sj] + Y[c + sj];
+            const T bv = B[c], zv = HAS_Z ? Z[c] : T(0);
+            if (stop) return;
             T w = cf.cc * yc[u];
             w = fmx(cf.cx, sx, w);
             w = fmx(cf.cy, sy, w);
             w = fmx(cf.cz, ym[u] + yp, w);
-            w = fmx(cf.cb, B[c], w);
-            if (HAS_Z) w = fmx(cf.cw, Z[c], w);
+            w = fmx(cf.cb, bv, w);
+            if (HAS_Z) w = fmx(cf.cw, zv, w);
             store_mirrored<NEU>(g, W, c, w, q.i + 32 * u, q.j, k);
             ym[u] = yc[u];
             yc[u] = yp;
@@ -2168,7 +2178,7 @@ __global__ void __launch_bounds__(256) k_fcg_update_xr_flat(long long n, T* __re
                                                             T* __restrict__ r, const T* __restrict__ Ap, RedCtx rc)
 {
     pdl_enter();
-    EARLY_EXIT(&rc.st->done);
+    const int stop = stop_of(&rc.st->done);
     typedef Vec16<T> VT;
     typedef typename VT::type V;
     const T a = (T)rc.st->alpha;
@@ -2178,6 +2188,7 @@ __global__ void __launch_bounds__(256) k_fcg_update_xr_flat(long long n, T* __re
     for (long long i = t0; i < nv; i += stride) {
         V xv = reinterpret_cast<const V*>(x)[i], rv = reinterpret_cast<const V*>(r)[i];
         V pv = reinterpret_cast<const V*>(p)[i], av = reinterpret_cast<const V*>(Ap)[i];
+        if (stop) return;
 #pragma unroll
         for (int e = 0; e < VT::n; e++) {
             VT::at(xv, e) = fmx(a, VT::at(pv, e), VT::at(xv, e));
@@ -2187,6 +2198,7 @@ __global__ void __launch_bounds__(256) k_fcg_update_xr_flat(long long n, T* __re
         reinterpret_cast<V*>(x)[i] = xv;
         reinterpret_cast<V*>(r)[i] = rv;
     }
+    if (stop) return;
     for (long long i = nv * VT::n + t0; i < n; i += stride) {
         x[i] = fmx(a, p[i], x[i]);
         const T rn = fmx(-a, Ap[i], r[i]);
@@ -2227,7 +2239,7 @@ __global__ void __launch_bounds__(256) k_fcg_dot_flat(long long n, const T* __re
                                                       const T* __restrict__ Ap, RedCtx rc)
 {
     pdl_enter();
-    EARLY_EXIT(&rc.st->done);
+    const int stop = stop_of(&rc.st->done);
     typedef Vec16<T> VT;
     typedef typename VT::type V;
     Acc<T> a1, a2, a3;
@@ -2237,6 +2249,7 @@ __global__ void __launch_bounds__(256) k_fcg_dot_flat(long long n, const T* __re
         V rv = reinterpret_cast<const V*>(r)[i], zv = reinterpret_cast<const V*>(z)[i];
         V av;
         if (Ap) av = reinterpret_cast<const V*>(Ap)[i];
+        if (stop) return;
 #pragma unroll
         for (int e = 0; e < VT::n; e++) {
             a1.add(VT::at(zv, e), VT::at(rv, e));
@@ -2244,6 +2257,7 @@ __global__ void __launch_bounds__(256) k_fcg_dot_flat(long long n, const T* __re
             a3.add(VT::at(rv, e), VT::at(rv, e));
         }
     }
+    if (stop) return;
     for (long long i = nv * VT::n + t0; i < n; i += stride) {
         a1.add(z[i], r[i]);
         if (Ap) a2.add(z[i], Ap[i]);
@@ -2510,7 +2524,7 @@ __global__ void __launch_bounds__(256) k_cheb_iso64(Geo g, Shape sh, const doubl
     pdl_enter();
     const Col q = column(g, sh);
     if (!q.active) return;
-    const int stop = done ? *(volatile const int*)done : 0;
+    const int stop = stop_of(done);
     const long long sj = g.sj, sk = g.sk;
     long long c = q.c;
     double um = U[c - sk], uc = U[c], up = U[c + sk];
