@@ -43,28 +43,17 @@ template <int NS>
 __device__ __forceinline__ void breduce_finalize(double (&v)[NS], const BatchDev& B, const BCol& q,
                                                  double* partials, unsigned* counters, BState* bst, int kind)
 {
-    __shared__ double sm[32][NS];
+    __shared__ double st[NS][256], sm[NS];
     __shared__ int is_last;
     const int tid = threadIdx.x + blockDim.x * threadIdx.y;
     const int nthr = blockDim.x * blockDim.y;
-    const int lane = tid & 31, warp = tid >> 5, nwarp = (nthr + 31) >> 5;
-#pragma unroll
-    for (int s = 0; s < NS; s++) {
-        const double w = warp_sum(v[s]);
-        if (lane == 0) sm[warp][s] = w;
-    }
-    __syncthreads();
-    if (tid == 0) {
-#pragma unroll
-        for (int s = 0; s < NS; s++) {
-            double t = 0.0;
-            for (int w = 0; w < nwarp; w++) t += sm[w][s];
-            partials[(size_t)blockIdx.x * 4 + s] = t;
-        }
+    const int nwarp = nthr >> 5;
+    block_sums<NS>(v, st, tid, nwarp, [&](int s, double t) {
+        partials[(size_t)blockIdx.x * 4 + s] = t;
         __threadfence();
-        const unsigned ticket = atomicAdd(&counters[q.p], 1u);
-        is_last = (ticket == q.P->nblocks - 1);
-    }
+    });
+    __syncthreads();
+    if (tid == 0) is_last = atomicAdd(&counters[q.p], 1u) == q.P->nblocks - 1;
     __syncthreads();
     if (!is_last) return;
     __threadfence();
@@ -76,21 +65,12 @@ __device__ __forceinline__ void breduce_finalize(double (&v)[NS], const BatchDev
 #pragma unroll
         for (int s = 0; s < NS; s++) acc[s] += __ldcg(&partials[(size_t)(b0 + b) * 4 + s]);
     }
-    __syncthreads();
-#pragma unroll
-    for (int s = 0; s < NS; s++) {
-        const double w = warp_sum(acc[s]);
-        if (lane == 0) sm[warp][s] = w;
-    }
+    block_sums<NS>(acc, st, tid, nwarp, [&](int s, double t) { sm[s] = t; });
     __syncthreads();
     if (tid == 0) {
         double tot[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-        for (int s = 0; s < NS; s++) {
-            double t = 0.0;
-            for (int w = 0; w < nwarp; w++) t += sm[w][s];
-            tot[s] = t;
-        }
+        for (int s = 0; s < NS; s++) tot[s] = sm[s];
         BState* b = &bst[q.p];
         RedCtx rc;
         rc.partials = partials;

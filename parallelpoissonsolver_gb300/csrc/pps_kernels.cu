@@ -1664,7 +1664,7 @@ __global__ void __launch_bounds__(256) k_axpy_alpha(Geo g, Shape sh, T* __restri
 }
 
 // x += alpha*Mp + omega*z; r -= omega*Az; sums r0*r, r*r   (BiCGSTAB.hpp:227-257)
-template <typename T>
+template <typename T, bool CELLS>
 __global__ void __launch_bounds__(256) k_update_xr(Geo g, Shape sh, T* __restrict__ x, const T* __restrict__ Mp,
                                                    const T* __restrict__ z, T* __restrict__ r,
                                                    const T* __restrict__ Az, const T* __restrict__ r0, RedCtx rc)
@@ -1676,7 +1676,9 @@ __global__ void __launch_bounds__(256) k_update_xr(Geo g, Shape sh, T* __restric
     if (q.active) {
         const T a = (T)rc.st->alpha, w = (T)rc.st->omega;
         long long c = q.c;
-#pragma unroll 4
+        // not unrolled: 32 registers and eight blocks an SM; unrolled by 4, 80 registers (a 128 x 128
+        // x 256 solve with Neumann faces 116 ms against 109)
+#pragma unroll 1
         for (int k = q.k0; k < q.k1; k++) {
             x[c] = fmx(w, z[c], fmx(a, Mp[c], x[c]));
             const T rn = fmx(-w, Az[c], r[c]);
@@ -1687,7 +1689,8 @@ __global__ void __launch_bounds__(256) k_update_xr(Geo g, Shape sh, T* __restric
         }
     }
     double v[2] = {a1.value(), a2.value()};
-    reduce_emit<2>(v, rc, sh);
+    if (CELLS) store_cells<2>(v, rc, sh);
+    else reduce_finalize<2>(v, rc);
 }
 
 // p = r + beta*(p - omega*AMp)   (BiCGSTAB.hpp:261-272)
@@ -2354,81 +2357,106 @@ __global__ void __launch_bounds__(256) k_axpy_alpha_flat(long long n, T* __restr
     for (long long i = nv * VT::n + t0; i < n; i += stride) r[i] = fmx(-a, v[i], r[i]);
 }
 
-// The BiCGSTAB stencils on the x-vectorised FP32 tiles: Au = A u and, NS = 1, sum
-// w.Au (k_stencil_dot, w = r0) or, NS = 2, sums w.Au and Au.Au (k_stencil_dot2,
-// w = r); per point the arithmetic of the one-column kernels, the sums in another
-// order.
+// Resident blocks an SM of k_stencil_dots_v4 (40 registers a thread).
+static constexpr int DOTS_RESIDENT = 6;
+
+// Two of Acc<float>'s double-float sums at once, on the packed operations.
+struct Acc2 {
+    float2 hi = make_float2(0.f, 0.f), lo = make_float2(0.f, 0.f);
+    __device__ __forceinline__ static float2 sub2(float2 a, float2 b) { return fma2(b, make_float2(-1.f, -1.f), a); }
+    __device__ __forceinline__ void add(float2 a, float2 b)
+    {
+        const float2 p = mul2(a, b);
+        const float2 e = fma2(a, b, make_float2(-p.x, -p.y));
+        const float2 s = add2(hi, p);
+        const float2 bb = sub2(s, hi);
+        const float2 t = add2(sub2(hi, sub2(s, bb)), sub2(p, bb));
+        hi = s;
+        lo = add2(lo, add2(t, e));
+    }
+    __device__ __forceinline__ double value() const
+    {
+        return (widen(hi.x) + widen(lo.x)) + (widen(hi.y) + widen(lo.y));
+    }
+};
+
+// The BiCGSTAB stencils on float4s along x: Au = A u and, NS = 1, sum w.Au
+// (k_stencil_dot, w = r0) or, NS = 2, sums w.Au and Au.Au (k_stencil_dot2, w = r); per
+// point the arithmetic of the one-column kernels, the sums in another order.  The
+// threads take the float4s of all rows in turn (dots_grid), so no lane falls beyond a
+// row's end: with tiles of 128 columns, rows of 256 unknowns from x = 1 took three tiles,
+// the third for one column.  The sums of two neighbouring points run as packed pairs.
+// What bounds it is instruction issue, then the FP64 of the block sums: in tiles of 128
+// columns with a shuffle tree per warp and sum, 4128 blocks kept the FP64 pipe busy for 61%
+// of 93 us (NS = 2, 256^3 unknowns; 73 us for NS = 1).  The mixed solve of that size took
+// 118.6 ms, 114.2 with block_sums, 109.1 with these tiles and packed sums.
 template <int NS>
-__global__ void __launch_bounds__(256) k_stencil_dots_v4(Geo g, Shape sh, const float* __restrict__ u,
-                                                         const float* __restrict__ wv, float* __restrict__ Au,
-                                                         Coef cf, RedCtx rc)
+__global__ void __launch_bounds__(256, DOTS_RESIDENT) k_stencil_dots_v4(Geo g, int kchunk, const float* __restrict__ u,
+                                                                        const float* __restrict__ wv,
+                                                                        float* __restrict__ Au, Coef cf, RedCtx rc)
 {
     pdl_enter();
     EARLY_EXIT(&rc.st->done);
-    const Col4 q = column4(g, sh);
-    Acc<float> a1, a2;
-    if (q.j < g.hi[1]) {   // a warp shares its row: the shuffles below see all 32 lanes
-        const bool act = q.act;
-        const int lane = threadIdx.x;
-        const bool m0 = q.i0 >= g.lo[0] && q.i0 < g.hi[0], m1 = q.i0 + 1 >= g.lo[0] && q.i0 + 1 < g.hi[0];
-        const bool m2 = q.i0 + 2 >= g.lo[0] && q.i0 + 2 < g.hi[0], m3 = q.i0 + 3 >= g.lo[0] && q.i0 + 3 < g.hi[0];
-        const bool all4 = m0 && m1 && m2 && m3;
-        const float cc = (float)cf.cc, cx = (float)cf.cx, cy = (float)cf.cy, cz = (float)cf.cz;
-        const long long sj = g.sj, sk = g.sk;
-        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-        long long c = q.c;
-        float4 um = act ? ld4(u + c - sk) : zero, uc = act ? ld4(u + c) : zero;
+    const int quads = (g.hi[0] + 3) >> 2, lane = threadIdx.x & 31;
+    const int t = blockIdx.x * 256 + threadIdx.x;
+    const int j = g.lo[1] + t / quads, i0 = t % quads * 4;
+    const int k0 = g.lo[2] + blockIdx.y * kchunk, k1 = min(k0 + kchunk, g.hi[2]);
+    const bool act = j < g.hi[1] && i0 + 4 > g.lo[0];
+    // x neighbours come by shuffle.  A lane that starts a row gets another row's value on its
+    // left, but x = 0 is no unknown.
+    const bool ldl = act && lane == 0, ldr = act && (lane == 31 || i0 + 4 >= g.hi[0]) && i0 + 4 < g.sj;
+    const bool m0 = i0 >= g.lo[0] && i0 < g.hi[0], m1 = i0 + 1 >= g.lo[0] && i0 + 1 < g.hi[0];
+    const bool m2 = i0 + 2 >= g.lo[0] && i0 + 2 < g.hi[0], m3 = i0 + 3 >= g.lo[0] && i0 + 3 < g.hi[0];
+    const bool all4 = m0 && m1 && m2 && m3;
+    const float cc = (float)cf.cc, cx = (float)cf.cx, cy = (float)cf.cy, cz = (float)cf.cz;
+    const float2 cc2 = make_float2(cc, cc), cx2 = make_float2(cx, cx), cy2 = make_float2(cy, cy), cz2 = make_float2(cz, cz);
+    const long long sj = g.sj, sk = g.sk;
+    long long c = i0 + sj * j + sk * k0;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 um = act ? ld4(u + c - sk) : zero, uc = act ? ld4(u + c) : zero;
+    Acc2 a1, a2;
 #pragma unroll 1
-        for (int k = q.k0; k < q.k1; k++) {
-            const float4 up = act ? ld4(u + c + sk) : zero;
-            const float4 uy = act ? add4(ld4(u + c - sj), ld4(u + c + sj)) : zero;
-            float left = __shfl_up_sync(0xffffffffu, uc.w, 1), right = __shfl_down_sync(0xffffffffu, uc.x, 1);
-            if (lane == 0) left = act ? u[c - 1] : 0.f;
-            if (lane == 31) right = act && q.i0 + 4 < sj ? u[c + 4] : 0.f;
-            float4 a;
-            a.x = fmx(cz, um.x + up.x, fmx(cy, uy.x, fmx(cx, left + uc.y, cc * uc.x)));
-            a.y = fmx(cz, um.y + up.y, fmx(cy, uy.y, fmx(cx, uc.x + uc.z, cc * uc.y)));
-            a.z = fmx(cz, um.z + up.z, fmx(cy, uy.z, fmx(cx, uc.y + uc.w, cc * uc.z)));
-            a.w = fmx(cz, um.w + up.w, fmx(cy, uy.w, fmx(cx, uc.z + right, cc * uc.w)));
-            if (act) {
-                const float4 w4 = ld4(wv + c);
-                if (all4) {
-                    *reinterpret_cast<float4*>(Au + c) = a;
-                } else {
-                    if (m0) Au[c] = a.x;
-                    if (m1) Au[c + 1] = a.y;
-                    if (m2) Au[c + 2] = a.z;
-                    if (m3) Au[c + 3] = a.w;
-                }
-                if (m0) {
-                    a1.add(w4.x, a.x);
-                    if (NS == 2) a2.add(a.x, a.x);
-                }
-                if (m1) {
-                    a1.add(w4.y, a.y);
-                    if (NS == 2) a2.add(a.y, a.y);
-                }
-                if (m2) {
-                    a1.add(w4.z, a.z);
-                    if (NS == 2) a2.add(a.z, a.z);
-                }
-                if (m3) {
-                    a1.add(w4.w, a.w);
-                    if (NS == 2) a2.add(a.w, a.w);
-                }
+    for (int k = k0; k < k1; k++) {
+        const float4 up = act ? ld4(u + c + sk) : zero;
+        const float4 ys = act ? ld4(u + c - sj) : zero, yn = act ? ld4(u + c + sj) : zero;
+        float left = __shfl_up_sync(0xffffffffu, uc.w, 1), right = __shfl_down_sync(0xffffffffu, uc.x, 1);
+        if (ldl) left = u[c - 1];
+        if (ldr) right = u[c + 4];
+        const float2 x01 = make_float2(left + uc.y, uc.x + uc.z), x23 = make_float2(uc.y + uc.w, uc.z + right);
+        float2 lo = fma2(cx2, x01, mul2(cc2, lo2f(uc))), hi = fma2(cx2, x23, mul2(cc2, hi2f(uc)));
+        lo = fma2(cy2, add2(lo2f(ys), lo2f(yn)), lo);
+        hi = fma2(cy2, add2(hi2f(ys), hi2f(yn)), hi);
+        lo = fma2(cz2, add2(lo2f(um), lo2f(up)), lo);
+        hi = fma2(cz2, add2(hi2f(um), hi2f(up)), hi);
+        if (act) {
+            float4 w4 = ld4(wv + c);
+            if (all4) {
+                *reinterpret_cast<float4*>(Au + c) = make_float4(lo.x, lo.y, hi.x, hi.y);
+            } else {   // points that are no unknowns add zeros to the sums
+                if (m0) Au[c] = lo.x;
+                else lo.x = w4.x = 0.f;
+                if (m1) Au[c + 1] = lo.y;
+                else lo.y = w4.y = 0.f;
+                if (m2) Au[c + 2] = hi.x;
+                else hi.x = w4.z = 0.f;
+                if (m3) Au[c + 3] = hi.y;
+                else hi.y = w4.w = 0.f;
             }
-            um = uc;
-            uc = up;
-            c += sk;
+            a1.add(lo2f(w4), lo);
+            a1.add(hi2f(w4), hi);
+            if (NS == 2) {
+                a2.add(lo, lo);
+                a2.add(hi, hi);
+            }
         }
+        um = uc;
+        uc = up;
+        c += sk;
     }
-    if (NS == 1) {
-        double v[1] = {a1.value()};
-        reduce_finalize<1>(v, rc);
-    } else {
-        double v[2] = {a1.value(), a2.value()};
-        reduce_finalize<2>(v, rc);
-    }
+    double v[NS];
+    v[0] = a1.value();
+    if (NS == 2) v[NS - 1] = a2.value();
+    reduce_finalize<NS>(v, rc);
 }
 
 // r = b - A x in FP64 (computeErrorOperatorA, iterativeSolverBase.hpp:236-280),
@@ -2569,7 +2597,7 @@ __global__ void __launch_bounds__(256) k_cheb_iso64(Geo g, Shape sh, const doubl
 // Au = A u with the six-neighbour sum on the integer pipe (equal spacings), and
 // NS = 1: sum w.Au (k_stencil_dot, w = r0); NS = 2: sums w.Au, Au.Au (k_stencil_dot2,
 // w = r).  Three FP64 operations per unknown for A u instead of seven.
-template <int NS>
+template <int NS, bool CELLS>
 __global__ void __launch_bounds__(256, 4) k_stencil_dots_iso64(Geo g, Shape sh, const double* __restrict__ u,
                                                             const double* __restrict__ w, double* __restrict__ Au,
                                                             Coef cf, RedCtx rc)
@@ -2610,7 +2638,8 @@ __global__ void __launch_bounds__(256, 4) k_stencil_dots_iso64(Geo g, Shape sh, 
     double v[NS];
     v[0] = a1.value();
     if (NS == 2) v[NS - 1] = a2.value();
-    reduce_emit<NS>(v, rc, sh);
+    if (CELLS) store_cells<NS>(v, rc, sh);
+    else reduce_finalize<NS>(v, rc);
 }
 
 // out = r - A z at the unknowns (equal spacings, the neighbour sum on the integer pipe).
@@ -3102,6 +3131,30 @@ void fast_scale_copy(const Geo& g, const Shape& sh, const T* B, T* X, double a, 
     launch_pdl(k_scale_copy<T>, grid_of(sh), block_of(sh), 0, s, g, sh, B, X, (T)a, done);
     PPS_COUNT_LAUNCH();
 }
+// Grid of k_stencil_dots_v4: 256 float4s a tile, and z chunks that fill whole waves of
+// resident blocks, as few as do (every block pays the FP64 of its sums), of 2 planes or more.
+struct DotsGrid {
+    unsigned tiles, chunks;
+    int kchunk;
+};
+static DotsGrid dots_grid(const Geo& g)
+{
+    DotsGrid d;
+    const int uz = g.hi[2] - g.lo[2];
+    const long long rows = g.hi[1] - g.lo[1], quads = (g.hi[0] + 3) / 4, wave = (long long)DOTS_RESIDENT * sm_count();
+    d.tiles = (unsigned)((rows * quads + 255) / 256);
+    long long chunks = 1, full = 0;
+    for (int m = 1; m <= 4 && full * 10 < 9 * wave; m++) {   // 9 tenths of m waves will do
+        const long long n = std::max(1LL, m * wave / d.tiles), f = n * d.tiles / m;
+        if (f > full && f <= wave) chunks = n, full = f;
+    }
+    if (full == 0) chunks = std::max(1LL, 4 * wave / d.tiles);
+    // 100 x 90 x 110: 8.8 ms a solve with chunks of 2 planes, 9.4 with 4, 10.3 with 8
+    chunks = std::min(chunks, (long long)std::max(1, uz / 2));
+    d.kchunk = (int)((uz + chunks - 1) / chunks);
+    d.chunks = (unsigned)((uz + d.kchunk - 1) / d.kchunk);
+    return d;
+}
 template <typename T>
 void fast_stencil_dot(const Geo& g, const Shape& sh, const T* u, const T* r0, T* Au, const Coef& a, RedCtx rc,
                       cudaStream_t s)
@@ -3109,10 +3162,15 @@ void fast_stencil_dot(const Geo& g, const Shape& sh, const T* u, const T* r0, T*
     if constexpr (std::is_same<T, double>::value) {
         if (iso_coef(a)) {   // equal spacings: the neighbour sum on the integer pipe
             Shape c = sh.cx == 1 ? sh : make_shape(g, sh.ty, (int)sh.nblocks(), 1);
-            if (rc.cells) canon_launch(g, c, rc);
-            launch_pdl(k_stencil_dots_iso64<1>, grid_of(c), block_of(c), 0, s, g, c, u, r0, Au, a, rc);
+            if (rc.cells) {
+                canon_launch(g, c, rc);
+                launch_pdl(k_stencil_dots_iso64<1, true>, grid_of(c), block_of(c), 0, s, g, c, u, r0, Au, a, rc);
+                PPS_COUNT_LAUNCH();
+                canon_finalize<1>(rc, &rc.st->done, s);
+                return;
+            }
+            launch_pdl(k_stencil_dots_iso64<1, false>, grid_of(c), block_of(c), 0, s, g, c, u, r0, Au, a, rc);
             PPS_COUNT_LAUNCH();
-            if (rc.cells) canon_finalize<1>(rc, &rc.st->done, s);
             return;
         }
     }
@@ -3127,7 +3185,8 @@ void fast_stencil_dot(const Geo& g, const Shape& sh, const T* u, const T* r0, T*
     if (sh.cx != 1) {   // the Chebyshev tiles: x-vectorised FP32, else the one-column tiles
         if constexpr (std::is_same<T, float>::value) {
             if (sh.cx == 4 && v4_ok<T>(g, u, r0, Au, nullptr)) {
-                launch_pdl(k_stencil_dots_v4<1>, grid_of(sh), block_of(sh), 0, s, g, sh, u, r0, Au, a, rc);
+                const DotsGrid d = dots_grid(g);
+                launch_pdl(k_stencil_dots_v4<1>, dim3(d.tiles, d.chunks), 256, 0, s, g, d.kchunk, u, r0, Au, a, rc);
                 PPS_COUNT_LAUNCH();
                 return;
             }
@@ -3145,10 +3204,15 @@ void fast_stencil_dot2(const Geo& g, const Shape& sh, const T* u, const T* r, T*
     if constexpr (std::is_same<T, double>::value) {
         if (iso_coef(a)) {   // equal spacings: the neighbour sum on the integer pipe
             Shape c = sh.cx == 1 ? sh : make_shape(g, sh.ty, (int)sh.nblocks(), 1);
-            if (rc.cells) canon_launch(g, c, rc);
-            launch_pdl(k_stencil_dots_iso64<2>, grid_of(c), block_of(c), 0, s, g, c, u, r, Au, a, rc);
+            if (rc.cells) {
+                canon_launch(g, c, rc);
+                launch_pdl(k_stencil_dots_iso64<2, true>, grid_of(c), block_of(c), 0, s, g, c, u, r, Au, a, rc);
+                PPS_COUNT_LAUNCH();
+                canon_finalize<2>(rc, &rc.st->done, s);
+                return;
+            }
+            launch_pdl(k_stencil_dots_iso64<2, false>, grid_of(c), block_of(c), 0, s, g, c, u, r, Au, a, rc);
             PPS_COUNT_LAUNCH();
-            if (rc.cells) canon_finalize<2>(rc, &rc.st->done, s);
             return;
         }
     }
@@ -3163,7 +3227,8 @@ void fast_stencil_dot2(const Geo& g, const Shape& sh, const T* u, const T* r, T*
     if (sh.cx != 1) {
         if constexpr (std::is_same<T, float>::value) {
             if (sh.cx == 4 && v4_ok<T>(g, u, r, Au, nullptr)) {
-                launch_pdl(k_stencil_dots_v4<2>, grid_of(sh), block_of(sh), 0, s, g, sh, u, r, Au, a, rc);
+                const DotsGrid d = dots_grid(g);
+                launch_pdl(k_stencil_dots_v4<2>, dim3(d.tiles, d.chunks), 256, 0, s, g, d.kchunk, u, r, Au, a, rc);
                 PPS_COUNT_LAUNCH();
                 return;
             }
@@ -3211,7 +3276,7 @@ void fast_update_xr(const Geo& g, const Shape& sh, T* x, const T* Mp, const T* z
     if (rc.cells) {
         Shape c = sh;
         canon_launch(g, c, rc);
-        launch_pdl(k_update_xr<T>, grid_of(c), block_of(c), 0, s, g, c, x, Mp, z, r, Az, r0, rc);
+        launch_pdl(k_update_xr<T, true>, grid_of(c), block_of(c), 0, s, g, c, x, Mp, z, r, Az, r0, rc);
         PPS_COUNT_LAUNCH();
         canon_finalize<2>(rc, &rc.st->done, s);
         return;
@@ -3221,7 +3286,7 @@ void fast_update_xr(const Geo& g, const Shape& sh, T* x, const T* Mp, const T* z
         PPS_COUNT_LAUNCH();
         return;
     }
-    launch_pdl(k_update_xr<T>, grid_of(sh), block_of(sh), 0, s, g, sh, x, Mp, z, r, Az, r0, rc);
+    launch_pdl(k_update_xr<T, false>, grid_of(sh), block_of(sh), 0, s, g, sh, x, Mp, z, r, Az, r0, rc);
     PPS_COUNT_LAUNCH();
 }
 template <typename T>
