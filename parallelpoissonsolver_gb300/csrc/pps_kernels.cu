@@ -727,6 +727,17 @@ struct CT {
     T cc, cx, cy, cz, cb, cw;
 };
 
+// The operator's weights in the kernel's type, converted by the host: converted in the
+// kernel, the compiler repeated the four conversions (FP64 pipe, 16 clocks a warp each) for
+// every plane to save registers, and k_stencil_dots_v4<1> kept that pipe busy for 73% of its
+// 50 us on 256^3 unknowns (46 us with this).  k_fcg_p_stencil_v4, which memory bounds, converts by
+// itself: with these weights it took 417 us instead of 402 on 512^3.
+template <typename T>
+static CT<T> as_coef(const Coef& c)
+{
+    return CT<T>{(T)c.cc, (T)c.cx, (T)c.cy, (T)c.cz, T(0), T(0)};
+}
+
 template <typename T>
 static CT<T> cast_coef(const Coef& c)
 {
@@ -1579,14 +1590,14 @@ __global__ void __launch_bounds__(256) k_scale_copy(Geo g, Shape sh, const T* __
 // Au = A(u); sum r0*Au   (BiCGSTAB.hpp:142-164, BiCGstab1Kernel)
 template <typename T>
 __global__ void __launch_bounds__(256) k_stencil_dot(Geo g, Shape sh, const T* __restrict__ u,
-                                                     const T* __restrict__ r0, T* __restrict__ Au, Coef cf, RedCtx rc)
+                                                     const T* __restrict__ r0, T* __restrict__ Au, CT<T> cf, RedCtx rc)
 {
     pdl_enter();
     EARLY_EXIT(&rc.st->done);
     const Col q = column(g, sh);
     Acc<T> acc;
     if (q.active) {
-        const T cc = (T)cf.cc, cx = (T)cf.cx, cy = (T)cf.cy, cz = (T)cf.cz;
+        const T cc = cf.cc, cx = cf.cx, cy = cf.cy, cz = cf.cz;
         const long long sj = g.sj, sk = g.sk;
         long long c = q.c;
         T um = u[c - sk], uc = u[c];
@@ -1613,14 +1624,14 @@ __global__ void __launch_bounds__(256) k_stencil_dot(Geo g, Shape sh, const T* _
 // Au = A(u); sum r*Au, sum Au*Au   (BiCGSTAB.hpp:189-225, BiCGstab2Kernel)
 template <typename T>
 __global__ void __launch_bounds__(256) k_stencil_dot2(Geo g, Shape sh, const T* __restrict__ u,
-                                                      const T* __restrict__ r, T* __restrict__ Au, Coef cf, RedCtx rc)
+                                                      const T* __restrict__ r, T* __restrict__ Au, CT<T> cf, RedCtx rc)
 {
     pdl_enter();
     EARLY_EXIT(&rc.st->done);
     const Col q = column(g, sh);
     Acc<T> a1, a2;
     if (q.active) {
-        const T cc = (T)cf.cc, cx = (T)cf.cx, cy = (T)cf.cy, cz = (T)cf.cz;
+        const T cc = cf.cc, cx = cf.cx, cy = cf.cy, cz = cf.cz;
         const long long sj = g.sj, sk = g.sk;
         long long c = q.c;
         T um = u[c - sk], uc = u[c];
@@ -1715,14 +1726,14 @@ __global__ void __launch_bounds__(256) k_update_p(Geo g, Shape sh, T* __restrict
 template <typename T>
 __global__ void __launch_bounds__(256) k_cg_stencil_dot(Geo g, Shape sh, const T* __restrict__ p,
                                                         const T* __restrict__ r, const T* __restrict__ z,
-                                                        T* __restrict__ Ap, Coef cf, RedCtx rc)
+                                                        T* __restrict__ Ap, CT<T> cf, RedCtx rc)
 {
     pdl_enter();
     EARLY_EXIT(&rc.st->done);
     const Col q = column(g, sh);
     Acc<T> a1, a2;
     if (q.active) {
-        const T cc = (T)cf.cc, cx = (T)cf.cx, cy = (T)cf.cy, cz = (T)cf.cz;
+        const T cc = cf.cc, cx = cf.cx, cy = cf.cy, cz = cf.cz;
         const long long sj = g.sj, sk = g.sk;
         long long c = q.c;
         T um = p[c - sk], uc = p[c];
@@ -1813,14 +1824,14 @@ __global__ void __launch_bounds__(256) k_cg_update_p(Geo g, Shape sh, T* __restr
 template <typename T>
 __global__ void __launch_bounds__(256) k_fcg_p_stencil(Geo g, Shape sh, const T* __restrict__ z,
                                                        const T* __restrict__ pin, T* __restrict__ pout,
-                                                       T* __restrict__ Ap, Coef cf, RedCtx rc)
+                                                       T* __restrict__ Ap, CT<T> cf, RedCtx rc)
 {
     pdl_enter();
     EARLY_EXIT(&rc.st->done);
     const Col q = column(g, sh);
     Acc<T> a1;
     if (q.active) {
-        const T cc = (T)cf.cc, cx = (T)cf.cx, cy = (T)cf.cy, cz = (T)cf.cz;
+        const T cc = cf.cc, cx = cf.cx, cy = cf.cy, cz = cf.cz;
         const bool restart = rc.st->beta == 0.0;
         const T be = (T)rc.st->beta;
         const long long sj = g.sj, sk = g.sk;
@@ -1986,7 +1997,7 @@ static size_t stage_smem_bytes(int ty)
 // what the guard cells the register-marching kernel reads there hold.
 __global__ void __launch_bounds__(256) k_fcg_p_stencil_staged(Geo g, Shape sh, const __grid_constant__ CUtensorMap tz,
                                                               const __grid_constant__ CUtensorMap tp,
-                                                              float* __restrict__ pout, float* __restrict__ Ap, Coef cf,
+                                                              float* __restrict__ pout, float* __restrict__ Ap, CT<float> cf,
                                                               RedCtx rc)
 {
     pdl_enter();
@@ -2041,7 +2052,7 @@ __global__ void __launch_bounds__(256) k_fcg_p_stencil_staged(Geo g, Shape sh, c
     const bool m0 = q.i0 >= g.lo[0] && q.i0 < g.hi[0], m1 = q.i0 + 1 >= g.lo[0] && q.i0 + 1 < g.hi[0];
     const bool m2 = q.i0 + 2 >= g.lo[0] && q.i0 + 2 < g.hi[0], m3 = q.i0 + 3 >= g.lo[0] && q.i0 + 3 < g.hi[0];
     const bool all4 = m0 && m1 && m2 && m3;
-    const float cc = (float)cf.cc, cx = (float)cf.cx, cy = (float)cf.cy, cz = (float)cf.cz;
+    const float cc = cf.cc, cx = cf.cx, cy = cf.cy, cz = cf.cz;
     const float be = (float)rc.st->beta;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     const int xo = q.i0 - xs;   // the thread's float4 in a staged row (4 * lane + 4)
@@ -2393,7 +2404,7 @@ struct Acc2 {
 template <int NS>
 __global__ void __launch_bounds__(256, DOTS_RESIDENT) k_stencil_dots_v4(Geo g, int kchunk, const float* __restrict__ u,
                                                                         const float* __restrict__ wv,
-                                                                        float* __restrict__ Au, Coef cf, RedCtx rc)
+                                                                        float* __restrict__ Au, CT<float> cf, RedCtx rc)
 {
     pdl_enter();
     EARLY_EXIT(&rc.st->done);
@@ -2408,7 +2419,7 @@ __global__ void __launch_bounds__(256, DOTS_RESIDENT) k_stencil_dots_v4(Geo g, i
     const bool m0 = i0 >= g.lo[0] && i0 < g.hi[0], m1 = i0 + 1 >= g.lo[0] && i0 + 1 < g.hi[0];
     const bool m2 = i0 + 2 >= g.lo[0] && i0 + 2 < g.hi[0], m3 = i0 + 3 >= g.lo[0] && i0 + 3 < g.hi[0];
     const bool all4 = m0 && m1 && m2 && m3;
-    const float cc = (float)cf.cc, cx = (float)cf.cx, cy = (float)cf.cy, cz = (float)cf.cz;
+    const float cc = cf.cc, cx = cf.cx, cy = cf.cy, cz = cf.cz;
     const float2 cc2 = make_float2(cc, cc), cx2 = make_float2(cx, cx), cy2 = make_float2(cy, cy), cz2 = make_float2(cz, cz);
     const long long sj = g.sj, sk = g.sk;
     long long c = i0 + sj * j + sk * k0;
@@ -3177,7 +3188,7 @@ void fast_stencil_dot(const Geo& g, const Shape& sh, const T* u, const T* r0, T*
     if (rc.cells) {   // canonical sums: one-column kernel on the canonical shape
         Shape c = sh;
         canon_launch(g, c, rc);
-        launch_pdl(k_stencil_dot<T>, grid_of(c), block_of(c), 0, s, g, c, u, r0, Au, a, rc);
+        launch_pdl(k_stencil_dot<T>, grid_of(c), block_of(c), 0, s, g, c, u, r0, Au, as_coef<T>(a), rc);
         PPS_COUNT_LAUNCH();
         canon_finalize<1>(rc, &rc.st->done, s);
         return;
@@ -3186,7 +3197,7 @@ void fast_stencil_dot(const Geo& g, const Shape& sh, const T* u, const T* r0, T*
         if constexpr (std::is_same<T, float>::value) {
             if (sh.cx == 4 && v4_ok<T>(g, u, r0, Au, nullptr)) {
                 const DotsGrid d = dots_grid(g);
-                launch_pdl(k_stencil_dots_v4<1>, dim3(d.tiles, d.chunks), 256, 0, s, g, d.kchunk, u, r0, Au, a, rc);
+                launch_pdl(k_stencil_dots_v4<1>, dim3(d.tiles, d.chunks), 256, 0, s, g, d.kchunk, u, r0, Au, as_coef<float>(a), rc);
                 PPS_COUNT_LAUNCH();
                 return;
             }
@@ -3194,7 +3205,7 @@ void fast_stencil_dot(const Geo& g, const Shape& sh, const T* u, const T* r0, T*
         fast_stencil_dot<T>(g, make_shape(g, sh.ty, (int)sh.nblocks(), 1), u, r0, Au, a, rc, s);
         return;
     }
-    launch_pdl(k_stencil_dot<T>, grid_of(sh), block_of(sh), 0, s, g, sh, u, r0, Au, a, rc);
+    launch_pdl(k_stencil_dot<T>, grid_of(sh), block_of(sh), 0, s, g, sh, u, r0, Au, as_coef<T>(a), rc);
     PPS_COUNT_LAUNCH();
 }
 template <typename T>
@@ -3219,7 +3230,7 @@ void fast_stencil_dot2(const Geo& g, const Shape& sh, const T* u, const T* r, T*
     if (rc.cells) {
         Shape c = sh;
         canon_launch(g, c, rc);
-        launch_pdl(k_stencil_dot2<T>, grid_of(c), block_of(c), 0, s, g, c, u, r, Au, a, rc);
+        launch_pdl(k_stencil_dot2<T>, grid_of(c), block_of(c), 0, s, g, c, u, r, Au, as_coef<T>(a), rc);
         PPS_COUNT_LAUNCH();
         canon_finalize<2>(rc, &rc.st->done, s);
         return;
@@ -3228,7 +3239,7 @@ void fast_stencil_dot2(const Geo& g, const Shape& sh, const T* u, const T* r, T*
         if constexpr (std::is_same<T, float>::value) {
             if (sh.cx == 4 && v4_ok<T>(g, u, r, Au, nullptr)) {
                 const DotsGrid d = dots_grid(g);
-                launch_pdl(k_stencil_dots_v4<2>, dim3(d.tiles, d.chunks), 256, 0, s, g, d.kchunk, u, r, Au, a, rc);
+                launch_pdl(k_stencil_dots_v4<2>, dim3(d.tiles, d.chunks), 256, 0, s, g, d.kchunk, u, r, Au, as_coef<float>(a), rc);
                 PPS_COUNT_LAUNCH();
                 return;
             }
@@ -3236,7 +3247,7 @@ void fast_stencil_dot2(const Geo& g, const Shape& sh, const T* u, const T* r, T*
         fast_stencil_dot2<T>(g, make_shape(g, sh.ty, (int)sh.nblocks(), 1), u, r, Au, a, rc, s);
         return;
     }
-    launch_pdl(k_stencil_dot2<T>, grid_of(sh), block_of(sh), 0, s, g, sh, u, r, Au, a, rc);
+    launch_pdl(k_stencil_dot2<T>, grid_of(sh), block_of(sh), 0, s, g, sh, u, r, Au, as_coef<T>(a), rc);
     PPS_COUNT_LAUNCH();
 }
 // Dirichlet grids with 16-byte aligned fields: the flat vector forms of the updates.
@@ -3307,12 +3318,12 @@ void fast_cg_stencil_dot(const Geo& g, const Shape& sh, const T* p, const T* r, 
     if (rc.cells) {
         Shape c = sh;
         canon_launch(g, c, rc);
-        launch_pdl(k_cg_stencil_dot<T>, grid_of(c), block_of(c), 0, s, g, c, p, r, z, Ap, a, rc);
+        launch_pdl(k_cg_stencil_dot<T>, grid_of(c), block_of(c), 0, s, g, c, p, r, z, Ap, as_coef<T>(a), rc);
         PPS_COUNT_LAUNCH();
         canon_finalize<2>(rc, &rc.st->done, s);
         return;
     }
-    launch_pdl(k_cg_stencil_dot<T>, grid_of(sh), block_of(sh), 0, s, g, sh, p, r, z, Ap, a, rc);
+    launch_pdl(k_cg_stencil_dot<T>, grid_of(sh), block_of(sh), 0, s, g, sh, p, r, z, Ap, as_coef<T>(a), rc);
     PPS_COUNT_LAUNCH();
 }
 template <typename T>
@@ -3422,7 +3433,7 @@ void fast_fcg_p_stencil(const Geo& g, const Shape& sh, const T* z, const T* pin,
                         attr_set = (int)smem;
                     }
                     launch_pdl(k_fcg_p_stencil_staged, grid_of(sh), block_of(sh), smem, s, g, sh, mz, mp, pout, Ap,
-                               a, rc);
+                               as_coef<float>(a), rc);
                 } else {
                     launch_pdl(k_fcg_p_stencil_v4, grid_of(sh), block_of(sh), 0, s, g, sh, z, pin, pout, Ap, a, rc);
                 }
@@ -3444,7 +3455,7 @@ void fast_fcg_p_stencil(const Geo& g, const Shape& sh, const T* z, const T* pin,
             return;
         }
     }
-    launch_pdl(k_fcg_p_stencil<T>, grid_of(sh), block_of(sh), 0, s, g, sh, z, pin, pout, Ap, a, rc);
+    launch_pdl(k_fcg_p_stencil<T>, grid_of(sh), block_of(sh), 0, s, g, sh, z, pin, pout, Ap, as_coef<T>(a), rc);
     PPS_COUNT_LAUNCH();
 }
 void flag_nonzero(long long n, const double* x, int* flag, cudaStream_t s)
