@@ -2796,13 +2796,24 @@ __global__ void __launch_bounds__(256) k_residual(Geo g, Shape sh, const double*
         const long long sj = g.sj, sk = g.sk;
         long long c = q.c;
         MI um = msplit(x[c - sk]), uc = msplit(x[c]);
+        double xp = x[c + sk], xw = x[c - 1], xe = x[c + 1], xs = x[c - sj], xn = x[c + sj], bn = b[c];
+#pragma unroll 1
         for (int k = q.k0; k < q.k1; k++) {
-            const MI up = msplit(x[c + sk]);
-            const MI w = msplit(x[c - 1]), e = msplit(x[c + 1]), sv = msplit(x[c - sj]), nv = msplit(x[c + sj]);
+            const MI up = msplit(xp), w = msplit(xw), e = msplit(xe), sv = msplit(xs), nv = msplit(xn);
+            const double bv = bn;
+            if (k + 1 < q.k1) {   // the next plane's loads, under way while this one is summed
+                const long long o = c + sk;
+                xp = x[o + sk];
+                xw = x[o - 1];
+                xe = x[o + 1];
+                xs = x[o - sj];
+                xn = x[o + sj];
+                bn = b[o];
+            }
             const int E = max(max(max(um.e, uc.e), max(up.e, w.e)), max(max(e.e, sv.e), nv.e));
             double rv;
             if (E == 2047) {   // an Inf or NaN: let FP64 arithmetic propagate it
-                rv = b[c] - cf.cx * (x[c - 1] + x[c + 1] + x[c - sj] + x[c + sj] + x[c - sk] + x[c + sk] - 6.0 * x[c]);
+                rv = bv - cf.cx * (x[c - 1] + x[c + 1] + x[c - sj] + x[c + sj] + x[c - sk] + x[c + sk] - 6.0 * x[c]);
             } else {
                 const long long D = malign(w, E) + malign(e, E) + malign(sv, E) + malign(nv, E) + malign(um, E) +
                                     malign(up, E) - 6 * malign(uc, E);
@@ -2813,14 +2824,14 @@ __global__ void __launch_bounds__(256) k_residual(Geo g, Shape sh, const double*
                 if (E >= 53 && E <= 2000) {
                     const double Ds = D != 0 ? __longlong_as_double(__double_as_longlong(Dd) + ((long long)(E - 1075) << 52))
                                              : 0.0;
-                    rv = fmx(-cf.cx, Ds, b[c]);
+                    rv = fmx(-cf.cx, Ds, bv);
                 } else if (E > 2000) {
                     // magnitudes near the top of the range: cx * D first, then the power of
                     // two 2^(E-1075) (a normal double), so nothing overflows while A x is
                     // finite, and D = 0 gives b exactly
-                    rv = fmx(-(cf.cx * Dd), __longlong_as_double((long long)(E - 52) << 52), b[c]);
+                    rv = fmx(-(cf.cx * Dd), __longlong_as_double((long long)(E - 52) << 52), bv);
                 } else {
-                    rv = b[c];   // every value below 2^-1022: A x is far under b's rounding
+                    rv = bv;   // every value below 2^-1022: A x is far under b's rounding
                 }
             }
             const TR rs = (TR)rv;
