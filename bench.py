@@ -58,7 +58,6 @@ DEGREE = 11
 # convergence at 512^3 on the GB300 host (16 threads: 172 s, true ||r||/||b|| 9.3e-11).
 # The CPU leg multiplies its timed per-iteration cost by it.
 REFERENCE_ITERATIONS = {512: 166}
-PROFILE_TRAFFIC = os.path.join(ROOT, "profiles", "cheb_sweep_fp32_traffic.txt")
 PROFILE_TRAFFIC_FCG = os.path.join(ROOT, "profiles", "fcg_kernels_traffic.txt")
 
 
@@ -165,9 +164,8 @@ def measured_peaks():
     return 6800.0, "fallback"
 
 
-def traffic_ratio(path=PROFILE_TRAFFIC):
-    """dram bytes / algorithmic bytes of the kernel a committed ncu summary covers
-    (default: one FP32 sweep launch)."""
+def traffic_ratio(path):
+    """dram bytes / algorithmic bytes of the kernels a committed ncu summary covers."""
     if not os.path.exists(path):
         return None
     for line in open(path):
@@ -327,14 +325,13 @@ def run_gpu(args, dist: Dist):
     kry_b = sum(s["krylov_bytes"] for s in kstats)
     kry_n = sum(s["krylov_launches"] for s in kstats)
 
-    # ---- roofline of the FP32 Chebyshev sweep (the reference method's dominant kernel),
-    # event-timed in the mixed BiCGSTAB solves (degree 11: all 16 B sweeps) ----
+    # ---- roofline of the FP32 Chebyshev passes (the reference method's dominant kernel),
+    # event-timed in the mixed BiCGSTAB solves (degree 11: three passes of three steps) ----
     sweep_s = sum(s["sweep_seconds"] for s in mixed_stats)
     sweep_n = sum(s["sweep_launches"] for s in mixed_stats)
     sweep_b = sum(s["sweep_bytes"] for s in mixed_stats)
     peak, peak_src = measured_peaks()
     achieved = (sweep_b / sweep_s) / 1e9 if sweep_s > 0 else None
-    ratio = traffic_ratio()
     per_launch_alg = sweep_b / sweep_n if sweep_n else None
 
     def summary(s, t):
@@ -408,15 +405,15 @@ def run_gpu(args, dist: Dist):
         },
         "roofline_sweep": {
             "bound": "hbm",
-            "kernel": "k_cheb_v4<1>, k_cheb_v4<2> (the FP32 Chebyshev sweeps, one float4 per thread: Y with its "
-                      "6 neighbours, B, [Z] in, W out; 12 / 16 B per unknown; timed in the mixed BiCGSTAB solves, "
-                      "the smoother kernels of the headline too)",
+            "kernel": "k_cheb3<0>, k_cheb3<2> (the FP32 Chebyshev passes of three steps each: B, [Y, Z] in, the last "
+                      "two iterates out; 12, 20 and 16 B per unknown and pass, a third of that per step; timed in "
+                      "the mixed BiCGSTAB solves, the smoother of the headline too)",
             "achieved": achieved,
             "peak": peak,
             "unit": "GB/s",
             "frac": (achieved / peak) if achieved else None,
             "peak_source": f"{peak_src} (MEASURED_PEAKS.json hbm_gbs)" if peak_src == "measured" else peak_src,
-            "traffic": (ratio * per_launch_alg) if (ratio and per_launch_alg) else None,
+            "traffic": None,   # no ncu capture of these passes: the committed one is of the one-step sweep
             "algorithmic_bytes_per_launch": per_launch_alg,
             "launches_timed": sweep_n,
         },
