@@ -413,7 +413,8 @@ pps_status pps_prolong2(int nx, int ny, int nz, const float* coarse_dev, float* 
  * device current and keeps it; make that first call before any stream capture,
  * and do not use the entry point across a cudaDeviceReset.  All calls
  * share the one array, so calls that overlap on the GPU (other streams, other
- * threads) race: serialise them. */
+ * threads) race: serialise them.  The energies of calls that overlapped are
+ * undefined; calls made after they ended are not affected. */
 #define PPS_NOALLOC_MAX_BLOCKS 16384
 pps_status pps_apply_operator_noalloc(const pps_grid* grid, const double* u_dev, double* out_dev,
                                       double* energy_dev, void* stream);

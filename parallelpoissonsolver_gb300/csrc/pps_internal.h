@@ -29,6 +29,26 @@ __device__ __forceinline__ void pdl_enter()
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 #endif
+
+// What block `bid` of `nblocks` adds to a completion counter that outlives the launch.  The
+// shares of a launch come to 2^32, which is 0: the counter is back at zero when, and
+// before that never but at the start, all blocks have counted.  So nothing resets it, and
+// two launches that overlap on one counter by mistake still leave it at zero when both have
+// ended (a count from zero that the last block resets keeps what the other launch's blocks
+// added after the reset, and every later launch then ends too early).
+__host__ __device__ constexpr unsigned block_share(unsigned bid, unsigned nblocks)
+{
+    return bid == 0 ? 1u - nblocks : 1u;
+}
+#ifdef __CUDACC__
+// Counts the calling block (one thread calls it, the block's results stored and fenced);
+// true in the launch's last block.
+__device__ __forceinline__ bool count_block(unsigned* counter, unsigned bid, unsigned nblocks)
+{
+    const unsigned share = block_share(bid, nblocks);
+    return atomicAdd(counter, share) + share == 0u;
+}
+#endif
 // Kernel launches that failed on this thread.  A failed launch leaves no sticky CUDA
 // error for a later synchronisation to report, so the entry points compare this count
 // before and after their work and return PPS_ERR_CUDA when it grew.
@@ -157,7 +177,7 @@ enum FinKind : int {
 
 struct RedCtx {
     double* partials;   // nblocks * 4 doubles
-    unsigned* counter;  // zero between launches; the last block resets it
+    unsigned* counter;  // zero between launches (count_block)
     DevState* st;
     double* hist;
     int kind;

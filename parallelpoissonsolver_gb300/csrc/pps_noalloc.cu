@@ -120,10 +120,11 @@ extern "C" pps_status pps_apply_operator_noalloc(const pps_grid* grid, const dou
     DevState* st = (DevState*)(base + kStateOffset);
     unsigned* counter = (unsigned*)(base + kCounterOffset);
     double* partials = (double*)(base + kPartialsOffset);
-    // One launch: the scratch starts as zeros, the kernel's last block resets the
-    // completion counter, and a reduction that only stores never sets the stop flag, so
-    // no call has anything to reset (a state kernel, a fill and a copy of the energy
-    // around the stencil took 17 of 39 us on a 64 x 48 x 80 box).
+    // One launch: the scratch starts as zeros, the completion counter is back at zero when
+    // a launch ends (count_block; after overlapping launches too, whose energies are then
+    // undefined but not those of the calls after them), and a reduction that only stores
+    // never sets the stop flag, so no call has anything to reset (a state kernel, a fill
+    // and a copy of the energy around the stencil took 17 of 39 us on a 64 x 48 x 80 box).
     const unsigned long long failures = launch_failures();
 
     RedCtx rc;

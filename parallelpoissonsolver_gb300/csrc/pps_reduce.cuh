@@ -256,7 +256,7 @@ __device__ __forceinline__ void reduce_finalize(double (&v)[NS], const RedCtx& r
         __threadfence();
     });
     __syncthreads();
-    if (tid == 0) is_last = atomicAdd(rc.counter, 1u) == nblocks - 1;
+    if (tid == 0) is_last = count_block(rc.counter, bid, nblocks);
     __syncthreads();
     if (!is_last) return;
     __threadfence();
@@ -274,8 +274,6 @@ __device__ __forceinline__ void reduce_finalize(double (&v)[NS], const RedCtx& r
 #pragma unroll
         for (int q = 0; q < NS; q++) tot[q] = sm[q];
         finalize(rc, tot);
-        __threadfence();
-        *rc.counter = 0u;
     }
 }
 

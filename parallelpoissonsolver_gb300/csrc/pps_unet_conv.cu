@@ -811,16 +811,13 @@ __global__ void __launch_bounds__(256) k_rms(long long n, const float* __restric
     if (tid == 0) {
         sc->part[blockIdx.x] = s;
         __threadfence();
-        is_last = atomicAdd(&sc->count, 1u) == gridDim.x - 1;
+        is_last = count_block(&sc->count, blockIdx.x, gridDim.x);
     }
     __syncthreads();
     if (!is_last) return;
     __threadfence();
     s = block_sum(tid < (int)gridDim.x ? __ldcg(&sc->part[tid]) : 0.0);
-    if (tid == 0) {
-        *out = (float)sqrt(s / (double)(n > 0 ? n : 1));
-        sc->count = 0u;
-    }
+    if (tid == 0) *out = (float)sqrt(s / (double)(n > 0 ? n : 1));
 }
 
 void rms(long long n, const float* a, float* out, RmsScratch* scratch, cudaStream_t s)

@@ -97,7 +97,7 @@ void adam(const PackTable& T, int n, float* p, const float* g, float* m, float* 
           float b1, float b2, float eps, int step, const float* g_rms, float max_norm, cudaStream_t s);
 struct RmsScratch {
     double part[256];
-    unsigned count;   // zero between launches
+    unsigned count;   // zero between launches (count_block)
 };
 void rms(long long n, const float* a, float* out, RmsScratch* scratch, cudaStream_t s);
 // Lets the convolution kernels use the shared memory their tiles take (current device).
