@@ -400,7 +400,8 @@ pps_status pps_prolong2(int nx, int ny, int nz, const float* coarse_dev, float* 
  *
  * On device pointers of the field layout: out_dev = A u at the unknowns (the FP64
  * form's kernel; every other entry of out_dev is left as it was) and
- * *energy_dev = sum of u*(A u) over the unknowns.  u_dev, out_dev and energy_dev
+ * *energy_dev = sum of u*(A u) over the unknowns (8 bytes at any address, aligned or
+ * not; the fields are aligned to 8 bytes).  u_dev, out_dev and energy_dev
  * must not overlap (an in-place call is rejected with PPS_ERR_INVALID_ARG).  Work
  * is queued on `stream` (a cudaStream_t; NULL = the legacy default stream); the
  * call does not wait.

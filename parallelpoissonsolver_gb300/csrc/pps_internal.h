@@ -189,7 +189,7 @@ struct RedCtx {
     // k_canon_finalize then sums the cells in a fixed tree.  The result depends on
     // the grid alone, not on the tile shape the autotuner picked or the SM count.
     double* cells = nullptr;
-    double* store = nullptr;   // FIN_STORE: the first sum goes here as well
+    void* store = nullptr;   // FIN_STORE: the first sum goes here as well (any alignment)
     int cell_ntx = 0, cell_ny = 0;
     long long cell_n = 0;
 };

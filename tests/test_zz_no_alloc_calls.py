@@ -70,3 +70,18 @@ def test_calls_after_overlapping_ones_are_right(gpu):
         c.queue(streams[0])
     torch.cuda.synchronize()
     assert [c.grid.npglobal for c in calls if not c.right()] == []
+
+
+@pytest.mark.parametrize("offset", [1, 2, 4, 7])
+def test_the_energy_may_lie_at_any_address(gpu, offset):
+    torch = pytest.importorskip("torch")
+    for k, n in enumerate([(1, 1, 1), (64, 48, 80)]):
+        c = Call(torch, n, k)
+        room = torch.full((24,), 0xA5, dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+        c.queue(torch.cuda.current_stream(), room.data_ptr() + offset)
+        torch.cuda.synchronize()
+        got = room.cpu().numpy()
+        value = got[offset:offset + 8].copy().view(np.float64)[0]
+        assert abs(value - c.want) <= 1e-12 * c.scale
+        assert np.all(got[:offset] == 0xA5) and np.all(got[offset + 8:] == 0xA5)
