@@ -314,10 +314,10 @@ void fast_cheb_fused(const Geo& g, int nsteps, const T* B, T* X, const Coef* c, 
 template <typename T>
 void fast_cheb_sweep(const Geo& g, const Shape& sh, const T* Y, const T* B, const T* Z, T* W, const Coef& c,
                      const int* done, cudaStream_t s, bool mirror = true);
-// Three steps in one pass (FP32, Dirichlet, even rows on 8-byte boundaries: cheb3_ok).
+// Three steps in one pass (FP32, Dirichlet, even rows: cheb3_ok; fields on 8-byte boundaries).
 // mode 0: s1..s3 from U = B; 1: from U = s1 without Z; 2: from U, Z and B.  X = the third
 // step, X2 (may be null) the second.  No output may be an input.
-bool cheb3_ok(const Geo& g, std::initializer_list<const void*> ptrs);
+bool cheb3_ok(const Geo& g);
 cudaError_t cheb3_prepare();   // shared memory of its blocks (current device)
 void fast_cheb3(const Geo& g, int mode, const float* U, const float* B, const float* Z, float* X, float* X2,
                 const Coef* c, const int* done, cudaStream_t s);

@@ -82,7 +82,6 @@ template <typename T>
 struct Fields {
     T *p = nullptr, *r = nullptr, *r0 = nullptr, *Mp = nullptr, *AMp = nullptr, *z = nullptr, *Az = nullptr;
     T *Y = nullptr, *Z = nullptr, *W = nullptr, *e = nullptr;
-    T* V = nullptr;   // FP32: the Chebyshev passes' fourth buffer
 };
 
 }  // namespace
@@ -271,10 +270,6 @@ void alloc_fields(Fields<T>& F, long long ntot, bool with_e, bool with_cheb = tr
         CK(cudaMalloc((void**)q, sizeof(T) * (size_t)ntot));
         CK(cudaMemset(*q, 0, sizeof(T) * (size_t)ntot));
     }
-    if (with_cheb && sizeof(T) == 4) {
-        CK(cudaMalloc((void**)&F.V, sizeof(T) * (size_t)ntot));
-        CK(cudaMemset(F.V, 0, sizeof(T) * (size_t)ntot));
-    }
     if (with_e) {
         CK(cudaMalloc((void**)&F.e, sizeof(T) * (size_t)ntot));
         CK(cudaMemset(F.e, 0, sizeof(T) * (size_t)ntot));
@@ -284,7 +279,7 @@ void alloc_fields(Fields<T>& F, long long ntot, bool with_e, bool with_cheb = tr
 template <typename T>
 void free_fields(Fields<T>& F)
 {
-    T* all[] = {F.p, F.r, F.r0, F.Mp, F.AMp, F.z, F.Az, F.Y, F.Z, F.W, F.e, F.V};
+    T* all[] = {F.p, F.r, F.r0, F.Mp, F.AMp, F.z, F.Az, F.Y, F.Z, F.W, F.e};
     for (T* q : all)
         if (q) cudaFree(q);
     F = Fields<T>();
@@ -702,6 +697,25 @@ void fast_precond(pps_solver* s, Fields<T>& F, T* B, T* X, Launcher& L, bool mir
     fast_cheb<T>(s, F, B, X, L, cheb_of(s), mirror);
 }
 
+// The launches of an application of degree n >= 4: one-step kernels, passes of three steps
+// (k_cheb3: FP32, Dirichlet, even rows), one-step kernels.  Below 64 K unknowns a pass's 6
+// extra planes and rows cost more than two launches (BiCGSTAB iteration: 32^3 106 us alone,
+// 115 in passes; 48 x 40 x 64 137, 125).  The steps that do not divide by three come first;
+// of two with an even number of passes one comes last, so that three work buffers and X
+// do (fast_cheb).
+struct ChebPlan {
+    int lead, passes, tail;
+};
+template <typename T>
+ChebPlan cheb_plan(const pps_solver* s, int n)
+{
+    if (!std::is_same<T, float>::value || s->n_unknowns < 65536 || n < 5 || !cheb3_ok(s->geo))
+        return ChebPlan{n - 2, 0, 0};
+    const int passes = (n - 2) / 3, rest = (n - 2) % 3;
+    if (rest == 2 && passes % 2 == 0) return ChebPlan{1, passes, 1};
+    return ChebPlan{rest, passes, 0};
+}
+
 // X = -s_{n-2} of the Chebyshev recurrence p on B (the preconditioner, or a smoother).
 template <typename T>
 void fast_cheb(pps_solver* s, Fields<T>& F, T* B, T* X, Launcher& L, const ChebP& p, bool mirror)
@@ -768,9 +782,6 @@ void fast_cheb(pps_solver* s, Fields<T>& F, T* B, T* X, Launcher& L, const ChebP
         s->sweep_launch_acc++;
         return;
     }
-    T* Y = F.Y;
-    T* Z = F.Z;
-    T* W = F.W;
     // coefficients of step it (2..n-2); the first step's Z = s0 = B/theta is folded into B's
     auto next_coef = [&](int it) {
         rhoOld = rhoCurr;
@@ -782,15 +793,16 @@ void fast_cheb(pps_solver* s, Fields<T>& F, T* B, T* X, Launcher& L, const ChebP
         }
         return c;
     };
-    // FP32: three steps a pass (k_cheb3), the steps that do not divide by three first.
-    // Below 64 K unknowns a pass's 6 extra planes and rows cost more than two launches
-    // (BiCGSTAB iteration: 32^3 106 us alone, 115 in passes; 48 x 40 x 64 137, 125).
-    int lead = n - 2;
-    if constexpr (std::is_same<T, float>::value) {
-        if (N >= 65536 && n >= 5 && F.V && cheb3_ok(g, {B, X, Y, Z, W, F.V})) lead = (n - 2) % 3;
-    }
-    if (lead > 0) {
-        fast_cheb_s01<T>(g, shc, B, Y, c01, done, st);
+    // y, z: the buffers of the last two steps; other(u): a work buffer that is neither, nor u
+    T *y = nullptr, *z = nullptr;
+    auto other = [&](const T* u) {
+        auto taken = [&](const T* w) { return w == y || w == z || w == u; };
+        return !taken(F.Y) ? F.Y : !taken(F.Z) ? F.Z : F.W;
+    };
+    const ChebPlan plan = cheb_plan<T>(s, n);
+    if (plan.lead > 0) {
+        y = other(nullptr);
+        fast_cheb_s01<T>(g, shc, B, y, c01, done, st);
         L.bytes += bytes_of<T>(N, 2);
         L.launches++;
     }
@@ -802,30 +814,38 @@ void fast_cheb(pps_solver* s, Fields<T>& F, T* B, T* X, Launcher& L, const ChebP
         s->sweep_bytes_acc += bytes_of<T>(N, words);
         s->sweep_launch_acc++;
     };
-    for (int it = 2; it <= lead; it++) {
-        const bool last = (it == n - 2);
-        const Coef c = next_coef(it);
-        fast_cheb_sweep<T>(g, shc, Y, B, it == 2 ? nullptr : Z, last ? X : W, c, done, st, !last || mirror);
+    auto sweep = [&](int it) {
+        const bool last = it == n - 2;
+        T* w = last ? X : other(nullptr);
+        fast_cheb_sweep<T>(g, shc, y, B, it == 2 ? nullptr : z, w, next_coef(it), done, st, !last || mirror);
         count(it == 2 ? 3 : 4);
-        if (!last) {
-            T* t = Z;   // (Y, Z, W) <- (W, Y, Z)
-            Z = Y;
-            Y = W;
-            W = t;
-        }
-    }
+        z = y;
+        y = w;
+    };
+    int it = 2;
+    for (; it <= plan.lead; it++) sweep(it);
     if constexpr (std::is_same<T, float>::value) {
-        T* V = F.V;
-        for (int it = lead + 1; it <= n - 2; it += 3) {   // steps it, it+1, it+2
+        // A pass that is not the last step leaves two: the later one in a work buffer, the one
+        // before it in another or in X.  X's values off the unknowns are the caller's: the
+        // next kernel may read them as Z, which it takes at unknowns only, but not as Y.  The
+        // pass before the kernel that writes X leaves X alone, so they take X in turns.
+        const int pairs = plan.passes - (plan.tail == 0 ? 1 : 0);
+        for (int q = 0; q < plan.passes; q++) {   // steps t, t+1, t+2
+            const int t = plan.lead + 1 + 3 * q;
             Coef c[3];
-            for (int q = 0; q < 3; q++) c[q] = it + q == 1 ? c01 : next_coef(it + q);
-            const bool last = it + 2 == n - 2;
-            const int mode = it == 1 ? 0 : it == 2 ? 1 : 2;
-            fast_cheb3(g, mode, mode == 0 ? B : Y, B, Z, last ? X : W, last ? nullptr : V, c, done, st);
-            count(1 + mode + (last ? 1 : 2));
-            std::swap(Y, W);   // the step just made is the next pass's Y, the one before it its Z
-            std::swap(Z, V);
+            for (int u = 0; u < 3; u++) c[u] = t + u == 1 ? c01 : next_coef(t + u);
+            const int mode = t == 1 ? 0 : t == 2 ? 1 : 2;
+            T *o = X, *o2 = nullptr;
+            if (q < pairs) {
+                o = other(nullptr);
+                o2 = (pairs - 1 - q) % 2 == 0 ? other(o) : X;
+            }
+            fast_cheb3(g, mode, mode == 0 ? B : y, B, z, o, o2, c, done, st);
+            count(1 + mode + (o2 ? 2 : 1));
+            y = o;
+            z = o2;
         }
+        for (int u = 0; u < plan.tail; u++) sweep(n - 1 - plan.tail + u);
     }
     if (prof) {
         CK(cudaEventRecord(s->sweep_ev[s->sweep_ev_used + 1], st));
