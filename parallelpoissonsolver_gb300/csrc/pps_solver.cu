@@ -2468,6 +2468,7 @@ pps_status pps_apply_operator(pps_solver* s, const double* u, double* out)
                 CK(cudaMemsetAsync(o32, 0, sizeof(float) * (size_t)s->geo.ntot, s->stream));
                 fast_stencil_dot<float>(s->geo, s->shape, u32, t32, o32, op_coef(s->geo), red(s, FIN_STORE), s->stream);
                 CK(cudaMemcpyAsync(ho.data(), o32, sizeof(float) * (size_t)s->geo.ntot, cudaMemcpyDeviceToHost, s->stream));
+                zero_off_unknowns<float>(s->geo, u32, s->stream);   // a work field again
                 CK(cudaStreamSynchronize(s->stream));
                 const long long sj = s->geo.sj, sk = s->geo.sk;
                 for (int k = s->geo.lo[2]; k < s->geo.hi[2]; k++)
