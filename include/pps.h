@@ -233,8 +233,10 @@ pps_status pps_apply_preconditioner(pps_solver* s, const double* B, double* X);
  * prolongation), other_* to the remaining Krylov update/stencil kernels.  cheb_cx 4
  * selects the x-vectorised FP32 kernels (one float4 per thread, the default where
  * npglobal[0] + 2 is a multiple of 4; FP64 fields and other rows run cx 1 tiles of
- * the same size).  cheb_us: the sweep's time per launch; other_us: the
- * stencil+dot kernel's. */
+ * the same size).  Applications in the three-step passes of the MIXED form (Dirichlet
+ * grids of 65,536 unknowns and more, npglobal[0] even, degree 5 and more) take no tile but
+ * for the steps that three does not divide.  cheb_us: time per launch of the sweep, or of
+ * an application in passes; other_us: the stencil+dot kernel's. */
 typedef struct {
     int cheb_ty, cheb_cx, cheb_waves;
     int other_ty, other_waves;
@@ -251,10 +253,10 @@ typedef struct {
 /* Autotuner (no reference counterpart; the reference fixes its launch shapes,
  * ALP/include/alpakaHelper.hpp:122-140): times every candidate shape on this
  * solver's grid and buffers, applies the fastest and returns it.  The Chebyshev
- * tiles are scored by the sweep's time, weighted by the Chebyshev launches per
- * Krylov stencil launch of an iteration (cheb_degree - 2, or the learned cycle's
- * fine degree - 2), plus that of the method's Krylov stencil kernel on the same
- * tiles; the other tiles by the stencil+dot kernel.
+ * tiles are scored by the sweep's time, weighted by its launches per Krylov stencil
+ * launch of an iteration (cheb_degree - 2, or the learned cycle's fine degree - 2; in
+ * passes the steps left over, 0 to 2), plus that of the method's Krylov stencil kernel
+ * on the same tiles; the other tiles by the stencil+dot kernel.
  * Candidates: ty 2/4/8, cx 1/2/4 (4: FP32 only), waves 1/2/4/8. */
 pps_status pps_autotune(pps_solver* s, pps_tuning* out);
 pps_status pps_get_tuning(const pps_solver* s, pps_tuning* out);
