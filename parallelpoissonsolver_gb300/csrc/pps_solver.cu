@@ -698,20 +698,27 @@ void fast_precond(pps_solver* s, Fields<T>& F, T* B, T* X, Launcher& L, bool mir
 }
 
 // The launches of an application of degree n >= 4: one-step kernels, passes of three steps
-// (k_cheb3: FP32, Dirichlet, even rows), one-step kernels.  Below 64 K unknowns a pass's 6
-// extra planes and rows cost more than two launches (BiCGSTAB iteration: 32^3 106 us alone,
-// 115 in passes; 48 x 40 x 64 137, 125).  The steps that do not divide by three come first;
-// of two with an even number of passes one comes last, so that three work buffers and X
-// do (fast_cheb).
+// (k_cheb3: FP32, Dirichlet, even rows), one-step kernels.  The steps that do not divide by
+// three come first; of two with an even number of passes one comes last, so that three
+// work buffers and X do (fast_cheb).
+//
+// Where passes pay (BiCGSTAB iteration, one step a launch -> passes): a pass takes 12 us and
+// more however small the grid, three launches 9.  An application of one pass reads B alone:
+// even at 64 K unknowns (62 x 62 x 20, degree 5: 51.6 -> 50.6 us; 256 x 256 x 1 57.7 -> 53.8).  Of
+// more, from 120 K (degree 11: 62 x 62 x 18 79 -> 107 us, 128 x 25 x 24 84 -> 115, 62 x 62 x 30 98 -> 106;
+// 62 x 62 x 40 103 -> 100, 46 x 46 x 60 106 -> 98, 64^3 107 -> 104).  Rows of 32 unknowns or
+// fewer make one tile along x of 90 rows, most of it idle on a few rows and planes: from
+// 200 K (30 x 62 x 71 97 -> 122 us; 30 x 60 x 120 118 -> 116, 16 x 128 x 128 168 -> 111).
 struct ChebPlan {
     int lead, passes, tail;
 };
 template <typename T>
 ChebPlan cheb_plan(const pps_solver* s, int n)
 {
-    if (!std::is_same<T, float>::value || s->n_unknowns < 65536 || n < 5 || !cheb3_ok(s->geo))
-        return ChebPlan{n - 2, 0, 0};
     const int passes = (n - 2) / 3, rest = (n - 2) % 3;
+    const long long from = passes == 1 ? 65536 : s->geo.hi[0] - s->geo.lo[0] > 32 ? 122880 : 204800;
+    if (!std::is_same<T, float>::value || passes == 0 || s->n_unknowns < from || !cheb3_ok(s->geo))
+        return ChebPlan{n - 2, 0, 0};
     if (rest == 2 && passes % 2 == 0) return ChebPlan{1, passes, 1};
     return ChebPlan{rest, passes, 0};
 }

@@ -12,7 +12,9 @@ pytestmark = pytest.mark.gpu
 
 # degree - 2 steps: passes of three, 0, 1 or 2 left over (an even and an odd number of passes)
 @pytest.mark.parametrize("degree", [5, 8, 9, 10, 11, 12, 13, 14, 15, 16, 17, 19])
-@pytest.mark.parametrize("n", [(64, 32, 33), (252, 40, 7)])   # 8-byte and 16-byte quads, several tiles along y
+#                                       8-byte quads (one tile along x, several along y), 16-byte quads (several
+#                                       along both), rows of 8 lanes; one that runs in passes up to degree 7 alone
+@pytest.mark.parametrize("n", [(62, 50, 40), (252, 40, 13), (30, 80, 86), (64, 32, 33)])
 def test_passes_ignore_the_output_field_off_the_unknowns(gpu, oracle, n, degree):
     """Against the oracle with the one-step FP32 preconditioner's tolerance (2e-5)."""
     npg, ds = tuple(v + 2 for v in n), (0.03, 0.035, 0.025)

@@ -83,11 +83,30 @@ def test_mixed_solves_with_neumann_faces_on_float4_rows(gpu, oracle, faces):
 
 
 @pytest.mark.parametrize("degree", [5, 9, 10, 11])
-@pytest.mark.parametrize("n", [(252, 47, 6), (500, 40, 4), (60, 95, 12), (252, 18, 17)])   # 16-byte quads, tiles along y (and x)
+@pytest.mark.parametrize("n", [(252, 47, 11), (500, 40, 7), (60, 95, 22), (252, 18, 28)])   # 16-byte quads, tiles along y (and x)
 def test_16_byte_passes_over_several_tiles_match_the_oracle(gpu, oracle, n, degree):
     npg, ds = tuple(v + 2 for v in n), (0.03, 0.035, 0.025)
     grid = pps.BlockGrid(npglobal=npg, ds=ds)
-    assert grid.shape[2] % 4 == 0 and np.prod(n) >= 65536
+    assert grid.shape[2] % 4 == 0 and np.prod(n) >= 122880
+    B = np.random.default_rng(degree).standard_normal(grid.shape)
+    s = pps.BiCGSTAB(grid, pps.ChebyshevIteration(degree), form="mixed")
+    got = s.apply_preconditioner(B.copy())
+    s.close()
+    want = oracle.cheb_apply(oracle.Grid(npg, ds, (0.0, 0.0, 0.0), (0,) * 6), config(oracle, degree), B.copy())
+    sl = grid.unknowns()
+    assert np.linalg.norm(got[sl] - want[sl]) <= 2e-5 * np.linalg.norm(want[sl])
+
+
+@pytest.mark.parametrize("degree", [8, 9, 10, 11])
+@pytest.mark.parametrize("n", [(62, 32, 66),      # 16 lanes a row
+                               (30, 62, 113),     # 8 lanes a row, the last quad half full
+                               (128, 25, 41),     # a row is exactly 32 quads from its first unknown
+                               (130, 19, 52),     # two tiles along x, ragged
+                               (250, 18, 29),     # 8-byte quads, three tiles
+                               (252, 7, 72)])     # fewer rows than a tile
+def test_several_passes_on_ragged_tiles_match_the_oracle(gpu, oracle, n, degree):
+    npg, ds = tuple(v + 2 for v in n), (0.03, 0.035, 0.025)
+    grid = pps.BlockGrid(npglobal=npg, ds=ds)
     B = np.random.default_rng(degree).standard_normal(grid.shape)
     s = pps.BiCGSTAB(grid, pps.ChebyshevIteration(degree), form="mixed")
     got = s.apply_preconditioner(B.copy())
