@@ -3275,14 +3275,19 @@ static bool flat_ok(const Geo& g, std::initializer_list<const void*> ptrs)
     return true;
 }
 // Blocks of a flat pass that ends in a reduction: at most the shape's, each with 8
-// vectors per thread or more.  Every block pays a shuffle tree and a chain of FP64
-// additions (2 lanes per clock and SM on GB300) for its sums: on 128^3 doubles one
-// vector per thread, 4096 blocks, took 68 us for z.r, z.Ap, r.r against 26 us with 561.
+// vectors per thread or, where that leaves fewer than two blocks an SM, 4, 2 or 1.  Every
+// block pays a chain of FP64 additions (2 lanes per clock and SM on GB300) for its sums:
+// on 128^3 doubles one vector per thread, 4096 blocks, took 68 us for z.r, z.Ap, r.r
+// against 26 us with 561.  On small grids it is the loads in flight that count: with 8
+// vectors throughout, FP64 flexible CG with the polynomial took 2.94 ms at 32^3 (12 blocks;
+// 2.38 now) and 7.03 at 64^3 (77; 5.77), mixed 4.42 at 44^3 (14; 3.74).
 template <typename T>
 static unsigned flat_red_blocks(const Geo& g, const Shape& sh)
 {
-    const long long vecs = g.ntot / Vec16<T>::n, per = 8LL * 32 * sh.ty;
-    return (unsigned)std::max(1LL, std::min((long long)sh.nblocks(), (vecs + per - 1) / per));
+    const long long vecs = g.ntot / Vec16<T>::n, threads = 32 * sh.ty;
+    long long per = 8;
+    while (per > 1 && vecs < per * threads * 2 * sm_count()) per /= 2;
+    return (unsigned)std::max(1LL, std::min((long long)sh.nblocks(), (vecs + per * threads - 1) / (per * threads)));
 }
 template <typename T>
 void fast_axpy_alpha(const Geo& g, const Shape& sh, T* r, const T* v, const DevState* st, cudaStream_t s)
