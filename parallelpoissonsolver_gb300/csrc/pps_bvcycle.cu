@@ -45,7 +45,7 @@ namespace bvc {
 constexpr int MAXLEV = 6;          // levels 0..5
 constexpr int NT = 256;            // threads per block: 32 x 8 columns of a tile
 constexpr int EX_MAX = 32;         // coarsest level: at most 32 unknowns per axis
-constexpr int KZ0 = 128, KZ1 = 16, WAVES = 8;   // longest z chunks of work items; items per resident block
+constexpr int KZ0 = 128, KZ1 = 16;   // longest z chunks of work items: level 0, coarse levels
 constexpr double RATIO = 8.0;      // smoothing interval [lmax/RATIO, lmax]
 
 struct Prob {
@@ -1368,12 +1368,23 @@ bool bvc_create(BvcPlan** out, int nprob, const Geo* geo, const long long* off, 
         table[(size_t)t] = P->prob[(size_t)order[(size_t)t]];
         P->slot[(size_t)order[(size_t)t]] = t;
     }
+    // one resident wave: the grid barrier needs every block resident
+    VK(cudaFuncSetAttribute(k_bvc_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P->ex_smem));
+    int per_sm = 0;
+    VK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bvc_solve, NT, P->ex_smem));
+    if (per_sm < 1) {
+        err = "the persistent kernel does not fit on an SM";
+        return fail();
+    }
+    P->grid = per_sm * sm_count();
     // Work items of every level: a tile of columns (quads on level 0: 256 >> lwlog rows of
-    // 1 << lwlog quads; else 32 x 8 columns) by a chunk of planes.  The chunks are as long
-    // as KZ0 / KZ1 planes where that leaves 8 items for each of the 4 blocks of every
-    // SM, and shorter down to 4 planes where it does not: a phase of a small batch is
-    // one march long (8 problems of 32 and 64: 9.3 ms with 128 planes, 2.4 with 4; 256
-    // problems: 70.3 ms with 4 items a block, 66.7 with 8, 69.8 with 16).
+    // 1 << lwlog quads; else 32 x 8 columns) by a chunk of planes, block b taking items b,
+    // b + grid and so on.  A chunk costs its planes and about 4 more (its start, the plane
+    // on either side, the block sum), and the phase ends with its fullest block: of chunks
+    // of 128 (coarse levels 16) down to 4 planes the level takes those for which that block
+    // has the least to do.  (Chunks that leave 8 items a block, whatever the sizes: 200
+    // problems of 26^3 5.31 ms, 30 of 62^3 20.1, 32 of 96^3 14.8; 4.16, 14.4 and 11.7 with
+    // this; 250 of 32 to 128 57.7 and 57.4.  Chunks of 128 throughout: 8 of 32 and 64 9.3 ms, 1.8 with this.)
     P->toff.assign((size_t)MAXLEV * (nprob + 1), 0);
     std::vector<int4> items;
     std::vector<size_t> items_at(MAXLEV + 1, 0);
@@ -1383,18 +1394,30 @@ bool bvc_create(BvcPlan** out, int nprob, const Geo* geo, const long long* off, 
             w = quads ? 4 << pr.lwlog : 32;
             hgt = quads ? NT >> pr.lwlog : 8;
         };
-        auto count = [&](const Prob& pr, int kz) -> long long {
-            if (l > pr.k) return 0;
-            int w, hgt;
-            tile(pr, w, hgt);
-            const int n = pr.n[l];
-            return (long long)((n + w - 1) / w) * ((n + hgt - 1) / hgt) * ((n + kz - 1) / kz);
+        auto fullest = [&](int kz) -> long long {   // planes of the fullest block
+            std::vector<long long> load((size_t)P->grid, 0);
+            size_t b = 0;
+            for (const Prob& pr : table) {
+                if (l > pr.k) continue;
+                int w, hgt;
+                tile(pr, w, hgt);
+                const int n = pr.n[l], tiles = ((n + w - 1) / w) * ((n + hgt - 1) / hgt);
+                for (int k0 = 0; k0 < n; k0 += kz)
+                    for (int q = 0; q < tiles; q++) {
+                        load[b] += std::min(kz, n - k0) + 4;
+                        b = b + 1 < load.size() ? b + 1 : 0;
+                    }
+            }
+            return *std::max_element(load.begin(), load.end());
         };
         int kz = l == 0 ? KZ0 : KZ1;
-        for (; kz > 4; kz /= 2) {
-            long long total = 0;
-            for (const Prob& pr : table) total += count(pr, kz);
-            if (total >= (long long)WAVES * 4 * sm_count()) break;
+        long long least = fullest(kz);
+        for (int c = kz / 2; c >= 4; c /= 2) {
+            const long long m = fullest(c);
+            if (m < least) {
+                least = m;
+                kz = c;
+            }
         }
         items_at[(size_t)l] = items.size();
         for (int t = 0; t < nprob; t++) {
@@ -1503,15 +1526,6 @@ bool bvc_create(BvcPlan** out, int nprob, const Geo* geo, const long long* off, 
     D.ja2 = (float)(2.0 * rho2 * sigma);
     D.jb2 = (float)(2.0 * rho2 / delta);
     D.jc2 = (float)(rho2 * rho1);
-    // one resident wave: the grid barrier needs every block resident
-    VK(cudaFuncSetAttribute(k_bvc_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P->ex_smem));
-    int per_sm = 0;
-    VK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bvc_solve, NT, P->ex_smem));
-    if (per_sm < 1) {
-        err = "the persistent kernel does not fit on an SM";
-        return fail();
-    }
-    P->grid = per_sm * sm_count();
     P->hst.resize((size_t)nprob);
     *out = reinterpret_cast<BvcPlan*>(P);
     return true;
