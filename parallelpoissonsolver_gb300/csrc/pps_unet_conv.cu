@@ -120,6 +120,14 @@ __device__ __forceinline__ void ldsm4(unsigned (&r)[4], unsigned addr)
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                  : "r"(addr));
 }
+// the same, kept in its place among the warp's shared-memory stores
+__device__ __forceinline__ void ldsm4_ordered(unsigned (&r)[4], unsigned addr)
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr)
+                 : "memory");
+}
 __device__ __forceinline__ void ldsm4t(unsigned (&r)[4], unsigned addr)
 {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -165,8 +173,11 @@ __device__ __forceinline__ double mse_term(const Epi& e, long long v, float val)
 // ---------------------------------------------------------------------------
 // Small grids.  One block: 16 consecutive voxels x 16 output channels, the K steps
 // dealt to NW warps, so a block's dependent chain is 1/NW of K (a 16^3 grid has 256
-// such blocks; latency, not the tensor pipe, is the limit).  Each lane loads its own
-// fragment words straight from the source, four steps' loads in flight at a time.
+// such blocks; latency, not the tensor pipe, is the limit).  A lane loads 8 channels of a
+// voxel, four steps' loads in flight at a time, and a matrix load hands them out: loaded
+// straight into the fragments, two channels at a time, they were twice the cache-line
+// lookups, and layers of 48 and more channels were bound by those (forward on 16^3,
+// 80/16/16 channels: 258 -> 184 us, 48/48/48 180 -> 137, 16/32/64 94 -> 84).
 // ---------------------------------------------------------------------------
 template <int NW, int KIND>
 __global__ void __launch_bounds__(32 * NW) k_conv_small(Dims d, Src in, const uint4* __restrict__ Wp, int Cin, int Cout,
@@ -174,56 +185,58 @@ __global__ void __launch_bounds__(32 * NW) k_conv_small(Dims d, Src in, const ui
 {
     pdl_enter();
     if (stop && *(volatile const int*)stop) return;
-    __shared__ __align__(16) float sC[NW][16 * 16];
-    __shared__ double sl[16];
     constexpr int U = 4;
+    __shared__ __align__(16) unsigned char buf[NW * U * 512];   // a warp's A blocks of U steps, then its sums
+    __shared__ double sl[16];
+    float (*sC)[16 * 16] = reinterpret_cast<float (*)[16 * 16]>(buf);
     const long long nvox = (long long)d.D * d.H * d.W;
     const long long v0 = (long long)blockIdx.x * 16;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int gid = lane >> 2, tig = lane & 3;
-    int xr[2], yr[2], zr[2];
-    bool vin[2];
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-        const long long v = v0 + gid + 8 * h;
-        vin[h] = v < nvox;
-        xr[h] = (int)(v % d.W);
-        yr[h] = (int)((v / d.W) % d.H);
-        zr[h] = (int)(v / ((long long)d.W * d.H));
-    }
+    // the voxel whose channels this lane loads, the 8 of 16 it loads, and where they go: rows
+    // of 32 bytes whose halves trade places every four rows, so that the eight rows of a
+    // matrix load lie in different banks
+    const int row = lane >> 1, half = lane & 1;
+    const long long vox = v0 + row;
+    const bool vin = vox < nvox;
+    const int x = (int)(vox % d.W), y = (int)((vox / d.W) % d.H), z = (int)(vox / ((long long)d.W * d.H));
+    unsigned char* const slot = buf + warp * (U * 512);
+    unsigned char* const st = slot + row * 32 + ((half ^ (row >> 2)) & 1) * 16;
+    const unsigned ld = smem_u32(slot) + (lane & 15) * 32 + (((lane >> 4) ^ ((lane & 15) >> 2)) & 1) * 16;
     const int csteps = Cin / 16, ksteps = 27 * csteps, n16 = Cout / 16;
     const float in_sc = src_scale(in);
     float acc[2][4] = {};
     for (int t0 = warp; t0 < ksteps; t0 += NW * U) {
-        unsigned a[U][4];
+        Words<4> a[U];
         uint4 b[U];
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const int t = t0 + NW * u;
-#pragma unroll
-            for (int q = 0; q < 4; q++) a[u][q] = 0u;
+            a[u] = Words<4>{};
             b[u] = make_uint4(0, 0, 0, 0);
             if (t < ksteps) {
                 b[u] = Wp[((long long)t * n16 + blockIdx.y) * 32 + lane];
                 const int tap = t / csteps, c0 = (t - tap * csteps) * 16;
-                const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const int zz = zr[h] + dz, yy = yr[h] + dy, xx = xr[h] + dx;
-                    if (vin[h] && zz >= 0 && zz < d.D && yy >= 0 && yy < d.H && xx >= 0 && xx < d.W) {
-                        a[u][h] = load_src<1, KIND>(in, d, zz, yy, xx, c0 + 2 * tig, in_sc).w[0];
-                        a[u][2 + h] = load_src<1, KIND>(in, d, zz, yy, xx, c0 + 8 + 2 * tig, in_sc).w[0];
-                    }
-                }
+                const int zz = z + tap / 9 - 1, yy = y + (tap / 3) % 3 - 1, xx = x + tap % 3 - 1;
+                if (vin && zz >= 0 && zz < d.D && yy >= 0 && yy < d.H && xx >= 0 && xx < d.W)
+                    a[u] = load_src<4, KIND>(in, d, zz, yy, xx, c0 + 8 * half, in_sc);
             }
         }
+        __syncwarp();   // the last round's matrix loads are done
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            *reinterpret_cast<uint4*>(st + u * 512) = make_uint4(a[u].w[0], a[u].w[1], a[u].w[2], a[u].w[3]);
+        __syncwarp();
 #pragma unroll
         for (int u = 0; u < U; u++)
             if (t0 + NW * u < ksteps) {
-                mma16816(acc[0], a[u], b[u].x, b[u].y);
-                mma16816(acc[1], a[u], b[u].z, b[u].w);
+                unsigned m[4];
+                ldsm4_ordered(m, ld + u * 512);
+                mma16816(acc[0], m, b[u].x, b[u].y);
+                mma16816(acc[1], m, b[u].z, b[u].w);
             }
     }
+    __syncthreads();   // the sums take the A blocks' place
 #pragma unroll
     for (int n = 0; n < 2; n++) {
         *reinterpret_cast<float2*>(&sC[warp][gid * 16 + n * 8 + 2 * tig]) = make_float2(acc[n][0], acc[n][1]);
