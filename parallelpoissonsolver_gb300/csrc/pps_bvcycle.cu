@@ -1379,12 +1379,13 @@ bool bvc_create(BvcPlan** out, int nprob, const Geo* geo, const long long* off, 
     P->grid = per_sm * sm_count();
     // Work items of every level: a tile of columns (quads on level 0: 256 >> lwlog rows of
     // 1 << lwlog quads; else 32 x 8 columns) by a chunk of planes, block b taking items b,
-    // b + grid and so on.  A chunk costs its planes and about 4 more (its start, the plane
+    // b + grid and so on.  A chunk costs its planes and about 2 more (its start, the plane
     // on either side, the block sum), and the phase ends with its fullest block: of chunks
     // of 128 (coarse levels 16) down to 4 planes the level takes those for which that block
     // has the least to do.  (Chunks that leave 8 items a block, whatever the sizes: 200
-    // problems of 26^3 5.31 ms, 30 of 62^3 20.1, 32 of 96^3 14.8; 4.16, 14.4 and 11.7 with
-    // this; 250 of 32 to 128 57.7 and 57.4.  Chunks of 128 throughout: 8 of 32 and 64 9.3 ms, 1.8 with this.)
+    // problems of 26^3 5.32 ms, 30 of 62^3 20.2, 32 of 96^3 14.8; 4.02, 14.6 and 11.6 with
+    // this; 250 of 32 to 128 57.8 and 57.4, none of 50 batches slower.  With 4 more planes a
+    // chunk instead of 2, 30 of 40 to 80 took 6.67 ms, with 1 100 of 26^3 2.92; 6.21 and 2.17.)
     P->toff.assign((size_t)MAXLEV * (nprob + 1), 0);
     std::vector<int4> items;
     std::vector<size_t> items_at(MAXLEV + 1, 0);
@@ -1404,7 +1405,7 @@ bool bvc_create(BvcPlan** out, int nprob, const Geo* geo, const long long* off, 
                 const int n = pr.n[l], tiles = ((n + w - 1) / w) * ((n + hgt - 1) / hgt);
                 for (int k0 = 0; k0 < n; k0 += kz)
                     for (int q = 0; q < tiles; q++) {
-                        load[b] += std::min(kz, n - k0) + 4;
+                        load[b] += std::min(kz, n - k0) + 2;
                         b = b + 1 < load.size() ? b + 1 : 0;
                     }
             }
