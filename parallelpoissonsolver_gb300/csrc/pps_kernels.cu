@@ -575,7 +575,7 @@ __global__ void __launch_bounds__(256) k_canon_finalize(RedCtx rc, const int* do
         for (int q = 0; q < NS; q++) acc[q] += rc.cells[q * n + c];
     }
     // a warp without cells sums zeros: skipped (a shuffle tree of FP64 additions holds the
-    // SM's FP64 pipe for 80 clocks a sum)
+    // SM's FP64 pipe for 95 clocks a sum)
 #pragma unroll
     for (int q = 0; q < NS; q++) {
         const double w = c0 + warp * 32 < c1 ? warp_sum(acc[q]) : 0.0;
@@ -2412,8 +2412,9 @@ __global__ void __launch_bounds__(256, DOTS_RESIDENT) k_stencil_dots_v4(Geo g, i
     const int k0 = g.lo[2] + blockIdx.y * kchunk, k1 = min(k0 + kchunk, g.hi[2]);
     const bool act = j < g.hi[1] && i0 + 4 > g.lo[0];
     // x neighbours come by shuffle.  A lane that starts a row gets another row's value on its
-    // left, but x = 0 is no unknown.
-    const bool ldl = act && lane == 0, ldr = act && (lane == 31 || i0 + 4 >= g.hi[0]) && i0 + 4 < g.sj;
+    // left, but x = 0 is no unknown; nor is the last point of a row, where the lane that ends
+    // it gets one on its right (the row's quads fill its stride, hi is at most that less 1).
+    const bool ldl = act && lane == 0, ldr = act && lane == 31 && i0 + 4 < g.sj;
     const bool m0 = i0 >= g.lo[0] && i0 < g.hi[0], m1 = i0 + 1 >= g.lo[0] && i0 + 1 < g.hi[0];
     const bool m2 = i0 + 2 >= g.lo[0] && i0 + 2 < g.hi[0], m3 = i0 + 3 >= g.lo[0] && i0 + 3 < g.hi[0];
     const bool all4 = m0 && m1 && m2 && m3;
@@ -3276,8 +3277,8 @@ static bool flat_ok(const Geo& g, std::initializer_list<const void*> ptrs)
 }
 // Blocks of a flat pass that ends in a reduction: at most the shape's, each with 8
 // vectors per thread or, where that leaves fewer than two blocks an SM, 4, 2 or 1.  Every
-// block pays a chain of FP64 additions (2 lanes per clock and SM on GB300) for its sums:
-// on 128^3 doubles one vector per thread, 4096 blocks, took 68 us for z.r, z.Ap, r.r
+// block pays a chain of FP64 additions (19 clocks a warp and SM on GB300) for its sums: on 128^3
+// doubles one vector per thread, 4096 blocks, took 68 us for z.r, z.Ap, r.r
 // against 26 us with 561.  On small grids it is the loads in flight that count: with 8
 // vectors throughout, FP64 flexible CG with the polynomial took 2.94 ms at 32^3 (12 blocks;
 // 2.38 now) and 7.03 at 64^3 (77; 5.77), mixed 4.42 at 44^3 (14; 3.74).

@@ -20,8 +20,8 @@ __device__ __forceinline__ double fmx(double a, double b, double c) { return __f
 // per point (GB300 runs FP64 at 1/64 of the FP32 rate).
 template <typename T>
 struct Acc;
-// float to double on the integer pipe: the FP64 pipe, which also converts, takes 32 clocks a
-// warp.  Infinities, NaNs and denormals are left to the conversion instruction.
+// float to double on the integer pipe: the FP64 pipe, which also converts, takes 16 clocks a
+// warp (measured, one SM with 8 warps and more).  Infinities, NaNs and denormals are left to the conversion instruction.
 __device__ __forceinline__ double widen(float f)
 {
     const unsigned u = __float_as_uint(f), e = (u >> 23) & 255u;
@@ -72,10 +72,11 @@ __device__ __forceinline__ double warp_sum2(double a, double b)
 }
 
 // Block sums of NS values per thread, at most 256 threads: warp q (mod the warps) adds sum q,
-// eight or fewer values a lane and one shuffle tree.  GB300 issues an FP64 addition of a
-// warp in about 32 clocks an SM, so what counts is their number: a tree in every warp took
-// 5 a warp and sum, this takes 1 and a last tree (with conversions, 64 -> 20 a block and
-// sum).  Mixed CG on 120 x 128 x 90: 17.8 -> 14.3 ms.  st is shared memory; emit(q, sum) runs on one lane per sum.
+// eight or fewer values a lane and one shuffle tree.  An SM of GB300
+// takes 19 clocks for the FP64 addition of a warp (95 for a tree of five, measured with 8 warps
+// and more), so what counts is their number: a tree in every warp took 5 a warp and sum,
+// this takes 1 and a last tree (with conversions, 64 -> 20 a block and sum).  Mixed CG on
+// 120 x 128 x 90: 17.8 -> 14.3 ms.  st is shared memory; emit(q, sum) runs on one lane per sum.
 template <int NS, typename Emit>
 __device__ __forceinline__ void block_sums(const double (&v)[NS], double (*st)[256], int tid, int nwarp, Emit emit)
 {

@@ -89,7 +89,7 @@ __device__ __forceinline__ Words<NWORD> load_src(const Src& s, const Dims& d, in
         Words<NWORD> r = ld_words<NWORD>(s.X + vox * s.ld + s.c0 + c), m;
         const long long cv = ((long long)(z >> 1) * (d.H / 2) + (y >> 1)) * (d.W / 2) + (x >> 1);
         const Words<NWORD> p = ld_words<NWORD>(s.up + cv * s.ld_up + c);
-        if (s.mask) m = ld_words<NWORD>(s.mask + vox * s.ldm + s.cm0 + c);
+        if (s.mask) m = ld_words<NWORD>(s.mask + vox * s.ldm + c);
 #pragma unroll
         for (int q = 0; q < NWORD; q++) {
             r.w[q] = pack_bf(lo_f(r.w[q]) + 0.125f * lo_f(p.w[q]), hi_f(r.w[q]) + 0.125f * hi_f(p.w[q]));
@@ -258,8 +258,8 @@ __global__ void __launch_bounds__(32 * NW) k_conv_small(Dims d, Src in, const ui
             if (co == 0 && on) e.dense_out[v0 + v] = val * ((e.rms ? *e.rms : 1.0f) * e.gain);
         } else if (on) {
             bf16 r = __float2bfloat16(val);
-            if (e.mask && !(__bfloat162float(e.mask[(v0 + v) * e.ldm + e.cm0 + co]) > 0.0f)) r = __float2bfloat16(0.0f);
-            e.Y[(v0 + v) * e.ld + e.c0 + co] = r;
+            if (e.mask && !(__bfloat162float(e.mask[(v0 + v) * e.ldm + co]) > 0.0f)) r = __float2bfloat16(0.0f);
+            e.Y[(v0 + v) * e.ld + co] = r;
         }
     }
     if (e.target) {
@@ -408,8 +408,8 @@ __global__ void __launch_bounds__(32 * NWARP, NWARP > 8 || NC == 48 ? 1 : 2) k_c
                     if (co == 0) e.dense_out[vox] = v0 * ((e.rms ? *e.rms : 1.0f) * e.gain);
                 } else {
                     unsigned w = pack_bf(v0, v1);
-                    if (e.mask) w = relu_mask(w, *reinterpret_cast<const unsigned*>(e.mask + vox * e.ldm + e.cm0 + co));
-                    *reinterpret_cast<unsigned*>(e.Y + vox * e.ld + e.c0 + co) = w;
+                    if (e.mask) w = relu_mask(w, *reinterpret_cast<const unsigned*>(e.mask + vox * e.ldm + co));
+                    *reinterpret_cast<unsigned*>(e.Y + vox * e.ld + co) = w;
                 }
             }
         }

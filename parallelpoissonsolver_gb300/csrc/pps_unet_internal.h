@@ -40,7 +40,7 @@ struct Src {
     const bf16* up = nullptr;
     int ld_up = 0, c_up = 0;
     const bf16* mask = nullptr;   // null: no mask (identity activations)
-    int ldm = 0, cm0 = 0;
+    int ldm = 0;
 };
 // What a convolution does with its FP32 sums: + bias, ReLU, then one of
 //   Y (BF16, kept where mask > 0 when there is a mask);
@@ -49,11 +49,11 @@ struct Src {
 //   2 (val - target) inv_n into dense_out.
 struct Epi {
     bf16* Y = nullptr;
-    int ld = 0, c0 = 0;
+    int ld = 0;
     const float* bias = nullptr;
     int relu = 0;
     const bf16* mask = nullptr;
-    int ldm = 0, cm0 = 0;
+    int ldm = 0;
     float* dense_out = nullptr;
     const float* rms = nullptr;
     float gain = 1.0f;
