@@ -148,6 +148,7 @@ struct pps_solver {
     double g_sweep_bytes = 0;
     int g_sweep_launches = 0;
     bool g_learned = false;   // captured with the learned preconditioner active
+    unsigned long long g_net_version = 0;   // and with these buffers of the network's
     int g_learned_apps = 0;
 
     // learned preconditioner / initial guess (pps_set_learned)
@@ -1350,7 +1351,7 @@ pps_status run_iterations(pps_solver* s, Fields<T>& F, T* xacc, int form, Launch
         const bool learned = s->net && s->net_active;
         if (graph) {
             if (!(s->gexec && s->g_key_x == xacc && s->g_form == form && s->g_iters == chunk &&
-                  s->g_learned == learned)) {
+                  s->g_learned == learned && (!learned || s->g_net_version == pps_internal_unet_version(s->net)))) {
                 if (s->gexec) {
                     cudaGraphExecDestroy(s->gexec);
                     s->gexec = nullptr;
@@ -1383,6 +1384,7 @@ pps_status run_iterations(pps_solver* s, Fields<T>& F, T* xacc, int form, Launch
                 s->sweep_bytes_acc = sb;
                 s->sweep_launch_acc = sl;
                 s->g_learned = learned;
+                s->g_net_version = learned ? pps_internal_unet_version(s->net) : 0;
                 s->g_learned_apps = s->learned_apps - la;
                 s->learned_apps = la;
             }

@@ -85,6 +85,7 @@ struct pps_unet {
     RmsScratch* drms = nullptr;
     int step = 0;
     Acts A;
+    unsigned long long version = 0;   // of what a captured forward pass holds: A's buffers, the activation
     // Page-locked landing place of parameters and gradients (+ the loss behind them),
     // allocated when first read; reads of one network from several threads take turns.
     mutable float* stage = nullptr;
@@ -114,6 +115,7 @@ void ensure_acts(pps_unet* u, int nx, int ny, int nz, bool grads)
 {
     Acts& A = u->A;
     if (A.s1.W == nx && A.s1.H == ny && A.s1.D == nz && (A.grads || !grads)) return;
+    u->version++;
     free_acts(A);
     const long long v1 = (long long)nx * ny * nz, v2 = v1 / 8, v3 = v2 / 8;
     const int c1 = u->c1, c2 = u->c2, c3 = u->c3;
@@ -325,7 +327,11 @@ pps_status pps_internal_unet_apply(pps_unet* u, int nx, int ny, int nz, const fl
 {
     if (check_dims(nx, ny, nz) != PPS_OK) return PPS_ERR_INVALID_ARG;
     return uguard([&]() -> pps_status {
-        cudaStream_t saved = u->stream;
+        struct OnStream {   // the network's own stream again afterwards, an error included
+            pps_unet* u;
+            cudaStream_t own;
+            ~OnStream() { u->stream = own; }
+        } on{u, u->stream};
         u->stream = s;
         ensure_acts(u, nx, ny, nz, false);
         const long long nv = (long long)nx * ny * nz;
@@ -335,10 +341,11 @@ pps_status pps_internal_unet_apply(pps_unet* u, int nx, int ny, int nz, const fl
         last.rms = u->dtmp;
         last.gain = gain;
         forward(u, in, u->dtmp, last);
-        u->stream = saved;
         return PPS_OK;
     });
 }
+
+unsigned long long pps_internal_unet_version(const pps_unet* u) { return u->version; }
 
 extern "C" {
 
@@ -445,6 +452,7 @@ int pps_unet_param_count(const pps_unet* u) { return u ? (int)u->nreal : -1; }
 pps_status pps_unet_set_activation(pps_unet* u, int linear)
 {
     if (!u || (linear != 0 && linear != 1)) return PPS_ERR_INVALID_ARG;
+    if (u->linear != linear) u->version++;
     u->linear = linear;
     return PPS_OK;
 }

@@ -181,3 +181,6 @@ struct pps_unet;
 // out = gain * rms(in) * N(in / rms(in)).
 pps_status pps_internal_unet_apply(pps_unet* u, int nx, int ny, int nz, const float* in, float* out, float gain,
                                    cudaStream_t s);
+// Changes with the network's buffers and activation: a captured forward pass is valid while
+// this is what it was at the capture.
+unsigned long long pps_internal_unet_version(const pps_unet* u);
