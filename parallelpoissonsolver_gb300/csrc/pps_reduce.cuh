@@ -232,14 +232,10 @@ static __device__ void finalize(const RedCtx& rc, const double* tot)
         break;
     }
     case FIN_STORE:
-        if (rc.store) {
-            if (((unsigned long long)rc.store & 7) == 0) {
-                *reinterpret_cast<double*>(rc.store) = tot[0];
-            } else {   // a caller's address of any alignment: byte by byte
-                unsigned char* to = reinterpret_cast<unsigned char*>(rc.store);
-                const long long bits = __double_as_longlong(tot[0]);
-                for (int q = 0; q < 8; q++) to[q] = (unsigned char)(bits >> (8 * q));
-            }
+        if (rc.store) {   // byte by byte: a caller's address of any alignment
+            unsigned char* to = static_cast<unsigned char*>(rc.store);
+            const long long bits = __double_as_longlong(tot[0]);
+            for (int q = 0; q < 8; q++) to[q] = (unsigned char)(bits >> (8 * q));
         }
         break;
     default:
