@@ -13,8 +13,9 @@
 // layers that follow (about 1e-4 of the output).  The K = 27 * Cin/16 steps are dealt
 // round-robin to 8 chains (16 from 64 steps up), each summed in step order by the
 // tensor core, and the chains are added in order; both kernels below keep exactly
-// that, so which of them runs cannot be told from the result.  (A tcgen05 accumulator
-// sums all steps in one chain of its own, hence mma.sync.)
+// that, so which of them runs cannot be told from the result.  (Both run the
+// same mma.sync products.  tcgen05 would need an accumulator for every chain, and whether
+// its products round as these has not been measured.)
 //
 // Weights come packed in fragment order (k_pack, k_adam): one uint4 per lane holds a
 // 16 x 16 block of W, so a step's weights are one coalesced 512-byte load.
