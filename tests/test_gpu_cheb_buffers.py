@@ -2,6 +2,8 @@
 steps they leave in the solver's three work buffers and the output field, so they need no
 device memory beyond the one-step kernels', and values of the output field off the unknowns
 (boundary nodes, guards: the caller's) never reach a result."""
+import gc
+
 import numpy as np
 import pytest
 
@@ -49,6 +51,7 @@ def test_a_mixed_solver_takes_60_bytes_a_point(gpu, bcs):
         return s, torch.cuda.mem_get_info()[0]
 
     make()[0].close()                     # the context's and the kernels' own memory
+    gc.collect()                          # nor what earlier tests left behind
     torch.cuda.synchronize()
     before = torch.cuda.mem_get_info()[0]
     s, after = make()
