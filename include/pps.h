@@ -234,9 +234,8 @@ pps_status pps_apply_preconditioner(pps_solver* s, const double* B, double* X);
  * selects the x-vectorised FP32 kernels (one float4 per thread, the default where
  * npglobal[0] + 2 is a multiple of 4; FP64 fields and other rows run cx 1 tiles of
  * the same size).  Applications in the three-step passes of the MIXED form (Dirichlet
- * grids, npglobal[0] even, degree 5 and more; 65,536 unknowns and more up to degree 7,
- * 122,880 beyond, 204,800 with rows of at most 32 unknowns) take no tile but for the steps
- * that three does not divide.  cheb_us: time per launch of the sweep, or of
+ * grids, npglobal[0] even, degree 5 and more, from 65,536 unknowns up to degree 7 and from
+ * about 130,000 beyond) take no tile but for the steps that three does not divide.  cheb_us: time per launch of the sweep, or of
  * an application in passes; other_us: the stencil+dot kernel's. */
 typedef struct {
     int cheb_ty, cheb_cx, cheb_waves;

@@ -704,12 +704,15 @@ void fast_precond(pps_solver* s, Fields<T>& F, T* B, T* X, Launcher& L, bool mir
 // work buffers and X do (fast_cheb).
 //
 // Where passes pay (BiCGSTAB iteration, one step a launch -> passes): a pass takes 12 us and
-// more however small the grid, three launches 9.  An application of one pass reads B alone:
-// even at 64 K unknowns (62 x 62 x 20, degree 5: 51.6 -> 50.6 us; 256 x 256 x 1 57.7 -> 53.8).  Of
-// more, from 120 K (degree 11: 62 x 62 x 18 79 -> 107 us, 128 x 25 x 24 84 -> 115, 62 x 62 x 30 98 -> 106;
-// 62 x 62 x 40 103 -> 100, 46 x 46 x 60 106 -> 98, 64^3 107 -> 104).  Rows of 32 unknowns or
-// fewer make one tile along x of 90 rows, most of it idle on a few rows and planes: from
-// 200 K (30 x 62 x 71 97 -> 122 us; 30 x 60 x 120 118 -> 116, 16 x 128 x 128 168 -> 111).
+// more however small the grid, three launches 9 and more by the columns that their tiles
+// occupy.  An application of one pass reads B alone: from 64 K unknowns (62 x 62 x 20, degree
+// 5: 51.6 -> 50.6 us; 256 x 256 x 1 57.7 -> 53.8).  Of more, from 128 K points of one-column
+// tiles (degree 11: 62 x 62 x 18 79 -> 107 us, 62 x 62 x 30 98 -> 106; 50 x 52 x 46 and 46 x 46 x 60,
+// which fill three quarters of their tiles, 106 -> 98, 254 x 254 x 2 103 -> 96) or 288 K of
+// float4 tiles (100 x 60 x 30 89 -> 95, 128 x 25 x 24 84 -> 115; 48^3 95 -> 95, 44 x 44 x 60 98 -> 93,
+// 64^3 107 -> 104).  Rows of 32 unknowns or fewer make one tile along x of 90 rows, most of
+// it idle on a few rows and planes: from 8/5 of that (30 x 62 x 71 97 -> 122 us; 30 x 60 x 120
+// 118 -> 116, 16 x 128 x 128 168 -> 111).
 struct ChebPlan {
     int lead, passes, tail;
 };
@@ -717,9 +720,13 @@ template <typename T>
 ChebPlan cheb_plan(const pps_solver* s, int n)
 {
     const int passes = (n - 2) / 3, rest = (n - 2) % 3;
-    const long long from = passes == 1 ? 65536 : s->geo.hi[0] - s->geo.lo[0] > 32 ? 122880 : 204800;
-    if (!std::is_same<T, float>::value || passes == 0 || s->n_unknowns < from || !cheb3_ok(s->geo))
-        return ChebPlan{n - 2, 0, 0};
+    if (!std::is_same<T, float>::value || passes == 0 || !cheb3_ok(s->geo)) return ChebPlan{n - 2, 0, 0};
+    const Geo& g = s->geo;
+    const long long nx = g.hi[0] - g.lo[0], ny = g.hi[1] - g.lo[1], nz = g.hi[2] - g.lo[2];
+    const bool quads = g.sj % 4 == 0;   // float4 tiles from x = 0, else one-column tiles
+    const long long points = (quads ? (g.hi[0] + 127) / 128 * 128 : (nx + 31) / 32 * 32) * ((ny + 7) / 8 * 8) * nz;
+    const long long from = quads ? 294912 : 131072;
+    if (passes == 1 ? s->n_unknowns < 65536 : 5 * points < (nx > 32 ? 5 : 8) * from) return ChebPlan{n - 2, 0, 0};
     if (rest == 2 && passes % 2 == 0) return ChebPlan{1, passes, 1};
     return ChebPlan{rest, passes, 0};
 }

@@ -83,11 +83,11 @@ def test_mixed_solves_with_neumann_faces_on_float4_rows(gpu, oracle, faces):
 
 
 @pytest.mark.parametrize("degree", [5, 9, 10, 11])
-@pytest.mark.parametrize("n", [(252, 47, 11), (500, 40, 7), (60, 95, 22), (252, 18, 28)])   # 16-byte quads, tiles along y (and x)
+@pytest.mark.parametrize("n", [(252, 47, 25), (500, 40, 16), (60, 95, 24), (252, 18, 50)])   # 16-byte quads, tiles along y (and x)
 def test_16_byte_passes_over_several_tiles_match_the_oracle(gpu, oracle, n, degree):
     npg, ds = tuple(v + 2 for v in n), (0.03, 0.035, 0.025)
     grid = pps.BlockGrid(npglobal=npg, ds=ds)
-    assert grid.shape[2] % 4 == 0 and np.prod(n) >= 122880
+    assert grid.shape[2] % 4 == 0
     B = np.random.default_rng(degree).standard_normal(grid.shape)
     s = pps.BiCGSTAB(grid, pps.ChebyshevIteration(degree), form="mixed")
     got = s.apply_preconditioner(B.copy())
@@ -103,7 +103,7 @@ def test_16_byte_passes_over_several_tiles_match_the_oracle(gpu, oracle, n, degr
                                (128, 25, 41),     # a row is exactly 32 quads from its first unknown
                                (130, 19, 52),     # two tiles along x, ragged
                                (250, 18, 29),     # 8-byte quads, three tiles
-                               (252, 7, 72)])     # fewer rows than a tile
+                               (252, 7, 150)])    # fewer rows than a tile
 def test_several_passes_on_ragged_tiles_match_the_oracle(gpu, oracle, n, degree):
     npg, ds = tuple(v + 2 for v in n), (0.03, 0.035, 0.025)
     grid = pps.BlockGrid(npglobal=npg, ds=ds)
